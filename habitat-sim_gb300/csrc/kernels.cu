@@ -303,7 +303,8 @@ __global__ void __launch_bounds__(T) prepare_kernel(const PrepareParams p) {
     const uint32_t co = block_exclusive_scan<T>(clusters, s_warp, &s_total);
     const uint32_t ctot = s_total;
     if (vis) {
-      rec.ordinal = s_tris + to;
+      rec.ordinal = sc.ordinal_shift == kOrdinalRunning ? s_tris + to
+                                                        : (s_count + vo) << sc.ordinal_shift;
       rec.cluster = s_clusters + co;
       p.visible[vis_base + s_count + vo] = rec;
       if (p.model) p.model[vis_base + s_count + vo] = model;
@@ -751,6 +752,9 @@ __device__ __forceinline__ uint32_t find_draw(const uint32_t* prefix, const Visi
 
 __device__ __forceinline__ int wrap(int i, int n, int mode) {
   if (mode == 0) {
+    // Most textures have power-of-two sides: the residue is a mask (two's
+    // complement), a fifth of the instructions of the division below.
+    if ((n & (n - 1)) == 0) return i & (n - 1);
     int m = i % n;
     return m < 0 ? m + n : m;
   }
@@ -975,7 +979,8 @@ __device__ __noinline__ uint32_t lit_color(const float4* __restrict__ vertex_nor
   return unorm8(rgb[0]) | (unorm8(rgb[1]) << 8) | (unorm8(rgb[2]) << 16) | (unorm8(dif[3]) << 24);
 }
 
-// Shade the winning triangle `t` of visible draw `rec` at pixel (px, py).
+// Shade the winning triangle of visible draw `rec`, of ordinal `ord`, at pixel
+// (px, py), whose centre is (sx, sy) in normalised device coordinates.
 // Mode 0: every texture sampled at level 0 with its magnification filter
 // (no texture of the launch needs a level of detail).  Mode 1: textures that
 // need one (mip levels or a minification filter other than the magnification
@@ -983,8 +988,8 @@ __device__ __noinline__ uint32_t lit_color(const float4* __restrict__ vertex_nor
 // pixels again with Mode 2, the level-of-detail path, in a separate loop, so
 // that the derivative code does not add to the common path's registers.
 template <int Mode>
-__device__ __forceinline__ bool shade(const RasterParams& p, int W, int H, const VisibleRec* rec, uint32_t t,
-                                      int px, int py, const WorldLight* lights, uint32_t nl,
+__device__ __forceinline__ bool shade(const RasterParams& p, int W, int H, const VisibleRec* rec, uint32_t ord,
+                                      int px, int py, float sx, float sy, const WorldLight* lights, uint32_t nl,
                                       const ModelRec* model, uint32_t& color, float& lin, uint32_t& sid) {
   // The record in 16-byte loads: mvp, zrow, (vertex_base, first_index,
   // tri_count, material), (semantic_id, ordinal, flags, chunk).
@@ -1007,7 +1012,7 @@ __device__ __forceinline__ bool shade(const RasterParams& p, int W, int H, const
   const uint4 u6 = __ldg(reinterpret_cast<const uint4*>(rec) + 6);
   const uint32_t flags = u6.z;
   const uint32_t vb = u5.x;
-  const uint32_t fi = u5.y + 3u * t;
+  const uint32_t fi = u5.y + 3u * (ord - u6.y);
   uint32_t v[3];
   float4 c[3], q[3];
   float d[3];
@@ -1023,8 +1028,6 @@ __device__ __forceinline__ bool shade(const RasterParams& p, int W, int H, const
     ze = fma_(zr[2], q[k].z, ze);
     d[k] = -ze;
   }
-  const float sx = __fdiv_rn(float(2 * px + 1 - W), float(W));
-  const float sy = __fdiv_rn(float(2 * py + 1 - H), float(H));
   float l[3], ex[3], ey[3], ez[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
@@ -1264,7 +1267,9 @@ __global__ void __launch_bounds__(T, 1024 / T) raster_kernel(const RasterParams 
     const uint32_t nvis = p.vis_count[wi.scene];
     const uint32_t total = p.vis_tris[wi.scene];
     const VisibleRec* vis = p.visible + vis_base;
-    const bool cached = nvis <= uint32_t(p.prefix_cap);
+    // Ordinals that name their draw need no search (SceneRec::ordinal_shift).
+    const uint32_t shift = p.scenes[p.cameras[wi.scene].source].ordinal_shift;
+    const bool cached = shift == kOrdinalRunning && nvis <= uint32_t(p.prefix_cap);
     if (cached)
       for (uint32_t i = threadIdx.x; i < nvis; i += T) prefix[i] = vis[i].ordinal;
     if (threadIdx.x == 0) s_qcount = 0;
@@ -1534,8 +1539,28 @@ __global__ void __launch_bounds__(T, 1024 / T) raster_kernel(const RasterParams 
     // a second loop by the same thread.
     constexpr uint64_t kDeferred = 1ull << 63;
     bool deferred = false;
-    for (int i = threadIdx.x; i < npx; i += T) {
-      const int px = c.rx0 + i % c.rw, py = c.ry0 + i / c.rw;
+    // Pixel centres of the region's columns and rows in normalised device
+    // coordinates, in the idle queue (a side is at most 1024): one division
+    // per column and row instead of two per pixel.
+    float* ndc = reinterpret_cast<float*>(queue);
+    static_assert(sizeof(QEntry) * 256 >= 2 * 1024 * sizeof(float), "the queue holds both tables");
+    for (int i = threadIdx.x; i < c.rw + c.rh; i += T)
+      ndc[i] = i < c.rw ? __fdiv_rn(float(2 * (c.rx0 + i) + 1 - c.W), float(c.W))
+                        : __fdiv_rn(float(2 * (c.ry0 + i - c.rw) + 1 - c.H), float(c.H));
+    __syncthreads();
+    // A thread's pixels are T apart: (column, row) advance by fixed amounts.
+    const int step_x = T % c.rw, step_y = T / c.rw;
+    int cx = int(threadIdx.x) % c.rw, cy = int(threadIdx.x) / c.rw;
+    auto advance = [&]() {
+      cx += step_x;
+      cy += step_y;
+      if (cx >= c.rw) {
+        cx -= c.rw;
+        ++cy;
+      }
+    };
+    for (int i = threadIdx.x; i < npx; i += T, advance()) {
+      const int px = c.rx0 + cx, py = c.ry0 + cy;
       const uint64_t key = keys[i];
       const int64_t o = sc.fb_offset + int64_t(py) * sc.pitch + px;
       uint32_t col = kBackground, sid = 0;
@@ -1543,8 +1568,9 @@ __global__ void __launch_bounds__(T, 1024 / T) raster_kernel(const RasterParams 
       if (key != kEmptyKey) {
         const uint32_t ord = uint32_t(key);
         dep = __uint_as_float(uint32_t(key >> 32));
-        const uint32_t di = find_draw(prefix, vis, cached, nvis, ord);
-        if (!shade<Lod ? 1 : 0>(p, c.W, c.H, vis + di, ord - __ldg(&vis[di].ordinal), px, py,
+        const uint32_t di =
+            shift == kOrdinalRunning ? find_draw(prefix, vis, cached, nvis, ord) : ord >> shift;
+        if (!shade<Lod ? 1 : 0>(p, c.W, c.H, vis + di, ord, px, py, ndc[cx], ndc[c.rw + cy],
                                 lights, nlights, p.model ? p.model + vis_base + di : nullptr, col, lin, sid)) {
           keys[i] = key | kDeferred;
           deferred = true;
@@ -1557,17 +1583,20 @@ __global__ void __launch_bounds__(T, 1024 / T) raster_kernel(const RasterParams 
       if (p.out.semantic) p.out.semantic[o] = sid;
     }
     if (Lod && __syncthreads_or(deferred)) {
-      for (int i = threadIdx.x; i < npx; i += T) {
+      cx = int(threadIdx.x) % c.rw;
+      cy = int(threadIdx.x) / c.rw;
+      for (int i = threadIdx.x; i < npx; i += T, advance()) {
         const uint64_t key = keys[i];
         if (key == kEmptyKey || !(key & kDeferred)) continue;
-        const int px = c.rx0 + i % c.rw, py = c.ry0 + i / c.rw;
+        const int px = c.rx0 + cx, py = c.ry0 + cy;
         const int64_t o = sc.fb_offset + int64_t(py) * sc.pitch + px;
         const uint32_t ord = uint32_t(key);
         const float dep = __uint_as_float(uint32_t((key & ~kDeferred) >> 32));
-        const uint32_t di = find_draw(prefix, vis, cached, nvis, ord);
+        const uint32_t di =
+            shift == kOrdinalRunning ? find_draw(prefix, vis, cached, nvis, ord) : ord >> shift;
         uint32_t col, sid;
         float lin;
-        shade<2>(p, c.W, c.H, vis + di, ord - __ldg(&vis[di].ordinal), px, py, lights, nlights,
+        shade<2>(p, c.W, c.H, vis + di, ord, px, py, ndc[cx], ndc[c.rw + cy], lights, nlights,
                  p.model ? p.model + vis_base + di : nullptr, col, lin, sid);
         if (p.out.color) p.out.color[o] = col;
         if (p.out.depth) p.out.depth[o] = dep;
@@ -1794,6 +1823,7 @@ __global__ void no_alloc_setup(const NoAllocSetup a, NoAllocScratch* s) {
     sc.node_count = 2;
     sc.draw_base = 0;
     sc.draw_count = 1;
+    sc.ordinal_shift = ordinal_shift(1, kNoAllocMaxTriangles);
     s->scene = sc;
     CameraRec cam{};
     for (int i = 0; i < 16; ++i) cam.pv[i] = a.pv[i];

@@ -70,7 +70,22 @@ struct SceneRec {
   int64_t pitch;       // pixels per row
   uint32_t node_base, node_count;
   uint32_t draw_base, draw_count;
+  // Triangle ordinals of the scene's visible draws: visible draw i owns
+  // [i << ordinal_shift, (i + 1) << ordinal_shift), so that a pixel's winner
+  // names its draw; kOrdinalRunning when draw index and triangle index do not
+  // fit 32 bits together: ordinals then number the triangles consecutively
+  // and the draw is found by a search.
+  uint32_t ordinal_shift;
+  uint32_t pad;
 };
+constexpr uint32_t kOrdinalRunning = 32;
+// The shift for a scene of `draws` draws of at most `max_tris` triangles each.
+__host__ __device__ inline uint32_t ordinal_shift(uint32_t draws, uint32_t max_tris) {
+  uint32_t shift = 0, bits = 0;
+  while (shift < 31 && (1u << shift) < max_tris) ++shift;
+  while (bits < 31 && (1u << bits) < draws) ++bits;
+  return shift + bits <= 32 && shift < 32 ? shift : kOrdinalRunning;
+}
 
 struct DrawRec {
   uint32_t node;         // scene-local node index
@@ -135,7 +150,7 @@ struct alignas(16) VisibleRec {
   uint32_t tri_count;
   uint32_t material;
   uint32_t semantic_id;
-  uint32_t ordinal;    // index of this draw's first triangle in the scene
+  uint32_t ordinal;    // ordinal of this draw's first triangle (SceneRec::ordinal_shift)
   uint32_t flags;      // mesh flags
   uint32_t cluster;    // index of this draw's first cluster in the scene (draw order)
   uint32_t box_base;   // first chunk box of the draw's view; its cluster boxes follow

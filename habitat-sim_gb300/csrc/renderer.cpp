@@ -1060,6 +1060,7 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
       return sc.draws[a].batch < sc.draws[b].batch;
     });
     uint64_t tris = 0;
+    uint32_t max_tris = 0;
     for (uint32_t k : order) {
       const HostDraw& d = sc.draws[k];
       if (!mesh_live_[d.mesh] || !views_[d.view].live ||
@@ -1079,7 +1080,9 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
       dr.chunk_count = d.chunk_count;
       draws.push_back(dr);
       tris += dr.tri_count;
+      max_tris = std::max(max_tris, dr.tri_count);
     }
+    r.ordinal_shift = ordinal_shift(r.draw_count, max_tris);
     if (tris >= (1ull << 31))
       return fail(GBR_ERROR_INVALID_ARGUMENT, "draw: 2^31 or more triangles in one scene");
     cost[s] = tris;
