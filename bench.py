@@ -12,8 +12,8 @@ Printed (rank 0, one JSON line):
                and textures resident in HBM, L2 flushed before every step
                (a 256 MiB write outside the timed events); each step timed
                with CUDA events on the launching stream;
-  plain        the same workload through the plain per-scene path (two
-               launches per env, no graph);
+  plain        the same workload through the per-scene form of the draw (fixed
+               regions, one CTA each, no graph);
   e2e          the same metric through the C ABI with host buffers: poses
                from host arrays, framebuffer (colour, linear depth, ids) read
                back into pinned host memory by the imageInto calls;
@@ -360,7 +360,7 @@ def measure(pkg, procedural, name, wl, steps, warmup, plain_steps, e2e_steps, pa
     total_ms = max_over_ranks(sum(step_ms), world)
     value = job_frames_per_s(wl.envs, steps, world, total_ms)
 
-    # Plain per-scene path: one prepare + one raster launch per env, no graph.
+    # Per-scene form: fixed regions, one CTA each, no graph.
     plain_ms = []
     for k in range(plain_steps + 1 if plain_steps else 0):
         r.updateCameras(*poses[k % n])
@@ -445,8 +445,8 @@ def measure(pkg, procedural, name, wl, steps, warmup, plain_steps, e2e_steps, pa
             "p50_ms": float(np.percentile(plain_ms, 50)), "p99_ms": float(np.percentile(plain_ms, 99)),
             "ctas_per_env": {"min": min(plain_ctas), "max": max(plain_ctas),
                              "mean": float(np.mean(plain_ctas))},
-            "form": "per-scene prepare + raster launches (2 per env, one env after another), no graph; "
-                    "each env's raster launch is ctas_per_env CTAs of %d threads (%d x %d px regions)"
+            "form": "one prepare + one raster launch, no graph; "
+                    "ctas_per_env CTAs of %d threads per env (%d x %d px regions)"
                     % (t["threads"], t["plain_region_width"], t["plain_region_height"])},
         "batched_over_plain": value / plain_fps if plain_fps else None,
         "e2e": None if e2e_s is None else {

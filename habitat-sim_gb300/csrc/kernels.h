@@ -34,7 +34,7 @@ struct PrepareParams {
   uint32_t* vis_tris;
   uint32_t* vis_clusters;
   uint32_t* status;
-  uint32_t scene_base;
+  uint32_t* counter;  // the raster launch's work-item counter, reset here
   const LightSrc* light_src;  // [scene][max_lights] (lit renderers)
   WorldLight* lights;         // [scene][max_lights] (lit renderers)
   ModelRec* model;            // per visible draw (lit renderers, else null)
@@ -53,7 +53,13 @@ struct RasterParams {
   const uint32_t* vis_count;
   const uint32_t* vis_tris;
   const uint32_t* vis_clusters;
-  void* spill;                // per CTA (blockIdx) `threads` queue entries of spill space, or null
+  void* spill;                // per slot `threads` queue entries of spill space, or null
+  // Owners of the spill slots (0: free).  Null: CTA blockIdx.x owns slot
+  // blockIdx.x.  Else (a grid larger than what can be resident) there are
+  // `spill_slots` slots, as many as CTAs can be resident, and a CTA takes a
+  // free one.
+  uint32_t* spill_owner;
+  uint32_t spill_slots;
   const ChunkBox* boxes;      // chunk and cluster boxes (null: no box culling)
   const float4* pos;
   const float4* color;
@@ -95,7 +101,9 @@ size_t raster_spill_bytes(int threads, uint32_t grid);
 // Raises the kernel's dynamic shared-memory limit to the device maximum and
 // returns that maximum and the kernel's static shared memory.
 cudaError_t raster_configure(int threads, size_t* max_dynamic, size_t* static_bytes);
-cudaError_t launch_raster(const RasterParams& p, int threads, uint32_t grid, size_t smem,
+// early: the launch before it in the stream is the prepare kernel, and this
+// one's CTAs may start while it runs (the kernel waits for its completion).
+cudaError_t launch_raster(const RasterParams& p, int threads, uint32_t grid, size_t smem, bool early,
                           cudaStream_t stream);
 cudaError_t raster_max_ctas_per_sm(int threads, size_t smem, int* out);
 cudaError_t launch_unproject(float a, float b, float* depth, uint64_t rows, uint64_t cols,

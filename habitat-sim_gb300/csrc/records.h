@@ -82,8 +82,8 @@ constexpr uint32_t kOrdinalRunning = 32;
 // The shift for a scene of `draws` draws of at most `max_tris` triangles each.
 __host__ __device__ inline uint32_t ordinal_shift(uint32_t draws, uint32_t max_tris) {
   uint32_t shift = 0, bits = 0;
-  while (shift < 31 && (1u << shift) < max_tris) ++shift;
-  while (bits < 31 && (1u << bits) < draws) ++bits;
+  while (shift < 32 && (uint64_t(1) << shift) < max_tris) ++shift;
+  while (bits < 32 && (uint64_t(1) << bits) < draws) ++bits;
   return shift + bits <= 32 && shift < 32 ? shift : kOrdinalRunning;
 }
 

@@ -281,7 +281,7 @@ Renderer* Renderer::create(const gbr_config& cfg, std::string& err) {
 
 void Renderer::attach_budget() {
   DeviceBuffer* all[] = {&d_pos_, &d_color_, &d_uv_, &d_indices_, &d_texels_, &d_normal_, &d_lights_,
-                         &d_model_, &d_spill_, &d_gather_, &d_hbao_scenes_, &d_hbao_ao_, &d_meshes_,
+                         &d_model_, &d_spill_, &d_spill_owner_, &d_gather_, &d_hbao_scenes_, &d_hbao_ao_, &d_meshes_,
                          &d_materials_, &d_textures_, &d_boxes_, &d_scenes_, &d_parents_, &d_local_,
                          &d_draws_, &d_cameras_, &d_visible_, &d_order_, &d_vis_count_, &d_vis_tris_,
                          &d_vis_clusters_, &d_status_, &d_items_, &d_items_lpt_, &d_counter_};
@@ -1030,6 +1030,53 @@ gbr_status Renderer::upload_tables() {
   return GBR_OK;
 }
 
+// Launch shape of a renderer whose caller set none.  512-thread CTAs, two per
+// SM, on 128 x 64 regions with boxes of up to 4 px left to one lane: while one
+// CTA waits at a barrier the other issues (1024 textured 128 x 128 views: 2058
+// us against 2423 for one 1024-thread CTA on 128 x 128, 512 mixed views 745
+// against 826).  A draw too small for a region of 16 x 32 px on every other SM
+// takes 1024 threads per CTA: then the threads per region bound it (2 views:
+// 44 us against 51).  The per-scene form has a fixed region for all scenes:
+// the one of least step_cost.
+void Renderer::choose_shape() {
+  if (tuned_) return;
+  uint64_t cells = 0;
+  for (const SceneState& sc : scenes_) cells += uint64_t((sc.width + 15) / 16) * uint64_t((sc.height + 31) / 32);
+  const bool few = 2 * cells <= uint64_t(sm_count_);
+  gbr_tuning t = tuning_;
+  t.threads = few ? 1024 : 512;
+  t.ctas_per_sm = few ? 1 : 2;
+  t.region_width = 128;
+  t.region_height = 64;
+  t.small_area = 4;
+  const uint64_t grid = uint64_t(sm_count_) * uint64_t(t.ctas_per_sm);
+  const int sizes[][2] = {{128, 64}, {64, 64}, {64, 32}, {32, 32}, {16, 32}};
+  double best = -1.0;
+  for (const auto& r : sizes) {
+    uint64_t items = 0, total = 0, largest = 0;
+    for (const SceneState& sc : scenes_) {
+      ItemScene it;
+      it.width = sc.width;
+      it.height = sc.height;
+      it.tris = scenes_[sc.source].tris;
+      uint64_t n, cost;
+      split_cost(it, r[0], r[1], 0, n, cost);
+      items += n;
+      total += n * cost;
+      largest = std::max(largest, cost);
+    }
+    const double cost = step_cost(items, double(total), double(largest), grid);
+    if (best < 0.0 || cost < best) {
+      best = cost;
+      t.plain_region_width = r[0];
+      t.plain_region_height = r[1];
+    }
+  }
+  if (std::memcmp(&t, &tuning_, sizeof t) == 0) return;
+  tuning_ = t;
+  raster_configured_ = false;
+}
+
 gbr_status Renderer::rebuild(cudaStream_t stream) {
   GBR_CUDA(cudaStreamSynchronize(stream), "draw: synchronise before rebuild");
   if (gbr_status st = wait_uploads()) return st;
@@ -1093,13 +1140,16 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
   total_draws_ = uint32_t(draws.size());
   total_tris_ = std::accumulate(cost.begin(), cost.end(), uint64_t(0));
 
+  const bool search = search_ordinals_;
+  search_ordinals_ = false;
+  for (const SceneRec& r : recs) search_ordinals_ = search_ordinals_ || r.ordinal_shift == kOrdinalRunning;
+  if (search != search_ordinals_) raster_configured_ = false;
+  choose_shape();
   // Work items: each scene's viewport cut into regions.  The per-scene form
-  // uses small regions so that one scene spreads over several CTAs; the
-  // batched form uses large ones (fewer redundant triangle setups), ordered
-  // longest-processing-time first for the persistent grid by order_items().
+  // has one region size, small where few scenes have to spread over the GPU;
+  // the batched form uses large ones (fewer redundant triangle setups), split
+  // and ordered longest first for the persistent grid by order_items().
   std::vector<WorkItem> items;
-  scene_item_base_.assign(S, 0);
-  scene_item_count_.assign(S, 0);
   auto tile = [&](uint32_t s, int rwm, int rhm, std::vector<WorkItem>& out) {
     const SceneState& sc = scenes_[s];
     for (int y = 0; y < sc.height; y += rhm)
@@ -1115,9 +1165,7 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
   };
   std::vector<ItemScene> info(S);
   for (uint32_t s = 0; s < S; ++s) {
-    scene_item_base_[s] = uint32_t(items.size());
     tile(s, tuning_.plain_region_width, tuning_.plain_region_height, items);
-    scene_item_count_[s] = uint32_t(items.size()) - scene_item_base_[s];
     info[s].width = scenes_[s].width;
     info[s].height = scenes_[s].height;
   }
@@ -1187,7 +1235,9 @@ gbr_status Renderer::ensure_raster_config() {
     const size_t fixed = size_t(reserved) + static_smem;
     budget = std::min(budget, share > fixed ? share - fixed : size_t(0));
   }
-  int cap = kPrefixCapMax;
+  // Shared memory not used by the launch is L1 cache: no table of ordinals
+  // unless a scene needs it.
+  int cap = search_ordinals_ ? kPrefixCapMax : 0;
   size_t smem = raster_smem_bytes(tuning_.threads, std::max(region_px, plain_px), cap);
   while (smem > budget && cap > 64) {
     cap /= 2;
@@ -1200,8 +1250,8 @@ gbr_status Renderer::ensure_raster_config() {
   GBR_CUDA(raster_max_ctas_per_sm(tuning_.threads, smem, &occ), "raster occupancy");
   if (occ < 1) return fail(GBR_ERROR_INVALID_ARGUMENT, "tuning: raster kernel cannot be resident");
   ctas_per_sm_ = std::min(occ, std::max(1, tuning_.ctas_per_sm));
-  smem_bytes_ = smem;
   smem_plain_ = raster_smem_bytes(tuning_.threads, plain_px, cap);
+  GBR_CUDA(raster_max_ctas_per_sm(tuning_.threads, smem_plain_, &plain_ctas_per_sm_), "raster occupancy");
   prefix_cap_ = cap;
   raster_configured_ = true;
   return GBR_OK;
@@ -1327,6 +1377,19 @@ void Renderer::order_items() {
   }
   const uint64_t grid = std::max<uint64_t>(1, uint64_t(sm_count_) * uint64_t(ctas_per_sm_));
   const std::vector<WorkItem> items = build_work_items(info, tuning_.region_width, tuning_.region_height, grid);
+  // A step of few, small items is launched with a z-buffer of their size: the
+  // rest of the shared memory is L1 cache, which every region's culling reads
+  // the same boxes through (16 views of a room, 32 x 32 regions: 91 -> 81 us).
+  // The size is part of a captured graph, so a step that fills the grid keeps
+  // the shape's.
+  int px = tuning_.region_width * tuning_.region_height;
+  if (items.size() <= grid) {
+    int largest = 1024;
+    for (const WorkItem& it : items) largest = std::max(largest, int(it.w) * int(it.h));
+    while (px / 2 >= largest) px /= 2;
+  }
+  if (px != lpt_px_) graph_valid_ = false;
+  lpt_px_ = px;
   WorkItem* istage = reinterpret_cast<WorkItem*>(static_cast<char*>(h_stage_[slot_].ptr) +
                                                  camera_block_bytes() +
                                                  size_t(total_nodes_) * 64);
@@ -1357,6 +1420,7 @@ gbr_status Renderer::enqueue_step(cudaStream_t stream, uint32_t mode) {
   pp.vis_tris = d_vis_tris_.as<uint32_t>();
   pp.vis_clusters = d_vis_clusters_.as<uint32_t>();
   pp.status = d_status_.as<uint32_t>();
+  pp.counter = d_counter_.as<uint32_t>();
   RasterParams rp{};
   rp.scenes = pp.scenes;
   rp.cameras = pp.cameras;
@@ -1399,36 +1463,32 @@ gbr_status Renderer::enqueue_step(cudaStream_t stream, uint32_t mode) {
   }
   uint64_t launches = 0;
   if (mode == GBR_DRAW_BATCHED) {
-    pp.scene_base = 0;
     if (timing_) GBR_CUDA(cudaEventRecordWithFlags(ev_[0], stream, cudaEventRecordExternal), "timing event");
     GBR_CUDA(launch_prepare(pp, S, stream), "prepare launch");
-    GBR_CUDA(cudaMemsetAsync(d_counter_.ptr, 0, 4, stream), "counter reset");
     if (timing_) GBR_CUDA(cudaEventRecordWithFlags(ev_[1], stream, cudaEventRecordExternal), "timing event");
     rp.items = d_items_lpt_.as<WorkItem>();
     rp.item_base = 0;
     rp.item_count = lpt_count_;
     rp.item_count_dev = reinterpret_cast<const uint32_t*>(d_items_lpt_.as<WorkItem>() + lpt_count_);
     rp.persistent = 1;
-    rp.region_px = tuning_.region_width * tuning_.region_height;
+    rp.region_px = lpt_px_;
     const uint32_t grid =
         std::min<uint32_t>(lpt_count_, uint32_t(sm_count_) * uint32_t(ctas_per_sm_));
-    GBR_CUDA(launch_raster(rp, tuning_.threads, grid, smem_bytes_, stream), "raster launch");
+    GBR_CUDA(launch_raster(rp, tuning_.threads, grid, raster_smem_bytes(tuning_.threads, lpt_px_, prefix_cap_),
+                           !timing_, stream), "raster launch");
     if (timing_) GBR_CUDA(cudaEventRecordWithFlags(ev_[2], stream, cudaEventRecordExternal), "timing event");
     launches = 2;
   } else {
     rp.items = d_items_.as<WorkItem>();
     rp.persistent = 0;
     rp.region_px = tuning_.plain_region_width * tuning_.plain_region_height;
-    for (uint32_t s = 0; s < S; ++s) {
-      if (!scenes_[s].enabled) continue;
-      pp.scene_base = s;
-      GBR_CUDA(launch_prepare(pp, 1, stream), "prepare launch");
-      rp.item_base = scene_item_base_[s];
-      rp.item_count = scene_item_count_[s];
-      GBR_CUDA(launch_raster(rp, tuning_.threads, scene_item_count_[s], smem_plain_, stream),
-               "raster launch");
-      launches += 2;
-    }
+    rp.spill_owner = d_spill_owner_.as<uint32_t>();
+    rp.spill_slots = uint32_t(sm_count_) * uint32_t(plain_ctas_per_sm_);
+    rp.item_base = 0;
+    rp.item_count = item_count_;
+    GBR_CUDA(launch_prepare(pp, S, stream), "prepare launch");
+    GBR_CUDA(launch_raster(rp, tuning_.threads, item_count_, smem_plain_, true, stream), "raster launch");
+    launches = 2;
   }
   launches_ = launches;
   return GBR_OK;
@@ -1444,14 +1504,17 @@ gbr_status Renderer::draw(cudaStream_t stream, uint32_t mode, bool use_graph) {
   if (tables_dirty_)
     if (gbr_status s = upload_tables()) return s;
   {
-    // Queue spill space for every CTA of the largest launch (allocated
-    // before any graph capture).
+    // Queue spill space for every CTA that can be resident (allocated before
+    // any graph capture).
     uint32_t grid = uint32_t(sm_count_) * uint32_t(ctas_per_sm_);
-    if (mode != GBR_DRAW_BATCHED)
-      for (uint32_t c : scene_item_count_) grid = std::max(grid, c);
+    if (mode != GBR_DRAW_BATCHED) grid = uint32_t(sm_count_) * uint32_t(plain_ctas_per_sm_);
     void* before = d_spill_.ptr;
-    if (!d_spill_.reserve(raster_spill_bytes(tuning_.threads, grid), false))
+    const size_t owners = d_spill_owner_.bytes;
+    if (!d_spill_.reserve(raster_spill_bytes(tuning_.threads, grid), false) ||
+        (mode != GBR_DRAW_BATCHED && !d_spill_owner_.reserve(size_t(grid) * 4, false)))
       return fail(GBR_ERROR_OUT_OF_MEMORY, "draw: out of device memory for the raster queue");
+    if (d_spill_owner_.bytes != owners)
+      GBR_CUDA(cudaMemsetAsync(d_spill_owner_.ptr, 0, d_spill_owner_.bytes, stream), "spill owners");
     if (d_spill_.ptr != before) graph_valid_ = false;
   }
   const int prev_slot = slot_;
@@ -1803,6 +1866,7 @@ gbr_status Renderer::set_tuning(const gbr_tuning& t) {
       t.queue_fill_percent > 100)
     return fail(GBR_ERROR_INVALID_ARGUMENT, "setTuning: out of range");
   tuning_ = t;
+  tuned_ = true;
   raster_configured_ = false;
   structure_dirty_ = true;  // regions change
   return GBR_OK;

@@ -175,6 +175,7 @@ class Renderer {
   gbr_status upload_step(cudaStream_t stream);
   gbr_status enqueue_step(cudaStream_t stream, uint32_t mode);
   gbr_status ensure_raster_config();
+  void choose_shape();
   void build_chunk_boxes(uint32_t first_view, uint32_t last_view);
   void* plane_ptr(uint32_t plane, size_t* elem) const;
   gbr_status sync_and_check();
@@ -215,7 +216,8 @@ class Renderer {
   void attach_budget();
   DeviceBuffer d_pos_, d_color_, d_uv_, d_indices_, d_texels_, d_normal_;
   DeviceBuffer d_lights_, d_model_;  // lit renderers: world lights, per-draw model data
-  DeviceBuffer d_spill_;  // raster queue spill area, per CTA
+  DeviceBuffer d_spill_;  // raster queue spill area, per resident CTA
+  DeviceBuffer d_spill_owner_;  // per-scene form: owners of its slots (zero between draws)
   DeviceBuffer d_gather_;  // packed scenes on their way to host memory
   DeviceBuffer d_hbao_scenes_, d_hbao_ao_;  // ambient occlusion: per-scene records, two 8-bit planes
   uint32_t max_lights_ = 0;
@@ -244,19 +246,22 @@ class Renderer {
 
   uint32_t total_nodes_ = 0, total_draws_ = 0;
   uint64_t total_tris_ = 0;
-  std::vector<uint32_t> scene_item_base_, scene_item_count_;
   uint32_t item_count_ = 0;
   uint32_t lpt_count_ = 0;  // batched form: capacity of the item list (every scene at its finest split)
   uint32_t lpt_items_ = 0;  // batched form: items in the current list
+  int lpt_px_ = 0;          // batched form: pixels of the z-buffer a CTA is launched with
   bool bindings_dirty_ = true;           // sources or enabled flags changed
   bool items_staged_ = false;            // a new item order waits in the staging buffer
   uint64_t vis_needed_ = 0;              // visible records the current bindings need
 
   gbr_tuning tuning_{1024, 128, 128, 1, 1, 16, 32, 1, 75};
-  size_t smem_bytes_ = 0, smem_plain_ = 0;
+  bool tuned_ = false;  // set by the caller: choose_shape() keeps out
+  size_t smem_plain_ = 0;
+  bool search_ordinals_ = false;  // some scene's triangle ordinals do not name their draw
   int prefix_cap_ = 0;
   bool raster_configured_ = false;
   int ctas_per_sm_ = 1;
+  int plain_ctas_per_sm_ = 1;  // CTAs of the per-scene form that can be resident on an SM
 
   // CUDA graphs of the batched step, one per plane set
   cudaGraphExec_t graph_exec_[2] = {nullptr, nullptr};

@@ -20,29 +20,54 @@ struct ItemScene {
   bool enabled = true;
 };
 
-// Region halvings a costly scene's items may get.
+// Region halvings a costly scene's items may get, and the most when the
+// whole step has fewer items than the grid has CTAs.
 constexpr int kMaxSplits = 2;
+constexpr int kMaxFewSplits = 6;
 
 // Region of a scene's items after `level` splits of the batched form's
 // region (clamped to the viewport): each split halves the longer side, down
-// to 32 pixels.
+// to 32 pixels (16 beyond kMaxSplits).
 inline void split_region(int width, int height, int region_w, int region_h, int level, int& rw, int& rh) {
   rw = std::max(1, std::min(region_w, width));
   rh = std::max(1, std::min(region_h, height));
   for (int l = 0; l < level; ++l) {
-    if (rw >= rh && rw > 32)
+    const int side = l < kMaxSplits ? 32 : 16;
+    if (rw >= rh && rw > side)
       rw = (rw + 1) / 2;
-    else if (rh > 32)
+    else if (rh > side)
       rh = (rh + 1) / 2;
-    else if (rw > 32)
+    else if (rw > side)
       rw = (rw + 1) / 2;
   }
 }
 
-// Estimated cost of a w x h region of a W x H viewport: its share of the
-// scene's triangles plus a quarter of them for the region's culling and setup.
+// Estimated cost of a w x h region of a W x H viewport, in triangles drawn:
+// half of its share of the scene's (the rest is out of view), a twentieth of
+// them for the region's culling, 6000 for the phases that every region goes
+// through, and four per pixel for rasterising and shading it.  (One 128 x 128
+// view of a furnished room, 500k triangles: 83 us for a 16 x 32 region, 96 for
+// 32 x 32, 119 for 64 x 32, about 160 for 64 x 64; of a bare room, 49k
+// triangles: 34, 42 and 47 us.)
 inline uint64_t item_cost(uint64_t tris, int w, int h, int W, int H) {
-  return (tris + 1) * uint64_t(w) * uint64_t(h) / (uint64_t(W) * uint64_t(H)) + tris / 4;
+  const uint64_t px = uint64_t(w) * uint64_t(h);
+  return tris * px / (2 * uint64_t(W) * uint64_t(H)) + tris / 20 + 6000 + 4 * px;
+}
+
+// Estimated time of `items` items of total cost `total`, the largest costing
+// `largest`, on `grid` CTAs.  Items of equal estimate differ by half of it
+// either way: a single wave ends with its longest; in more waves the last
+// one, of halved items (build_work_items), overlaps the rest.
+inline double step_cost(uint64_t items, double total, double largest, uint64_t grid) {
+  return items <= grid ? 1.4 * largest : total / double(grid) + 0.8 * largest;
+}
+
+// Items of one scene split `level` times and the cost of the largest.
+inline void split_cost(const ItemScene& sc, int region_w, int region_h, int level, uint64_t& items, uint64_t& cost) {
+  int rw, rh;
+  split_region(sc.width, sc.height, region_w, region_h, level, rw, rh);
+  items = uint64_t((sc.width + rw - 1) / rw) * uint64_t((sc.height + rh - 1) / rh);
+  cost = item_cost(sc.tris, rw, rh, sc.width, sc.height);
 }
 
 // Items the list can ever hold: every scene at its finest split, plus the
@@ -60,46 +85,74 @@ inline uint64_t work_item_capacity(const std::vector<ItemScene>& scenes, int reg
 }
 
 // The items of the enabled scenes for a persistent grid of `grid` CTAs,
-// longest first.  A scene whose regions would each cost more than half a
-// CTA's share of the whole step (a small viewport bound to a large scene)
-// gets smaller regions (at most kMaxSplits halvings), so that no single item
-// outlasts the others; then the cheapest `grid` items -- the last wave -- are
-// halved (longer side, not below 32 px), so that the CTAs finishing the step
-// wait for half an item at most.  Items of equal cost are grouped by
-// geometry, so that the CTAs in flight read the same vertices from L2.
-// Measured on the serving workload: splitting at half the share beat the
-// whole share by 9 % and a quarter of it by 16 %; halving two waves or
-// quartering the last one was slower than halving one.
+// longest first.  No item may cost more than a limit: a scene whose regions
+// do gets them halved (at most kMaxSplits times, or kMaxFewSplits while the
+// step has no more items than CTAs).  The limit, the largest whole region's
+// cost or one of a falling sequence below it, is the one with the least
+// step_cost: it breaks up a small viewport bound to a large scene beside light
+// ones, and spreads a few views over the whole GPU.  Then the cheapest `grid` items --
+// the last wave -- are halved (longer side, not below 32 px), so that the CTAs
+// finishing the step wait for half an item at most.  Items of equal cost are
+// grouped by geometry, so that the CTAs in flight read the same vertices from
+// L2.  Halving two waves or quartering the last one was slower than halving
+// one.
 inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scenes, int region_w, int region_h,
                                               uint64_t grid) {
   grid = std::max<uint64_t>(grid, 1);
   const uint32_t S = uint32_t(scenes.size());
-  uint64_t total = 0;
+  // Per scene and level: items and largest cost (levels that change nothing repeat).
+  struct Level {
+    uint64_t items, cost;
+  };
+  std::vector<Level> levels(size_t(S) * (kMaxFewSplits + 1), Level{0, 0});
+  uint64_t limit = 1;
   for (uint32_t s = 0; s < S; ++s) {
     const ItemScene& sc = scenes[s];
     if (!sc.enabled || sc.width <= 0 || sc.height <= 0) continue;
-    int rw, rh;
-    split_region(sc.width, sc.height, region_w, region_h, 0, rw, rh);
-    const uint64_t n = uint64_t((sc.width + rw - 1) / rw) * uint64_t((sc.height + rh - 1) / rh);
-    total += n * item_cost(sc.tris, rw, rh, sc.width, sc.height);
+    Level* l = &levels[size_t(s) * (kMaxFewSplits + 1)];
+    for (int k = 0; k <= kMaxFewSplits; ++k) split_cost(sc, region_w, region_h, k, l[k].items, l[k].cost);
+    limit = std::max(limit, l[0].cost);
   }
-  const uint64_t share = total / grid / 2;  // half a CTA's share of the step
+  auto level_of = [&](uint32_t s, uint64_t t, int most) {
+    const Level* l = &levels[size_t(s) * (kMaxFewSplits + 1)];
+    int k = 0;
+    while (k < most && l[k].cost > t) ++k;
+    return k;
+  };
+  int max_splits = kMaxSplits;
+  double best = -1.0;
+  uint64_t best_limit = limit;
+  for (int most : {kMaxSplits, kMaxFewSplits}) {
+    uint64_t t = limit;
+    for (int i = 0; i < 14 && t > 0; ++i, t = t * 7 / 10) {
+      uint64_t items = 0, total = 0, largest = 0;
+      bool few = false;
+      for (uint32_t s = 0; s < S; ++s) {
+        const Level* l = &levels[size_t(s) * (kMaxFewSplits + 1)];
+        if (!l[0].items) continue;
+        const int k = level_of(s, t, most);
+        few = few || k > kMaxSplits;
+        items += l[k].items;
+        total += l[k].items * l[k].cost;
+        largest = std::max(largest, l[k].cost);
+      }
+      if (few && items > grid) break;
+      const double cost = step_cost(items, double(total), double(largest), grid);
+      if (best < 0.0 || cost < best) {
+        best = cost;
+        best_limit = t;
+        max_splits = most;
+      }
+    }
+  }
   std::vector<WorkItem> items;
   std::vector<uint64_t> cost;
   std::vector<uint32_t> key;
   for (uint32_t s = 0; s < S; ++s) {
     const ItemScene& sc = scenes[s];
     if (!sc.enabled || sc.width <= 0 || sc.height <= 0) continue;
-    int rw, rh, level = 0;
-    split_region(sc.width, sc.height, region_w, region_h, 0, rw, rh);
-    while (level < kMaxSplits && item_cost(sc.tris, rw, rh, sc.width, sc.height) > share) {
-      int nw, nh;
-      split_region(sc.width, sc.height, region_w, region_h, level + 1, nw, nh);
-      if (nw == rw && nh == rh) break;
-      rw = nw;
-      rh = nh;
-      ++level;
-    }
+    int rw, rh;
+    split_region(sc.width, sc.height, region_w, region_h, level_of(s, best_limit, max_splits), rw, rh);
     for (int y = 0; y < sc.height; y += rh)
       for (int x = 0; x < sc.width; x += rw) {
         WorkItem it{};

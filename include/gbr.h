@@ -61,7 +61,7 @@ typedef struct gbr_renderer gbr_renderer;
 #define GBR_PLANE_ALL 15u
 
 /* Draw modes for gbr_draw_mode. */
-#define GBR_DRAW_PER_SCENE 0u /* one prepare + one raster launch per scene */
+#define GBR_DRAW_PER_SCENE 0u /* one prepare + one raster launch, one CTA per region */
 #define GBR_DRAW_BATCHED 1u   /* one prepare + one persistent raster launch */
 
 /* RendererConfiguration (Renderer.h:45-113) + RendererStandaloneConfiguration
