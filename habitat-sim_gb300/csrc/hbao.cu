@@ -51,7 +51,10 @@ __device__ __forceinline__ float poly_exp2(float x) {
   p = __fadd_rn(__fmul_rn(p, f), 0.24022650718688965f);
   p = __fadd_rn(__fmul_rn(p, f), 0.6931471824645996f);
   p = __fadd_rn(__fmul_rn(p, f), 1.0f);
-  return ldexpf(p, int(n));
+  // p 2^n for n in [-149, 0] (every caller's x is at most 0) in two factors:
+  // the first product is exact, the second rounds once, into the denormals.
+  const int k = int(n), k1 = max(k, -126);
+  return __fmul_rn(__fmul_rn(p, __int_as_float((k1 + 127) << 23)), __int_as_float((k - k1 + 127) << 23));
 }
 
 __device__ __forceinline__ float poly_log2(float x) {
@@ -113,32 +116,43 @@ __device__ __forceinline__ uint8_t unorm8(float v) {
   return uint8_t(__fadd_rn(__fmul_rn(clamp01(v), 255.0f), 0.5f));
 }
 
+// v / 255 correctly rounded for a byte v: 1/255 as the sum of two floats, one
+// multiply and one fused multiply-add (Brisebarre and Muller, "Correctly
+// rounded multiplication by arbitrary precision constants", IEEE Trans.
+// Computers 57(2), 2008; checked for all 256 v in exact rational arithmetic).
+__device__ __forceinline__ float byte_unit(uint32_t v) {
+  const float f = __fsub_rn(__uint_as_float(0x4b000000u | v), 8388608.0f);
+  return __fmaf_rn(f, 0x1.010102p-8f, __fmul_rn(f, -0x1.fdfdfep-33f));
+}
+
 __device__ __forceinline__ uint32_t modulate(uint32_t c, float ao) {
   uint32_t out = c & 0xFF000000u;  // alpha: blend factor one
   for (int ch = 0; ch < 3; ++ch) {
-    const float v = __fmul_rn(__fdiv_rn(float((c >> (8 * ch)) & 0xFFu), 255.0f), ao);
+    const float v = __fmul_rn(byte_unit((c >> (8 * ch)) & 0xFFu), ao);
     out |= uint32_t(unorm8(v)) << (8 * ch);
   }
   return out;
 }
 
-// The grid has one block per 256 pixels of the batch: scene i owns blocks
-// scenes[i].block0 .. scenes[i + 1].block0 - 1.  The block's scene, by a
-// binary search of thread 0.
-__device__ __forceinline__ int scene_of_block(const HbaoScene* scenes, int count) {
-  __shared__ int s_si;
+// The scene of this block, by a binary search of thread 0, and the block's
+// index among the scene's.  First: the scenes' first blocks (block0 or blur0).
+template <int HbaoScene::*First>
+__device__ __forceinline__ int scene_of_block(const HbaoScene* scenes, int count, int* local) {
+  __shared__ int s_si, s_local;
   if (threadIdx.x == 0) {
-    int lo = 0, hi = count;  // scenes[lo].block0 <= blockIdx.x < scenes[hi].block0
+    int lo = 0, hi = count;  // scenes[lo].*First <= blockIdx.x < scenes[hi].*First
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
-      if (scenes[mid].block0 <= int(blockIdx.x))
+      if (scenes[mid].*First <= int(blockIdx.x))
         lo = mid;
       else
         hi = mid;
     }
     s_si = lo;
+    s_local = int(blockIdx.x) - scenes[lo].*First;
   }
   __syncthreads();
+  *local = s_local;
   return s_si;
 }
 
@@ -173,6 +187,51 @@ __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
 __device__ __forceinline__ float half_lo(uint32_t v) { return __half2float(__ushort_as_half((unsigned short)(v & 0xFFFFu))); }
 __device__ __forceinline__ float half_hi(uint32_t v) { return __half2float(__ushort_as_half((unsigned short)(v >> 16))); }
 
+// What the samples of one pixel need.
+struct AoPixel {
+  float3 P, N;
+  float u, v, su_scale, sv_scale;
+  int x, y, qx, qy, ox, oy;
+};
+
+// The AO that a sample at (su, sv) with depth zs adds.
+__device__ __forceinline__ float ao_sample(const HbaoScene& s, const HbaoParams& p, const AoPixel& a, float ao,
+                                           float su, float sv, float zs) {
+  const float3 S = view_pos(s, su, sv, zs);
+  const float3 V = sub(S, a.P);
+  const float vv = dot3(V, V);
+  const float fall = __fadd_rn(__fmul_rn(vv, p.neg_inv_r2), 1.0f);
+  const float nv = dot3(a.N, V);
+  // Most samples add exactly nothing and leave before the square root and the
+  // division: beyond the radius (fall <= 0 or not a number), behind the
+  // tangent plane, or below the bias: N.V / |V| < bias, decided on squares
+  // with a margin (bias2 = bias^2 (1 - 1e-5)) far above the roundings of
+  // either side, for |V| where the squares are normal numbers.
+  if (!(fall > 0.0f) || !(nv > 0.0f) || (vv > 1e-20f && __fmul_rn(nv, nv) < __fmul_rn(p.bias2, vv))) return ao;
+  const float ndotv = __fdiv_rn(nv, __fsqrt_rn(vv));
+  return __fadd_rn(ao, __fmul_rn(clamp01(__fsub_rn(ndotv, p.bias)), clamp01(fall)));
+}
+
+// All samples of a pixel whose steps or image are too large for the 32-bit
+// texel arithmetic of hbao_ao_kernel.
+template <bool CacheAware>
+__device__ __noinline__ float ao_far_samples(const HbaoScene& s, const float* __restrict__ depth,
+                                             const HbaoParams& p, const AoPixel& a, const float2* rot,
+                                             const float* ray) {
+  float ao = 0.0f;
+  for (int d = 0; d < 8; ++d)
+    for (int k = 0; k < 4; ++k) {
+      const float kx = rintf(__fmul_rn(ray[k], rot[d].x)), ky = rintf(__fmul_rn(ray[k], rot[d].y));
+      const float su = __fadd_rn(__fmul_rn(kx, a.su_scale), a.u), sv = __fadd_rn(__fmul_rn(ky, a.sv_scale), a.v);
+      // Offsets beyond the image only select the clamped edge texel.
+      const int ix = int(fminf(fmaxf(kx, -65536.0f), 65536.0f)), iy = int(fminf(fmaxf(ky, -65536.0f), 65536.0f));
+      const float zs = CacheAware ? layer_depth(s, depth, a.qx + ix, a.qy + iy, a.ox, a.oy)
+                                  : depth_at(s, depth, a.x + ix, a.y + iy);
+      ao = ao_sample(s, p, a, ao, su, sv, zs);
+    }
+  return ao;
+}
+
 // AO per pixel.  Classic: the pixel's own view position and reconstructed
 // normal, samples at full resolution, the 16-bit jitter of texel
 // (x & 3, y & 3).  CacheAware: the pixel belongs to deinterleaved layer
@@ -182,161 +241,247 @@ __device__ __forceinline__ float half_hi(uint32_t v) { return __half2float(__ush
 // steps (radius / 4), its jitter the layer's unquantized one; the result
 // lands at the pixel, which is the reinterleave.  Special: (AO, view depth)
 // stored as two halves.
+//
+// Bound by instruction issue: 32 samples per pixel, their depths served by L1
+// (a 16 x 16 tile's samples overlap).  Per sample, what the arithmetic fixes
+// is about 45 operations; the rest was cut: the rotated directions come from a
+// table, the four ray lengths are shared by the eight directions, a sample's
+// offset is rounded to an integer by adding 1.5 * 2^23 (which leaves the
+// integer in the low bits: no conversion instructions, a quarter of the rate
+// here), texels are addressed in 32 bits, and ao_sample leaves early.
 template <bool CacheAware, bool Special>
-__global__ void __launch_bounds__(256) hbao_ao_kernel(const HbaoScene* __restrict__ scenes, int count,
-                                                      const float* __restrict__ depth, uint32_t* color,
-                                                      void* q1, const HbaoParams p) {
-  {
-    const HbaoScene s = scenes[scene_of_block(scenes, count)];
-    const int pixels = s.w * s.h;
-    const float inv_w = __fdiv_rn(1.0f, float(s.w)), inv_h = __fdiv_rn(1.0f, float(s.h));
-    const int idx = (int(blockIdx.x) - s.block0) * 256 + int(threadIdx.x);
-    if (idx < pixels) {
-      const int x = idx % s.w, y = idx / s.w;
-      float u = __fdiv_rn(__fadd_rn(float(x), 0.5f), float(s.w));
-      float v = __fdiv_rn(__fadd_rn(float(y), 0.5f), float(s.h));
-      float3 P = view_pos(s, u, v, depth_at(s, depth, x, y));
-      float inv_len;
-      const float3 c = reconstruct_normal(s, depth, x, y, u, v, inv_w, inv_h, P, inv_len);
-      float3 N;
-      float radius;
-      const float* j;
-      float su_scale = inv_w, sv_scale = inv_h;
-      const int ox = x & 3, oy = y & 3, qx = x >> 2, qy = y >> 2;
-      if (!CacheAware) {
-        N = f3(-__fmul_rn(c.x, inv_len), -__fmul_rn(c.y, inv_len), -__fmul_rn(c.z, inv_len));
-        radius = __fdiv_rn(s.radius_to_screen, s.ortho ? 1.0f : P.z);
-        j = p.jitter + 4 * ((y & 3) * 4 + (x & 3));
-      } else {
-        const float e[3] = {c.x, c.y, c.z};
-        float n[3];
+__global__ void __launch_bounds__(256) hbao_ao_kernel(const HbaoScene* __restrict__ scenes, const HbaoScene one,
+                                                      int count, const float* __restrict__ depth, uint32_t* color,
+                                                      void* q, const HbaoParams p) {
+  __shared__ float2 s_rot[16][8];  // rotated directions of jitter texel j
+  if (threadIdx.x < 128) {
+    const int t = threadIdx.x >> 3, d = threadIdx.x & 7;
+    const float* j = (CacheAware ? p.jitter_f : p.jitter) + 4 * t;
+    const float dc = p.dirs[2 * d], ds = p.dirs[2 * d + 1];
+    s_rot[t][d] = make_float2(__fsub_rn(__fmul_rn(dc, j[0]), __fmul_rn(ds, j[1])),
+                              __fadd_rn(__fmul_rn(dc, j[1]), __fmul_rn(ds, j[0])));
+  }
+  int local = blockIdx.x;
+  HbaoScene s;
+  if (scenes) {
+    s = scenes[scene_of_block<&HbaoScene::block0>(scenes, count, &local)];
+  } else {
+    s = one;
+    __syncthreads();
+  }
+  const int tiles_x = (s.w + kAoTile - 1) / kAoTile;
+  const int x = (local % tiles_x) * kAoTile + (int(threadIdx.x) & (kAoTile - 1));
+  const int y = (local / tiles_x) * kAoTile + int(threadIdx.x) / kAoTile;
+  if (x >= s.w || y >= s.h) return;
+  AoPixel a;
+  a.x = x;
+  a.y = y;
+  a.u = __fdiv_rn(__fadd_rn(float(x), 0.5f), float(s.w));
+  a.v = __fdiv_rn(__fadd_rn(float(y), 0.5f), float(s.h));
+  a.P = view_pos(s, a.u, a.v, depth_at(s, depth, x, y));
+  float inv_len;
+  const float3 c = reconstruct_normal(s, depth, x, y, a.u, a.v, s.inv_w, s.inv_h, a.P, inv_len);
+  float radius;
+  a.su_scale = s.inv_w;
+  a.sv_scale = s.inv_h;
+  a.ox = x & 3;
+  a.oy = y & 3;
+  a.qx = x >> 2;
+  a.qy = y >> 2;
+  const int jt = a.oy * 4 + a.ox;
+  if (!CacheAware) {
+    a.N = f3(-__fmul_rn(c.x, inv_len), -__fmul_rn(c.y, inv_len), -__fmul_rn(c.z, inv_len));
+    radius = __fdiv_rn(s.radius_to_screen, s.ortho ? 1.0f : a.P.z);
+  } else {
+    const float e[3] = {c.x, c.y, c.z};
+    float n[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const float enc = float(unorm8(__fadd_rn(__fmul_rn(__fmul_rn(e[k], inv_len), 0.5f), 0.5f)));
-          n[k] = -__fsub_rn(__fmul_rn(__fdiv_rn(enc, 255.0f), 2.0f), 1.0f);
-        }
-        N = f3(n[0], n[1], n[2]);
-        u = __fmul_rn(__fadd_rn(__fmul_rn(float(qx), 4.0f), __fadd_rn(float(ox), 0.5f)), __fdiv_rn(s.inv_qw, 4.0f));
-        v = __fmul_rn(__fadd_rn(__fmul_rn(float(qy), 4.0f), __fadd_rn(float(oy), 0.5f)), __fdiv_rn(s.inv_qh, 4.0f));
-        P = view_pos(s, u, v, P.z);
-        radius = __fdiv_rn(__fdiv_rn(s.radius_to_screen, s.ortho ? 1.0f : P.z), 4.0f);
-        j = p.jitter_f + 4 * (oy * 4 + ox);
-        su_scale = s.inv_qw;
-        sv_scale = s.inv_qh;
-      }
-      const float step = __fdiv_rn(radius, 5.0f);
-      float ao = 0.0f;
-#pragma unroll
-      for (int d = 0; d < 8; ++d) {
-        const float dc = p.dirs[2 * d], ds = p.dirs[2 * d + 1];
-        const float dx = __fsub_rn(__fmul_rn(dc, j[0]), __fmul_rn(ds, j[1]));
-        const float dy = __fadd_rn(__fmul_rn(dc, j[1]), __fmul_rn(ds, j[0]));
-        float ray = __fadd_rn(__fmul_rn(j[2], step), 1.0f);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float kx = rintf(__fmul_rn(ray, dx)), ky = rintf(__fmul_rn(ray, dy));
-          const float su = __fadd_rn(__fmul_rn(kx, su_scale), u), sv = __fadd_rn(__fmul_rn(ky, sv_scale), v);
-          // Offsets beyond the image only select the clamped edge texel.
-          const int ix = int(fminf(fmaxf(kx, -65536.0f), 65536.0f)), iy = int(fminf(fmaxf(ky, -65536.0f), 65536.0f));
-          const float zs = CacheAware ? layer_depth(s, depth, qx + ix, qy + iy, ox, oy)
-                                      : depth_at(s, depth, x + ix, y + iy);
-          const float3 S = view_pos(s, su, sv, zs);
-          ray = __fadd_rn(ray, step);
-          const float3 V = sub(S, P);
-          const float vv = dot3(V, V);
-          const float ndotv = __fdiv_rn(dot3(N, V), __fsqrt_rn(vv));
-          ao = __fadd_rn(ao, __fmul_rn(clamp01(__fsub_rn(ndotv, p.bias)),
-                                       clamp01(__fadd_rn(__fmul_rn(vv, p.neg_inv_r2), 1.0f))));
-        }
-      }
-      ao = __fmul_rn(ao, __fdiv_rn(p.ao_mult, 32.0f));
-      const float occl = poly_pow(clamp01(__fsub_rn(1.0f, __fmul_rn(ao, 2.0f))), p.pow_exp);
-      const long long at = s.offset + (long long)y * s.pitch + x;
-      if (p.no_blur) {
-        // The cache-aware result reaches the colour through its 8-bit layers.
-        color[at] = modulate(color[at], CacheAware ? __fdiv_rn(float(unorm8(occl)), 255.0f) : occl);
-      } else if (Special) {
-        static_cast<uint32_t*>(q1)[at] = pack_half2(occl, P.z);
-      } else {
-        static_cast<uint8_t*>(q1)[at] = unorm8(occl);
-      }
+    for (int k = 0; k < 3; ++k) {
+      const uint32_t enc = unorm8(__fadd_rn(__fmul_rn(__fmul_rn(e[k], inv_len), 0.5f), 0.5f));
+      n[k] = -__fsub_rn(__fmul_rn(byte_unit(enc), 2.0f), 1.0f);
     }
+    a.N = f3(n[0], n[1], n[2]);
+    a.u = __fmul_rn(__fadd_rn(__fmul_rn(float(a.qx), 4.0f), __fadd_rn(float(a.ox), 0.5f)), __fdiv_rn(s.inv_qw, 4.0f));
+    a.v = __fmul_rn(__fadd_rn(__fmul_rn(float(a.qy), 4.0f), __fadd_rn(float(a.oy), 0.5f)), __fdiv_rn(s.inv_qh, 4.0f));
+    a.P = view_pos(s, a.u, a.v, a.P.z);
+    radius = __fdiv_rn(__fdiv_rn(s.radius_to_screen, s.ortho ? 1.0f : a.P.z), 4.0f);
+    a.su_scale = s.inv_qw;
+    a.sv_scale = s.inv_qh;
+  }
+  const float step = __fdiv_rn(radius, 5.0f);
+  float ray[4];
+  ray[0] = __fadd_rn(__fmul_rn((CacheAware ? p.jitter_f : p.jitter)[4 * jt + 2], step), 1.0f);
+#pragma unroll
+  for (int k = 1; k < 4; ++k) ray[k] = __fadd_rn(ray[k - 1], step);
+  float ao = 0.0f;
+  // Directions have components of at most 1 (and a rounding): offsets stay
+  // below 2^22, where adding 1.5 * 2^23 rounds to the nearest integer, ties
+  // to even, as rintf does.
+  if (s.fits && fabsf(ray[0]) < 2097152.0f && fabsf(ray[3]) < 2097152.0f) {
+    const float* img = depth + s.offset;
+    const int pitch = int(s.pitch);
+    constexpr float kRound = 12582912.0f;
+    constexpr int kRoundBits = 0x4B400000;
+    const int bx = (CacheAware ? a.qx : x) - kRoundBits, by = (CacheAware ? a.qy : y) - kRoundBits;
+    const int mx = (CacheAware ? s.qw : s.w) - 1, my = (CacheAware ? s.qh : s.h) - 1;
+#pragma unroll 2
+    for (int d = 0; d < 8; ++d) {
+      const float2 rot = s_rot[jt][d];
+      float su[4], sv[4], zs[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float tx = __fadd_rn(__fmul_rn(ray[k], rot.x), kRound), ty = __fadd_rn(__fmul_rn(ray[k], rot.y), kRound);
+        su[k] = __fadd_rn(__fmul_rn(__fsub_rn(tx, kRound), a.su_scale), a.u);
+        sv[k] = __fadd_rn(__fmul_rn(__fsub_rn(ty, kRound), a.sv_scale), a.v);
+        const int ix = min(max(bx + __float_as_int(tx), 0), mx), iy = min(max(by + __float_as_int(ty), 0), my);
+        if (CacheAware) {
+          const int fx = 4 * ix + a.ox, fy = 4 * iy + a.oy;
+          zs[k] = fx < s.w && fy < s.h ? __ldg(img + (fy * pitch + fx)) : 0.0f;
+        } else {
+          zs[k] = __ldg(img + (iy * pitch + ix));
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) ao = ao_sample(s, p, a, ao, su[k], sv[k], zs[k] == 0.0f ? s.far_plane : zs[k]);
+    }
+  } else {
+    ao = ao_far_samples<CacheAware>(s, depth, p, a, s_rot[jt], ray);
+  }
+  ao = __fmul_rn(ao, p.ao_scale);
+  const float occl = poly_pow(clamp01(__fsub_rn(1.0f, __fmul_rn(ao, 2.0f))), p.pow_exp);
+  const long long at = s.offset + (long long)y * s.pitch + x;
+  if (p.no_blur) {
+    // The cache-aware result reaches the colour through its 8-bit layers.
+    color[at] = modulate(color[at], CacheAware ? byte_unit(unorm8(occl)) : occl);
+  } else if (Special) {
+    static_cast<uint32_t*>(q)[at] = pack_half2(occl, a.P.z);
+  } else {
+    static_cast<uint8_t*>(q)[at] = unorm8(occl);
   }
 }
 
-// One 7-tap pass along x (axis 0) or y (axis 1).  Bilateral: 8-bit AO, the
-// depths from the linear-depth plane.  Special: (AO, depth) halves, the
-// first pass storing (blurred AO, centre depth) as halves again.
-template <int Axis, bool Special>
-__global__ void __launch_bounds__(256) hbao_blur_kernel(const HbaoScene* __restrict__ scenes, int count,
-                                                        const float* __restrict__ depth,
-                                                        const void* __restrict__ src_v, void* dst_v,
-                                                        uint32_t* color, const HbaoParams p) {
-  const float falloff = 1.0f / (2.0f * 1.5f * 1.5f);
-  const uint8_t* src8 = static_cast<const uint8_t*>(src_v);
-  const uint32_t* src32 = static_cast<const uint32_t*>(src_v);
-  {
-    const HbaoScene s = scenes[scene_of_block(scenes, count)];
-    const int pixels = s.w * s.h;
-    const int idx = (int(blockIdx.x) - s.block0) * 256 + int(threadIdx.x);
-    if (idx < pixels) {
-      const int x = idx % s.w, y = idx / s.w;
-      const long long at = s.offset + (long long)y * s.pitch + x;
-      float cd, ct;
+// Weight of the pair of taps r pixels apart whose depths differ by d.
+__device__ __forceinline__ float blur_weight(int r, float d, float sharpness) {
+  constexpr float falloff = 1.0f / (2.0f * 1.5f * 1.5f);
+  const float dd = __fmul_rn(d, sharpness);
+  const float rf = float(r);
+  return poly_exp2(__fsub_rn(__fmul_rn(__fmul_rn(-rf, rf), falloff), __fmul_rn(dd, dd)));
+}
+
+// Both 7-tap passes, x then y, and the colour multiply.  Bilateral: 8-bit AO
+// between the passes, the depths from the linear-depth plane.  Special: (AO,
+// depth) halves throughout.
+//
+// Bound by instruction issue, the exponentials of the tap weights first.  A
+// weight depends on the pair of taps alone (the depth difference enters
+// squared), so each is computed once for both: along x a lane makes the three
+// to its right and takes those to its left from the lanes there (the tile's
+// left halo from a small table); along y a thread walks four rows of its
+// column and keeps the weights in registers: 8.3 exponentials per pixel, the
+// tile's halo included, instead of 12.  One 32 x 32 tile per block with 3
+// pixels of halo, clamped at the image's edges as the taps are, so that the
+// first pass's result stays in shared memory.
+template <bool Special>
+__global__ void __launch_bounds__(256) hbao_blur_kernel(const HbaoScene* __restrict__ scenes, const HbaoScene one,
+                                                        int count, const float* __restrict__ depth,
+                                                        const void* __restrict__ q, uint32_t* color,
+                                                        const HbaoParams p) {
+  constexpr int R = 3, kSide = kBlurTile + 2 * R;
+  __shared__ float s_d[kSide][kSide + 1], s_a[kSide][kSide + 1], s_q[kSide][kBlurTile + 1], s_left[kSide][6];
+  int local = blockIdx.x;
+  const HbaoScene s = scenes ? scenes[scene_of_block<&HbaoScene::blur0>(scenes, count, &local)] : one;
+  const int tiles_x = (s.w + kBlurTile - 1) / kBlurTile;
+  const int x0 = (local % tiles_x) * kBlurTile, y0 = (local / tiles_x) * kBlurTile;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cols = min(kBlurTile, s.w - x0) + 2 * R, rows = min(kBlurTile, s.h - y0) + 2 * R;
+  for (int r = warp; r < rows; r += 8) {
+    const long long row = s.offset + (long long)min(max(y0 + r - R, 0), s.h - 1) * s.pitch;
+    for (int c = lane; c < cols; c += 32) {
+      const long long at = row + min(max(x0 + c - R, 0), s.w - 1);
       if (Special) {
-        const uint32_t c0 = src32[at];
-        ct = half_lo(c0);
-        cd = half_hi(c0);
+        const uint32_t v = __ldg(static_cast<const uint32_t*>(q) + at);
+        s_a[r][c] = half_lo(v);
+        s_d[r][c] = half_hi(v);
       } else {
-        cd = depth_at(s, depth, x, y);
-        ct = __fdiv_rn(float(src8[at]), 255.0f);
+        const float z = __ldg(depth + at);
+        s_a[r][c] = byte_unit(__ldg(static_cast<const uint8_t*>(q) + at));
+        s_d[r][c] = z == 0.0f ? s.far_plane : z;
       }
-      float wt = 1.0f;
+    }
+  }
+  __syncthreads();
+  // Weights between the left halo and the tile: pairs (c, c + r), c < 3 <= c + r.
+  for (int i = threadIdx.x; i < rows * 6; i += 256) {
+    const int row = i / 6, k = i % 6;  // k: r = 1 | r = 2, c = 1, 2 | r = 3, c = 0, 1, 2
+    const int r = k == 0 ? 1 : (k < 3 ? 2 : 3), c = k == 0 ? 2 : (k < 3 ? k : k - 3);
+    s_left[row][k] = blur_weight(r, __fsub_rn(s_d[row][c + r], s_d[row][c]), p.sharpness);
+  }
+  __syncthreads();
+  for (int row = warp; row < rows; row += 8) {
+    const int c = lane + R;
+    const float cd = s_d[row][c];
+    float w[3], ct = s_a[row][c], wt = 1.0f;
 #pragma unroll
-      for (int side = 0; side < 2; ++side) {
+    for (int r = 1; r <= 3; ++r) {
+      w[r - 1] = blur_weight(r, __fsub_rn(s_d[row][c + r], cd), p.sharpness);
+      wt = __fadd_rn(wt, w[r - 1]);
+      ct = __fadd_rn(ct, __fmul_rn(s_a[row][c + r], w[r - 1]));
+    }
 #pragma unroll
-        for (int r = 1; r <= 3; ++r) {
-          const int o = side == 0 ? r : -r;
-          const int tx = Axis == 0 ? min(max(x + o, 0), s.w - 1) : x;
-          const int ty = Axis == 1 ? min(max(y + o, 0), s.h - 1) : y;
-          const long long t_at = s.offset + (long long)ty * s.pitch + tx;
-          float c, dz;
-          if (Special) {
-            const uint32_t t = src32[t_at];
-            c = half_lo(t);
-            dz = half_hi(t);
-          } else {
-            c = __fdiv_rn(float(src8[t_at]), 255.0f);
-            dz = depth_at(s, depth, tx, ty);
-          }
-          const float dd = __fmul_rn(__fsub_rn(dz, cd), p.sharpness);
-          const float rf = float(r);
-          const float w = poly_exp2(__fsub_rn(__fmul_rn(__fmul_rn(-rf, rf), falloff), __fmul_rn(dd, dd)));
-          wt = __fadd_rn(wt, w);
-          ct = __fadd_rn(ct, __fmul_rn(c, w));
-        }
-      }
-      const float out = __fdiv_rn(ct, wt);
-      if (Axis == 0) {
-        if (Special)
-          static_cast<uint32_t*>(dst_v)[at] = pack_half2(out, cd);
-        else
-          static_cast<uint8_t*>(dst_v)[at] = unorm8(out);
-      } else {
-        color[at] = modulate(color[at], out);
-      }
+    for (int r = 1; r <= 3; ++r) {
+      const int base = r == 1 ? 0 : (r == 2 ? 1 : 3);
+      float wl = __shfl_up_sync(0xffffffffu, w[r - 1], r);
+      if (lane < r) wl = s_left[row][base + lane];
+      wt = __fadd_rn(wt, wl);
+      ct = __fadd_rn(ct, __fmul_rn(s_a[row][c - r], wl));
+    }
+    const float out = __fdiv_rn(ct, wt);
+    s_q[row][lane] = Special ? __half2float(__float2half_rn(out)) : byte_unit(unorm8(out));
+  }
+  __syncthreads();
+  const int x = x0 + lane;
+  const int first = warp * 4;  // output rows first .. first + 3 of the tile: shared rows first .. first + 9
+  if (first + 2 * R >= rows) return;
+  float d[10], a[10], w1[5], w2[6], w3[7];
+#pragma unroll
+  for (int i = 0; i < 10; ++i) {
+    const int row = min(first + i, rows - 1);
+    d[i] = s_d[row][lane + R];
+    a[i] = s_q[row][lane];
+  }
+#pragma unroll
+  for (int i = 0; i < 5; ++i) w1[i] = blur_weight(1, __fsub_rn(d[i + 3], d[i + 2]), p.sharpness);
+#pragma unroll
+  for (int i = 0; i < 6; ++i) w2[i] = blur_weight(2, __fsub_rn(d[i + 3], d[i + 1]), p.sharpness);
+#pragma unroll
+  for (int i = 0; i < 7; ++i) w3[i] = blur_weight(3, __fsub_rn(d[i + 3], d[i]), p.sharpness);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float wd[3] = {w1[i + 1], w2[i + 2], w3[i + 3]}, wu[3] = {w1[i], w2[i], w3[i]};
+    float ct = a[i + 3], wt = 1.0f;
+#pragma unroll
+    for (int r = 1; r <= 3; ++r) {
+      wt = __fadd_rn(wt, wd[r - 1]);
+      ct = __fadd_rn(ct, __fmul_rn(a[i + 3 + r], wd[r - 1]));
+    }
+#pragma unroll
+    for (int r = 1; r <= 3; ++r) {
+      wt = __fadd_rn(wt, wu[r - 1]);
+      ct = __fadd_rn(ct, __fmul_rn(a[i + 3 - r], wu[r - 1]));
+    }
+    if (x < s.w && first + i + 2 * R < rows) {
+      const long long at = s.offset + (long long)(y0 + first + i) * s.pitch + x;
+      color[at] = modulate(color[at], __fdiv_rn(ct, wt));
     }
   }
 }
 
 template <bool CacheAware, bool Special>
-void hbao_launch_t(const HbaoScene* d_scenes, int count, const dim3& grid, const float* depth, uint32_t* color,
-                   void* q1, void* q2, const HbaoParams& p, cudaStream_t stream) {
-  hbao_ao_kernel<CacheAware, Special><<<grid, 256, 0, stream>>>(d_scenes, count, depth, color, q1, p);
-  if (!p.no_blur) {
-    hbao_blur_kernel<0, Special><<<grid, 256, 0, stream>>>(d_scenes, count, depth, q1, q2, color, p);
-    hbao_blur_kernel<1, Special><<<grid, 256, 0, stream>>>(d_scenes, count, depth, q2, nullptr, color, p);
-  }
+void hbao_launch_t(const HbaoScene* d_scenes, const HbaoScene& one, int count, int ao_blocks, int blur_blocks,
+                   const float* depth, uint32_t* color, void* q, const HbaoParams& p, cudaStream_t stream) {
+  hbao_ao_kernel<CacheAware, Special><<<ao_blocks, 256, 0, stream>>>(d_scenes, one, count, depth, color, q, p);
+  if (!p.no_blur)
+    hbao_blur_kernel<Special><<<blur_blocks, 256, 0, stream>>>(d_scenes, one, count, depth, q, color, p);
 }
 
 }  // namespace
@@ -376,7 +521,8 @@ bool hbao_params(const gbr_hbao_config& c, HbaoParams& p, std::string& err) {
   p.neg_inv_r2 = -1.0f / r2;
   p.pow_exp = std::max(c.intensity, 0.0f);
   p.bias = std::min(std::max(c.bias, 0.0f), 1.0f);
-  p.ao_mult = 1.0f / (1.0f - p.bias);
+  p.bias2 = p.bias >= 1e-4f ? p.bias * p.bias * (1.0f - 1e-5f) : 0.0f;
+  p.ao_scale = 1.0f / (1.0f - p.bias) / 32.0f;
   p.sharpness = c.blur_sharpness / 1.0f;
   p.no_blur = c.no_blur ? 1 : 0;
   p.special = c.special_blur ? 1 : 0;
@@ -399,6 +545,9 @@ HbaoScene hbao_scene(const float* m, int w, int h, long long offset, long long p
   s.h = h;
   s.qw = (w + 3) / 4;
   s.qh = (h + 3) / 4;
+  s.inv_w = 1.0f / float(w);
+  s.inv_h = 1.0f / float(h);
+  s.fits = w <= 65536 && h <= 65536 && (long long)h * pitch < (1LL << 31);
   s.inv_qw = 1.0f / float(s.qw);
   s.inv_qh = 1.0f / float(s.qh);
   const float p00 = m[0], p11 = m[5], p20 = m[8], p21 = m[9], p22 = m[10], p30 = m[12], p31 = m[13],
@@ -420,21 +569,13 @@ HbaoScene hbao_scene(const float* m, int w, int h, long long offset, long long p
   return s;
 }
 
-cudaError_t hbao_launch(const HbaoScene* d_scenes, int count, int blocks, const float* depth,
-                        uint32_t* color, void* q1, void* q2, const HbaoParams& p, cudaStream_t stream) {
-  if (count <= 0 || blocks <= 0) return cudaSuccess;
-  const dim3 grid(blocks);
-  if (p.cache_aware) {
-    if (p.special)
-      hbao_launch_t<true, true>(d_scenes, count, grid, depth, color, q1, q2, p, stream);
-    else
-      hbao_launch_t<true, false>(d_scenes, count, grid, depth, color, q1, q2, p, stream);
-  } else {
-    if (p.special)
-      hbao_launch_t<false, true>(d_scenes, count, grid, depth, color, q1, q2, p, stream);
-    else
-      hbao_launch_t<false, false>(d_scenes, count, grid, depth, color, q1, q2, p, stream);
-  }
+cudaError_t hbao_launch(const HbaoScene* d_scenes, const HbaoScene& one, int count, int ao_blocks,
+                        int blur_blocks, const float* depth, uint32_t* color, void* q, const HbaoParams& p,
+                        cudaStream_t stream) {
+  if (count <= 0 || ao_blocks <= 0) return cudaSuccess;
+  const auto launch = p.cache_aware ? (p.special ? hbao_launch_t<true, true> : hbao_launch_t<true, false>)
+                                    : (p.special ? hbao_launch_t<false, true> : hbao_launch_t<false, false>);
+  launch(d_scenes, one, count, ao_blocks, blur_blocks, depth, color, q, p, stream);
   return cudaGetLastError();
 }
 
@@ -489,15 +630,13 @@ gbr_status gbr_hbao_apply(const gbr_hbao_config* config, const float projection[
   }
   const gbr::HbaoScene s = gbr::hbao_scene(projection, w, h, 0, pitch, config->radius);
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
-  gbr::HbaoScene* d_scene = nullptr;
   uint8_t* q = nullptr;
-  const size_t plane = size_t(pitch) * size_t(h) * size_t(gbr::hbao_plane_bytes(p));
-  cudaError_t e = cudaMalloc(&d_scene, sizeof s);
-  if (!e) e = cudaMalloc(&q, 2 * plane);
-  if (!e) e = cudaMemcpyAsync(d_scene, &s, sizeof s, cudaMemcpyHostToDevice, st);
-  if (!e) e = gbr::hbao_launch(d_scene, 1, int((int64_t(w) * h + 255) / 256), depth, color, q, q + plane, p, st);
+  const size_t plane = p.no_blur ? 0 : size_t(pitch) * size_t(h) * size_t(gbr::hbao_plane_bytes(p));
+  cudaError_t e = plane ? cudaMalloc(&q, plane) : cudaSuccess;
+  if (!e)
+    e = gbr::hbao_launch(nullptr, s, 1, int(gbr::hbao_blocks(w, h, gbr::kAoTile)),
+                         int(gbr::hbao_blocks(w, h, gbr::kBlurTile)), depth, color, q, p, st);
   if (!e) e = cudaStreamSynchronize(st);
-  cudaFree(d_scene);
   cudaFree(q);
   if (e) {
     gbr::set_last_error(std::string("Hbao: ") + cudaGetErrorString(e));

@@ -19,13 +19,22 @@ struct HbaoScene {
   float radius_to_screen;
   float far_plane;   // depth given to background pixels (linear depth 0)
   int ortho;
-  int block0;        // first block of the scene in the launch grid (256 pixels per block)
+  int block0, blur0; // first block of the scene in the AO and in the blur grid
   int qw, qh;        // quarter resolution of the cache-aware algorithm: ceil(w / 4) x ceil(h / 4)
   float inv_qw, inv_qh;  // 1 / qw, 1 / qh
+  float inv_w, inv_h;    // 1 / w, 1 / h
+  int fits;          // w, h <= 65536 and h * pitch < 2^31: 32-bit texel arithmetic is exact
 };
 
+// One block of the AO grid covers kAoTile x kAoTile pixels of a scene, one of
+// the blur grid kBlurTile x kBlurTile.
+constexpr int kAoTile = 16, kBlurTile = 32;
+inline long long hbao_blocks(int w, int h, int tile) {
+  return ((w + tile - 1LL) / tile) * ((h + tile - 1LL) / tile);
+}
+
 struct HbaoParams {
-  float neg_inv_r2, bias, ao_mult, pow_exp, sharpness;
+  float neg_inv_r2, bias, bias2, ao_scale, pow_exp, sharpness;  // bias2: see hbao_ao_kernel
   int no_blur;
   int special;       // AO and view depth kept as two halves per pixel, blurred with that depth
   int cache_aware;   // the deinterleaved algorithm
@@ -40,14 +49,16 @@ bool hbao_params(const gbr_hbao_config& c, HbaoParams& p, std::string& err);
 // Per-image constants from a column-major projection (Hbao.cpp:761-786, 874-895).
 HbaoScene hbao_scene(const float* projection, int w, int h, long long offset, long long pitch,
                      float radius);
-// Bytes per pixel of each of the two intermediate planes: an 8-bit AO, or
-// with the special blur an (AO, view depth) pair of halves.
+// Bytes per pixel of the intermediate plane: an 8-bit AO, or with the special
+// blur an (AO, view depth) pair of halves.
 inline int hbao_plane_bytes(const HbaoParams& p) { return p.special ? 4 : 1; }
-// Three launches on `stream`: AO (into q1, or straight into colour without
-// blur), blur along x (q1 -> q2), blur along y and the colour multiply.
-// q1 / q2 have the colour plane's layout, hbao_plane_bytes(p) per pixel.
-cudaError_t hbao_launch(const HbaoScene* d_scenes, int count, int blocks, const float* depth,
-                        uint32_t* color, void* q1, void* q2, const HbaoParams& p,
+// Two launches on `stream`: AO (into q, or straight into colour without
+// blur), then both blur passes and the colour multiply.  q has the colour
+// plane's layout, hbao_plane_bytes(p) per pixel.  The scenes are read from
+// device memory, or with count 1 and d_scenes null from `one`; ao_blocks and
+// blur_blocks are the sums of hbao_blocks() over them.
+cudaError_t hbao_launch(const HbaoScene* d_scenes, const HbaoScene& one, int count, int ao_blocks,
+                        int blur_blocks, const float* depth, uint32_t* color, void* q, const HbaoParams& p,
                         cudaStream_t stream);
 
 }  // namespace gbr

@@ -1635,7 +1635,7 @@ gbr_status Renderer::image_into_async(uint32_t plane, const int32_t* rect, void*
 }
 
 // Hbao::drawEffect, classic (src/esp/gfx_batch/Hbao.cpp:874-935), over all
-// enabled scenes at once (three launches, csrc/hbao.cu).
+// enabled scenes at once (two launches, csrc/hbao.cu).
 gbr_status Renderer::hbao(const gbr_hbao_config& c, cudaStream_t stream) {
   TraceRange trace_("gbr.hbao");
   if (!(cfg_.planes & GBR_PLANE_COLOR) || !(cfg_.planes & GBR_PLANE_LINEAR_DEPTH))
@@ -1644,18 +1644,20 @@ gbr_status Renderer::hbao(const gbr_hbao_config& c, cudaStream_t stream) {
   std::string err;
   if (!hbao_params(c, params, err)) return fail(GBR_ERROR_INVALID_ARGUMENT, err);
   std::vector<HbaoScene> recs;
-  long long blocks = 0;  // one per 256 pixels of each scene
+  long long blocks = 0, blur_blocks = 0;
   for (const SceneState& sc : scenes_) {
     if (!sc.enabled || sc.width <= 0 || sc.height <= 0) continue;
     recs.push_back(hbao_scene(sc.proj, sc.width, sc.height, sc.fb_offset, sc.pitch, c.radius));
     recs.back().block0 = int(blocks);
-    blocks += (static_cast<long long>(sc.width) * sc.height + 255) / 256;
+    recs.back().blur0 = int(blur_blocks);
+    blocks += hbao_blocks(sc.width, sc.height, kAoTile);
+    blur_blocks += hbao_blocks(sc.width, sc.height, kBlurTile);
   }
   if (blocks > 0x7fffffffLL) return fail(GBR_ERROR_INVALID_ARGUMENT, "Hbao: too many pixels in one call");
   if (recs.empty()) return GBR_OK;
   cudaSetDevice(device_);
   const size_t fb = size_t(fb_w_) * size_t(fb_h_) * size_t(hbao_plane_bytes(params));
-  if (!d_hbao_scenes_.reserve(recs.size() * sizeof(HbaoScene), false) || !d_hbao_ao_.reserve(2 * fb, false))
+  if (!d_hbao_scenes_.reserve(recs.size() * sizeof(HbaoScene), false) || !d_hbao_ao_.reserve(fb, false))
     return fail(GBR_ERROR_OUT_OF_MEMORY, "Hbao: device allocation failed");
   if (upload_pending_[slot_])  // after the last draw, whatever stream it ran on
     GBR_CUDA(cudaStreamWaitEvent(stream, upload_done_[slot_], 0), "Hbao: wait for draw");
@@ -1666,8 +1668,8 @@ gbr_status Renderer::hbao(const gbr_hbao_config& c, cudaStream_t stream) {
   uint32_t* color = static_cast<uint32_t*>(plane_ptr(GBR_PLANE_COLOR, &elem));
   const float* depth = static_cast<const float*>(plane_ptr(GBR_PLANE_LINEAR_DEPTH, &elem));
   uint8_t* q = static_cast<uint8_t*>(d_hbao_ao_.ptr);
-  GBR_CUDA(hbao_launch(d_hbao_scenes_.as<HbaoScene>(), int(recs.size()), int(blocks), depth, color, q, q + fb,
-                       params, stream),
+  GBR_CUDA(hbao_launch(d_hbao_scenes_.as<HbaoScene>(), recs[0], int(recs.size()), int(blocks), int(blur_blocks),
+                       depth, color, q, params, stream),
            "Hbao launch");
   // Readbacks of this draw now follow the effect.
   GBR_CUDA(cudaEventRecord(upload_done_[slot_], stream), "Hbao: event");

@@ -219,7 +219,7 @@ class Renderer {
   DeviceBuffer d_spill_;  // raster queue spill area, per resident CTA
   DeviceBuffer d_spill_owner_;  // per-scene form: owners of its slots (zero between draws)
   DeviceBuffer d_gather_;  // packed scenes on their way to host memory
-  DeviceBuffer d_hbao_scenes_, d_hbao_ao_;  // ambient occlusion: per-scene records, two 8-bit planes
+  DeviceBuffer d_hbao_scenes_, d_hbao_ao_;  // ambient occlusion: per-scene records, the AO plane
   uint32_t max_lights_ = 0;
   DeviceBuffer d_meshes_, d_materials_, d_textures_, d_boxes_;
   DeviceBuffer d_scenes_, d_parents_, d_local_, d_draws_, d_cameras_;
