@@ -37,6 +37,41 @@ void set_last_error(const std::string& msg);
 
 namespace {
 
+// Two floats in a register pair: an addition of pairs is one instruction and
+// rounds each half as the scalar one does.  Products are left to two scalar
+// instructions, also where a pair's would do: the assembler contracts a pair's
+// multiplication and addition into one fused operation whatever their rounding
+// modifiers and flags say, and a fused result is another number.  (fma2 is for where
+// that is wanted.)
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ F2 f2(float a) { return f2(a, a); }
+__device__ __forceinline__ float2 split(F2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  const float2 x = split(a), y = split(b);
+  return f2(__fmul_rn(x.x, y.x), __fmul_rn(x.y, y.y));
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
 __device__ __forceinline__ float poly_exp2(float x) {
   if (x < -149.0f) return 0.0f;
   const float n = floorf(x);
@@ -55,6 +90,27 @@ __device__ __forceinline__ float poly_exp2(float x) {
   // the first product is exact, the second rounds once, into the denormals.
   const int k = int(n), k1 = max(k, -126);
   return __fmul_rn(__fmul_rn(p, __int_as_float((k1 + 127) << 23)), __int_as_float((k - k1 + 127) << 23));
+}
+
+// poly_exp2 of both halves.
+__device__ __forceinline__ float2 poly_exp2(F2 x2) {
+  const float2 x = split(x2);
+  const float n0 = floorf(x.x), n1 = floorf(x.y);
+  const F2 f = add2(x2, f2(-n0, -n1));
+  F2 p = f2(1.0178086284895471e-07f);
+  p = add2(mul2(p, f), f2(1.3215486660556053e-06f));
+  p = add2(mul2(p, f), f2(1.5252733646775596e-05f));
+  p = add2(mul2(p, f), f2(0.0001540352968731895f));
+  p = add2(mul2(p, f), f2(0.0013333557872101665f));
+  p = add2(mul2(p, f), f2(0.009618128649890423f));
+  p = add2(mul2(p, f), f2(0.05550410971045494f));
+  p = add2(mul2(p, f), f2(0.24022650718688965f));
+  p = add2(mul2(p, f), f2(0.6931471824645996f));
+  p = add2(mul2(p, f), f2(1.0f));
+  const int k0 = int(n0), k1 = int(n1), m0 = max(k0, -126), m1 = max(k1, -126);
+  p = mul2(p, f2(__int_as_float((m0 + 127) << 23), __int_as_float((m1 + 127) << 23)));
+  const float2 r = split(mul2(p, f2(__int_as_float((k0 - m0 + 127) << 23), __int_as_float((k1 - m1 + 127) << 23))));
+  return make_float2(x.x < -149.0f ? 0.0f : r.x, x.y < -149.0f ? 0.0f : r.y);
 }
 
 __device__ __forceinline__ float poly_log2(float x) {
@@ -77,6 +133,13 @@ __device__ __forceinline__ float poly_log2(float x) {
 __device__ __forceinline__ float poly_pow(float a, float e) {
   if (!(a > 0.0f)) return e == 0.0f ? 1.0f : 0.0f;
   return poly_exp2(__fmul_rn(e, poly_log2(a)));
+}
+
+// Relative error at most 2^-22.9.
+__device__ __forceinline__ float rsqrt_approx(float a) {
+  float r;
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
 }
 
 __device__ __forceinline__ float clamp01(float v) { return fminf(fmaxf(v, 0.0f), 1.0f); }
@@ -191,17 +254,11 @@ __device__ __forceinline__ float half_hi(uint32_t v) { return __half2float(__ush
 struct AoPixel {
   float3 P, N;
   float u, v, su_scale, sv_scale;
-  int x, y, qx, qy, ox, oy;
+  int x, y;
 };
 
-// The AO that a sample at (su, sv) with depth zs adds.
-__device__ __forceinline__ float ao_sample(const HbaoScene& s, const HbaoParams& p, const AoPixel& a, float ao,
-                                           float su, float sv, float zs) {
-  const float3 S = view_pos(s, su, sv, zs);
-  const float3 V = sub(S, a.P);
-  const float vv = dot3(V, V);
-  const float fall = __fadd_rn(__fmul_rn(vv, p.neg_inv_r2), 1.0f);
-  const float nv = dot3(a.N, V);
+// Adds a sample's AO: squared distance vv, N.V nv, and the falloff at vv.
+__device__ __forceinline__ float ao_add(const HbaoParams& p, float ao, float vv, float nv, float fall) {
   // Most samples add exactly nothing and leave before the square root and the
   // division: beyond the radius (fall <= 0 or not a number), behind the
   // tangent plane, or below the bias: N.V / |V| < bias, decided on squares
@@ -212,23 +269,33 @@ __device__ __forceinline__ float ao_sample(const HbaoScene& s, const HbaoParams&
   return __fadd_rn(ao, __fmul_rn(clamp01(__fsub_rn(ndotv, p.bias)), clamp01(fall)));
 }
 
-// All samples of a pixel whose steps or image are too large for the 32-bit
-// texel arithmetic of hbao_ao_kernel.
+// The AO of lane `src`'s pixel as the specification has it, by the whole warp:
+// for pixels whose steps or image are too large for the 32-bit texel
+// arithmetic of hbao_ao_kernel, and for those whose estimate does not decide
+// the result.  Lane i takes sample i (direction i / 4, step i % 4); the sum is
+// in that order.
 template <bool CacheAware>
-__device__ __noinline__ float ao_far_samples(const HbaoScene& s, const float* __restrict__ depth,
-                                             const HbaoParams& p, const AoPixel& a, const float2* rot,
-                                             const float* ray) {
+__device__ __forceinline__ float ao_by_warp(const HbaoScene& s, const float* __restrict__ depth, const HbaoParams& p,
+                                            const AoPixel& mine, const float ray[4], const float2 (*rot)[8], int src) {
+  const auto get = [&](float v) { return __shfl_sync(0xffffffffu, v, src); };
+  const int lane = threadIdx.x & 31, k = lane & 3;
+  const float3 P = f3(get(mine.P.x), get(mine.P.y), get(mine.P.z)), N = f3(get(mine.N.x), get(mine.N.y), get(mine.N.z));
+  const float u = get(mine.u), v = get(mine.v), r0 = get(ray[0]), r1 = get(ray[1]), r2 = get(ray[2]), r3 = get(ray[3]);
+  const int x = __shfl_sync(0xffffffffu, mine.x, src), y = __shfl_sync(0xffffffffu, mine.y, src);
+  const float r = k == 0 ? r0 : (k == 1 ? r1 : (k == 2 ? r2 : r3));
+  const float2 d = rot[(y & 3) * 4 + (x & 3)][lane >> 2];
+  const float kx = rintf(__fmul_rn(r, d.x)), ky = rintf(__fmul_rn(r, d.y));
+  const float su = __fadd_rn(__fmul_rn(kx, mine.su_scale), u), sv = __fadd_rn(__fmul_rn(ky, mine.sv_scale), v);
+  // Offsets beyond the image only select the clamped edge texel.
+  const int ix = int(fminf(fmaxf(kx, -65536.0f), 65536.0f)), iy = int(fminf(fmaxf(ky, -65536.0f), 65536.0f));
+  const float zs = CacheAware ? layer_depth(s, depth, (x >> 2) + ix, (y >> 2) + iy, x & 3, y & 3)
+                              : depth_at(s, depth, x + ix, y + iy);
+  const float3 V = sub(view_pos(s, su, sv, zs), P);
+  const float vv = dot3(V, V);
+  const float c = ao_add(p, 0.0f, vv, dot3(N, V), __fadd_rn(__fmul_rn(vv, p.neg_inv_r2), 1.0f));
   float ao = 0.0f;
-  for (int d = 0; d < 8; ++d)
-    for (int k = 0; k < 4; ++k) {
-      const float kx = rintf(__fmul_rn(ray[k], rot[d].x)), ky = rintf(__fmul_rn(ray[k], rot[d].y));
-      const float su = __fadd_rn(__fmul_rn(kx, a.su_scale), a.u), sv = __fadd_rn(__fmul_rn(ky, a.sv_scale), a.v);
-      // Offsets beyond the image only select the clamped edge texel.
-      const int ix = int(fminf(fmaxf(kx, -65536.0f), 65536.0f)), iy = int(fminf(fmaxf(ky, -65536.0f), 65536.0f));
-      const float zs = CacheAware ? layer_depth(s, depth, a.qx + ix, a.qy + iy, a.ox, a.oy)
-                                  : depth_at(s, depth, a.x + ix, a.y + iy);
-      ao = ao_sample(s, p, a, ao, su, sv, zs);
-    }
+  for (uint32_t m = __ballot_sync(0xffffffffu, c != 0.0f); m; m &= m - 1u)
+    ao = __fadd_rn(ao, __shfl_sync(0xffffffffu, c, __ffs(int(m)) - 1));
   return ao;
 }
 
@@ -248,11 +315,17 @@ __device__ __noinline__ float ao_far_samples(const HbaoScene& s, const float* __
 // table, the four ray lengths are shared by the eight directions, a sample's
 // offset is rounded to an integer by adding 1.5 * 2^23 (which leaves the
 // integer in the low bits: no conversion instructions, a quarter of the rate
-// here), texels are addressed in 32 bits, and ao_sample leaves early.
+// here), texels are addressed in 32 bits, and two samples of a direction go
+// through the float arithmetic as register pairs.  Where the result is a byte,
+// a sample's N.V / |V| is first taken with the approximate reciprocal root (2
+// instructions for about 30), the error of the sum is bounded, and the few
+// pixels whose byte the bound leaves open (one in 500) are done again in full, a
+// warp to a pixel; with halves (Special) it would leave one in 50 open, so every
+// sample is done in full.
 template <bool CacheAware, bool Special>
-__global__ void __launch_bounds__(256) hbao_ao_kernel(const HbaoScene* __restrict__ scenes, const HbaoScene one,
-                                                      int count, const float* __restrict__ depth, uint32_t* color,
-                                                      void* q, const HbaoParams p) {
+__global__ void __launch_bounds__(256, 5)
+    hbao_ao_kernel(const HbaoScene* __restrict__ scenes, const __grid_constant__ HbaoScene one, int count,
+                   const float* __restrict__ depth, uint32_t* color, void* q, const __grid_constant__ HbaoParams p) {
   __shared__ float2 s_rot[16][8];  // rotated directions of jitter texel j
   if (threadIdx.x < 128) {
     const int t = threadIdx.x >> 3, d = threadIdx.x & 7;
@@ -262,17 +335,18 @@ __global__ void __launch_bounds__(256) hbao_ao_kernel(const HbaoScene* __restric
                               __fadd_rn(__fmul_rn(dc, j[1]), __fmul_rn(ds, j[0])));
   }
   int local = blockIdx.x;
-  HbaoScene s;
-  if (scenes) {
-    s = scenes[scene_of_block<&HbaoScene::block0>(scenes, count, &local)];
-  } else {
-    s = one;
+  const HbaoScene* scene = &one;
+  if (scenes)
+    scene = scenes + scene_of_block<&HbaoScene::block0>(scenes, count, &local);
+  else
     __syncthreads();
-  }
+  const HbaoScene s = *scene;
   const int tiles_x = (s.w + kAoTile - 1) / kAoTile;
-  const int x = (local % tiles_x) * kAoTile + (int(threadIdx.x) & (kAoTile - 1));
-  const int y = (local / tiles_x) * kAoTile + int(threadIdx.x) / kAoTile;
-  if (x >= s.w || y >= s.h) return;
+  int x = (local % tiles_x) * kAoTile + (int(threadIdx.x) & (kAoTile - 1));
+  int y = (local / tiles_x) * kAoTile + int(threadIdx.x) / kAoTile;
+  const bool valid = x < s.w && y < s.h;  // the others stay for the warp's sake, at an edge pixel
+  x = min(x, s.w - 1);
+  y = min(y, s.h - 1);
   AoPixel a;
   a.x = x;
   a.y = y;
@@ -284,11 +358,7 @@ __global__ void __launch_bounds__(256) hbao_ao_kernel(const HbaoScene* __restric
   float radius;
   a.su_scale = s.inv_w;
   a.sv_scale = s.inv_h;
-  a.ox = x & 3;
-  a.oy = y & 3;
-  a.qx = x >> 2;
-  a.qy = y >> 2;
-  const int jt = a.oy * 4 + a.ox;
+  const int ox = x & 3, oy = y & 3, qx = x >> 2, qy = y >> 2, jt = oy * 4 + ox;
   if (!CacheAware) {
     a.N = f3(-__fmul_rn(c.x, inv_len), -__fmul_rn(c.y, inv_len), -__fmul_rn(c.z, inv_len));
     radius = __fdiv_rn(s.radius_to_screen, s.ortho ? 1.0f : a.P.z);
@@ -301,8 +371,8 @@ __global__ void __launch_bounds__(256) hbao_ao_kernel(const HbaoScene* __restric
       n[k] = -__fsub_rn(__fmul_rn(byte_unit(enc), 2.0f), 1.0f);
     }
     a.N = f3(n[0], n[1], n[2]);
-    a.u = __fmul_rn(__fadd_rn(__fmul_rn(float(a.qx), 4.0f), __fadd_rn(float(a.ox), 0.5f)), __fdiv_rn(s.inv_qw, 4.0f));
-    a.v = __fmul_rn(__fadd_rn(__fmul_rn(float(a.qy), 4.0f), __fadd_rn(float(a.oy), 0.5f)), __fdiv_rn(s.inv_qh, 4.0f));
+    a.u = __fmul_rn(__fadd_rn(__fmul_rn(float(qx), 4.0f), __fadd_rn(float(ox), 0.5f)), __fdiv_rn(s.inv_qw, 4.0f));
+    a.v = __fmul_rn(__fadd_rn(__fmul_rn(float(qy), 4.0f), __fadd_rn(float(oy), 0.5f)), __fdiv_rn(s.inv_qh, 4.0f));
     a.P = view_pos(s, a.u, a.v, a.P.z);
     radius = __fdiv_rn(__fdiv_rn(s.radius_to_screen, s.ortho ? 1.0f : a.P.z), 4.0f);
     a.su_scale = s.inv_qw;
@@ -317,48 +387,105 @@ __global__ void __launch_bounds__(256) hbao_ao_kernel(const HbaoScene* __restric
   // Directions have components of at most 1 (and a rounding): offsets stay
   // below 2^22, where adding 1.5 * 2^23 rounds to the nearest integer, ties
   // to even, as rintf does.
-  if (s.fits && fabsf(ray[0]) < 2097152.0f && fabsf(ray[3]) < 2097152.0f) {
+  const bool near = s.fits && fabsf(ray[0]) < 2097152.0f && fabsf(ray[3]) < 2097152.0f;
+  const bool estimated = near && !Special;
+  if (near) {
     const float* img = depth + s.offset;
     const int pitch = int(s.pitch);
     constexpr float kRound = 12582912.0f;
     constexpr int kRoundBits = 0x4B400000;
-    const int bx = (CacheAware ? a.qx : x) - kRoundBits, by = (CacheAware ? a.qy : y) - kRoundBits;
+    const int bx = (CacheAware ? qx : x) - kRoundBits, by = (CacheAware ? qy : y) - kRoundBits;
     const int mx = (CacheAware ? s.qw : s.w) - 1, my = (CacheAware ? s.qh : s.h) - 1;
+    const F2 round = f2(kRound), unround = f2(-kRound), su_scale = f2(a.su_scale), sv_scale = f2(a.sv_scale),
+             u2 = f2(a.u), v2 = f2(a.v), pi0 = f2(s.pi[0]), pi1 = f2(s.pi[1]), pi2 = f2(s.pi[2]), pi3 = f2(s.pi[3]),
+             px = f2(-a.P.x), py = f2(-a.P.y), pz = f2(-a.P.z), nx = f2(a.N.x), ny = f2(a.N.y), nz = f2(a.N.z),
+             falloff = f2(p.neg_inv_r2), unit = f2(1.0f);
+    const F2 rays[2] = {f2(ray[0], ray[1]), f2(ray[2], ray[3])};
+    const auto texel = [&](float tx, float ty) {
+      const int ix = min(max(bx + __float_as_int(tx), 0), mx), iy = min(max(by + __float_as_int(ty), 0), my);
+      float z;
+      if (CacheAware) {
+        const int fx = 4 * ix + ox, fy = 4 * iy + oy;
+        z = fx < s.w && fy < s.h ? __ldg(img + (fy * pitch + fx)) : 0.0f;
+      } else {
+        z = __ldg(img + (iy * pitch + ix));
+      }
+      return z == 0.0f ? s.far_plane : z;
+    };
 #pragma unroll 2
     for (int d = 0; d < 8; ++d) {
       const float2 rot = s_rot[jt][d];
-      float su[4], sv[4], zs[4];
+      const F2 rx = f2(rot.x), ry = f2(rot.y);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float tx = __fadd_rn(__fmul_rn(ray[k], rot.x), kRound), ty = __fadd_rn(__fmul_rn(ray[k], rot.y), kRound);
-        su[k] = __fadd_rn(__fmul_rn(__fsub_rn(tx, kRound), a.su_scale), a.u);
-        sv[k] = __fadd_rn(__fmul_rn(__fsub_rn(ty, kRound), a.sv_scale), a.v);
-        const int ix = min(max(bx + __float_as_int(tx), 0), mx), iy = min(max(by + __float_as_int(ty), 0), my);
-        if (CacheAware) {
-          const int fx = 4 * ix + a.ox, fy = 4 * iy + a.oy;
-          zs[k] = fx < s.w && fy < s.h ? __ldg(img + (fy * pitch + fx)) : 0.0f;
+      for (int k = 0; k < 2; ++k) {
+        const F2 tx = add2(mul2(rays[k], rx), round), ty = add2(mul2(rays[k], ry), round);
+        const float2 sx = split(tx), sy = split(ty);
+        const F2 z = f2(texel(sx.x, sy.x), texel(sx.y, sy.y));
+        const F2 zk = s.ortho ? unit : z;
+        const F2 su = add2(mul2(add2(tx, unround), su_scale), u2), sv = add2(mul2(add2(ty, unround), sv_scale), v2);
+        const F2 Vx = add2(mul2(add2(mul2(su, pi0), pi2), zk), px), Vy = add2(mul2(add2(mul2(sv, pi1), pi3), zk), py),
+                 Vz = add2(z, pz);
+        if (Special) {
+          const F2 vv = add2(add2(mul2(Vx, Vx), mul2(Vy, Vy)), mul2(Vz, Vz));
+          const F2 nv = add2(add2(mul2(nx, Vx), mul2(ny, Vy)), mul2(nz, Vz));
+          const float2 l = split(vv), n = split(nv), f = split(add2(mul2(vv, falloff), unit));
+          ao = ao_add(p, ao, l.x, n.x, f.x);
+          ao = ao_add(p, ao, l.y, n.y, f.y);
         } else {
-          zs[k] = __ldg(img + (iy * pitch + ix));
+          const float2 l = split(fma2(Vz, Vz, fma2(Vy, Vy, mul2(Vx, Vx))));
+          const F2 nv = fma2(nz, Vz, fma2(ny, Vy, mul2(nx, Vx)));
+          const float2 n = split(mul2(nv, f2(rsqrt_approx(l.x), rsqrt_approx(l.y))));
+          ao = __fmaf_rn(__saturatef(n.x - p.bias), __saturatef(__fmaf_rn(l.x, p.neg_inv_r2, 1.0f)), ao);
+          ao = __fmaf_rn(__saturatef(n.y - p.bias), __saturatef(__fmaf_rn(l.y, p.neg_inv_r2, 1.0f)), ao);
         }
       }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) ao = ao_sample(s, p, a, ao, su[k], sv[k], zs[k] == 0.0f ? s.far_plane : zs[k]);
     }
-  } else {
-    ao = ao_far_samples<CacheAware>(s, depth, p, a, s_rot[jt], ray);
   }
-  ao = __fmul_rn(ao, p.ao_scale);
-  const float occl = poly_pow(clamp01(__fsub_rn(1.0f, __fmul_rn(ao, 2.0f))), p.pow_exp);
+  // A byte result (or three, without the blur) is decided by the occlusion at
+  // both ends of the estimate's error unless they round differently.  Per
+  // sample the estimate is off by at most 8e-7: N.V / |V| by 5 roundings of
+  // products of at most |N| |V| on either side (6e-7), the reciprocal root's
+  // 2^-22.9 and as much for the falloff's; the sum by 2 x 32 roundings of at
+  // most 2^-24 of it; poly_pow by less than 2e-7 and 1.2e-7 of the exponent.
   const long long at = s.offset + (long long)y * s.pitch + x;
-  if (p.no_blur) {
-    // The cache-aware result reaches the colour through its 8-bit layers.
-    color[at] = modulate(color[at], CacheAware ? byte_unit(unorm8(occl)) : occl);
-  } else if (Special) {
-    static_cast<uint32_t*>(q)[at] = pack_half2(occl, a.P.z);
-  } else {
-    static_cast<uint8_t*>(q)[at] = unorm8(occl);
+  const bool byte_plane = !Special && (!p.no_blur || CacheAware);  // the result is a byte first
+  bool open = !near;
+  uint32_t result = 0;
+  if (estimated) {
+    const float est = 1.0f - 2.0f * p.ao_scale * ao;
+    const float err = 2.0f * p.ao_scale * (2.6e-5f + 5e-6f * ao) + 4e-7f, slack = 5e-7f + 3e-7f * p.pow_exp;
+    const float lo = poly_pow(clamp01(est - err), p.pow_exp) - slack, hi = poly_pow(clamp01(est + err), p.pow_exp) + slack;
+    if (byte_plane) {
+      result = unorm8(lo);
+      open = result != unorm8(hi);
+    } else {
+      const uint32_t old = color[at];
+      result = modulate(old, lo);
+      open = result != modulate(old, hi);
+    }
   }
+  for (uint32_t m = __ballot_sync(0xffffffffu, open && valid); m; m &= m - 1u) {
+    const int src = __ffs(int(m)) - 1;
+    const float v = ao_by_warp<CacheAware>(s, depth, p, a, ray, s_rot, src);
+    if ((int(threadIdx.x) & 31) == src) ao = v;
+  }
+  if (!valid) return;
+  if (open || !estimated) {
+    const float occl = poly_pow(clamp01(__fsub_rn(1.0f, __fmul_rn(__fmul_rn(ao, p.ao_scale), 2.0f))), p.pow_exp);
+    if (Special)
+      result = pack_half2(occl, a.P.z);
+    else
+      result = byte_plane ? unorm8(occl) : modulate(color[at], occl);
+  }
+  if (p.no_blur)  // the cache-aware result reaches the colour through its 8-bit layers
+    color[at] = CacheAware ? modulate(color[at], byte_unit(result)) : result;
+  else if (Special)
+    static_cast<uint32_t*>(q)[at] = result;
+  else
+    static_cast<uint8_t*>(q)[at] = uint8_t(result);
 }
+
+constexpr int kBlurThreads = 512;
 
 // Weight of the pair of taps r pixels apart whose depths differ by d.
 __device__ __forceinline__ float blur_weight(int r, float d, float sharpness) {
@@ -366,6 +493,15 @@ __device__ __forceinline__ float blur_weight(int r, float d, float sharpness) {
   const float dd = __fmul_rn(d, sharpness);
   const float rf = float(r);
   return poly_exp2(__fsub_rn(__fmul_rn(__fmul_rn(-rf, rf), falloff), __fmul_rn(dd, dd)));
+}
+
+// Both weights at once: taps ra and rb pixels apart, depths differing by a and b.
+__device__ __forceinline__ float2 blur_weights(int ra, int rb, float a, float b, float sharpness) {
+  constexpr float falloff = 1.0f / (2.0f * 1.5f * 1.5f);
+  const F2 d = f2(a, b), up = mul2(d, f2(sharpness)), down = mul2(d, f2(-sharpness));
+  const float fa = float(ra), fb = float(rb);
+  return poly_exp2(add2(f2(__fmul_rn(__fmul_rn(-fa, fa), falloff), __fmul_rn(__fmul_rn(-fb, fb), falloff)),
+                        mul2(up, down)));
 }
 
 // Both 7-tap passes, x then y, and the colour multiply.  Bilateral: 8-bit AO
@@ -376,25 +512,29 @@ __device__ __forceinline__ float blur_weight(int r, float d, float sharpness) {
 // weight depends on the pair of taps alone (the depth difference enters
 // squared), so each is computed once for both: along x a lane makes the three
 // to its right and takes those to its left from the lanes there (the tile's
-// left halo from a small table); along y a thread walks four rows of its
-// column and keeps the weights in registers: 8.3 exponentials per pixel, the
-// tile's halo included, instead of 12.  One 32 x 32 tile per block with 3
+// left halo from a small table); along y the weights of a row with the three
+// rows above it go through shared memory: 7.3 exponentials per pixel, the
+// tile's halo included, instead of 12, two at a time.  One 32 x 32 tile per block with 3
 // pixels of halo, clamped at the image's edges as the taps are, so that the
-// first pass's result stays in shared memory.
+// first pass's result stays in shared memory; 512 threads, because one image
+// is a few hundred tiles and the rows of a tile are what hides latency.
 template <bool Special>
-__global__ void __launch_bounds__(256) hbao_blur_kernel(const HbaoScene* __restrict__ scenes, const HbaoScene one,
-                                                        int count, const float* __restrict__ depth,
-                                                        const void* __restrict__ q, uint32_t* color,
-                                                        const HbaoParams p) {
-  constexpr int R = 3, kSide = kBlurTile + 2 * R;
+__global__ void __launch_bounds__(kBlurThreads, 4)
+    hbao_blur_kernel(const HbaoScene* __restrict__ scenes, const __grid_constant__ HbaoScene one, int count,
+                     const float* __restrict__ depth, const void* __restrict__ q, uint32_t* color,
+                     const __grid_constant__ HbaoParams p) {
+  constexpr int R = 3, kSide = kBlurTile + 2 * R, kWarps = kBlurThreads / 32;
   __shared__ float s_d[kSide][kSide + 1], s_a[kSide][kSide + 1], s_q[kSide][kBlurTile + 1], s_left[kSide][6];
+  __shared__ float s_w[R][kSide][kBlurTile];  // weight of rows (t, t + r): s_w[r - 1][t]
   int local = blockIdx.x;
-  const HbaoScene s = scenes ? scenes[scene_of_block<&HbaoScene::blur0>(scenes, count, &local)] : one;
+  const HbaoScene* scene = &one;
+  if (scenes) scene = scenes + scene_of_block<&HbaoScene::blur0>(scenes, count, &local);
+  const HbaoScene s = *scene;
   const int tiles_x = (s.w + kBlurTile - 1) / kBlurTile;
   const int x0 = (local % tiles_x) * kBlurTile, y0 = (local / tiles_x) * kBlurTile;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int cols = min(kBlurTile, s.w - x0) + 2 * R, rows = min(kBlurTile, s.h - y0) + 2 * R;
-  for (int r = warp; r < rows; r += 8) {
+  for (int r = warp; r < rows; r += kWarps) {
     const long long row = s.offset + (long long)min(max(y0 + r - R, 0), s.h - 1) * s.pitch;
     for (int c = lane; c < cols; c += 32) {
       const long long at = row + min(max(x0 + c - R, 0), s.w - 1);
@@ -411,19 +551,29 @@ __global__ void __launch_bounds__(256) hbao_blur_kernel(const HbaoScene* __restr
   }
   __syncthreads();
   // Weights between the left halo and the tile: pairs (c, c + r), c < 3 <= c + r.
-  for (int i = threadIdx.x; i < rows * 6; i += 256) {
+  for (int i = threadIdx.x; i < rows * 6; i += kBlurThreads) {
     const int row = i / 6, k = i % 6;  // k: r = 1 | r = 2, c = 1, 2 | r = 3, c = 0, 1, 2
     const int r = k == 0 ? 1 : (k < 3 ? 2 : 3), c = k == 0 ? 2 : (k < 3 ? k : k - 3);
     s_left[row][k] = blur_weight(r, __fsub_rn(s_d[row][c + r], s_d[row][c]), p.sharpness);
   }
   __syncthreads();
-  for (int row = warp; row < rows; row += 8) {
+  for (int row = warp; row < rows; row += kWarps) {
     const int c = lane + R;
     const float cd = s_d[row][c];
-    float w[3], ct = s_a[row][c], wt = 1.0f;
+    // Below the tile's last row the depth is that row's: its weights go unused.
+    const float* down = &s_d[0][c];
+    const float d1 = down[min(row + 1, rows - 1) * (kSide + 1)], d2 = down[min(row + 2, rows - 1) * (kSide + 1)],
+                d3 = down[min(row + 3, rows - 1) * (kSide + 1)];
+    const float2 w12 = blur_weights(1, 2, __fsub_rn(s_d[row][c + 1], cd), __fsub_rn(s_d[row][c + 2], cd), p.sharpness),
+                 w3d = blur_weights(3, 1, __fsub_rn(s_d[row][c + 3], cd), __fsub_rn(d1, cd), p.sharpness),
+                 d23 = blur_weights(2, 3, __fsub_rn(d2, cd), __fsub_rn(d3, cd), p.sharpness);
+    s_w[0][row][lane] = w3d.y;
+    s_w[1][row][lane] = d23.x;
+    s_w[2][row][lane] = d23.y;
+    const float w[3] = {w12.x, w12.y, w3d.x};
+    float ct = s_a[row][c], wt = 1.0f;
 #pragma unroll
     for (int r = 1; r <= 3; ++r) {
-      w[r - 1] = blur_weight(r, __fsub_rn(s_d[row][c + r], cd), p.sharpness);
       wt = __fadd_rn(wt, w[r - 1]);
       ct = __fadd_rn(ct, __fmul_rn(s_a[row][c + r], w[r - 1]));
     }
@@ -440,39 +590,23 @@ __global__ void __launch_bounds__(256) hbao_blur_kernel(const HbaoScene* __restr
   }
   __syncthreads();
   const int x = x0 + lane;
-  const int first = warp * 4;  // output rows first .. first + 3 of the tile: shared rows first .. first + 9
-  if (first + 2 * R >= rows) return;
-  float d[10], a[10], w1[5], w2[6], w3[7];
-#pragma unroll
-  for (int i = 0; i < 10; ++i) {
-    const int row = min(first + i, rows - 1);
-    d[i] = s_d[row][lane + R];
-    a[i] = s_q[row][lane];
-  }
-#pragma unroll
-  for (int i = 0; i < 5; ++i) w1[i] = blur_weight(1, __fsub_rn(d[i + 3], d[i + 2]), p.sharpness);
-#pragma unroll
-  for (int i = 0; i < 6; ++i) w2[i] = blur_weight(2, __fsub_rn(d[i + 3], d[i + 1]), p.sharpness);
-#pragma unroll
-  for (int i = 0; i < 7; ++i) w3[i] = blur_weight(3, __fsub_rn(d[i + 3], d[i]), p.sharpness);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float wd[3] = {w1[i + 1], w2[i + 2], w3[i + 3]}, wu[3] = {w1[i], w2[i], w3[i]};
-    float ct = a[i + 3], wt = 1.0f;
+  if (x >= s.w) return;
+  for (int row = warp + R; row < rows - R; row += kWarps) {
+    float ct = s_q[row][lane], wt = 1.0f;
 #pragma unroll
     for (int r = 1; r <= 3; ++r) {
-      wt = __fadd_rn(wt, wd[r - 1]);
-      ct = __fadd_rn(ct, __fmul_rn(a[i + 3 + r], wd[r - 1]));
+      const float w = s_w[r - 1][row][lane];
+      wt = __fadd_rn(wt, w);
+      ct = __fadd_rn(ct, __fmul_rn(s_q[row + r][lane], w));
     }
 #pragma unroll
     for (int r = 1; r <= 3; ++r) {
-      wt = __fadd_rn(wt, wu[r - 1]);
-      ct = __fadd_rn(ct, __fmul_rn(a[i + 3 - r], wu[r - 1]));
+      const float w = s_w[r - 1][row - r][lane];
+      wt = __fadd_rn(wt, w);
+      ct = __fadd_rn(ct, __fmul_rn(s_q[row - r][lane], w));
     }
-    if (x < s.w && first + i + 2 * R < rows) {
-      const long long at = s.offset + (long long)(y0 + first + i) * s.pitch + x;
-      color[at] = modulate(color[at], __fdiv_rn(ct, wt));
-    }
+    const long long at = s.offset + (long long)(y0 + row - R) * s.pitch + x;
+    color[at] = modulate(color[at], __fdiv_rn(ct, wt));
   }
 }
 
@@ -481,7 +615,7 @@ void hbao_launch_t(const HbaoScene* d_scenes, const HbaoScene& one, int count, i
                    const float* depth, uint32_t* color, void* q, const HbaoParams& p, cudaStream_t stream) {
   hbao_ao_kernel<CacheAware, Special><<<ao_blocks, 256, 0, stream>>>(d_scenes, one, count, depth, color, q, p);
   if (!p.no_blur)
-    hbao_blur_kernel<Special><<<blur_blocks, 256, 0, stream>>>(d_scenes, one, count, depth, q, color, p);
+    hbao_blur_kernel<Special><<<blur_blocks, kBlurThreads, 0, stream>>>(d_scenes, one, count, depth, q, color, p);
 }
 
 }  // namespace

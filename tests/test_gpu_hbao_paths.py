@@ -64,3 +64,11 @@ def test_offsets_beyond_the_image_and_beyond_32_bits(pkg, radius, cache_aware):
                                 dict(intensity=60.0), dict(blur_sharpness=0.0), dict(blur_sharpness=400.0)])
 def test_parameters(pkg, kw):
     check(pkg, 37, 45, **kw)
+
+
+@pytest.mark.parametrize("variant", [{}, {"special_blur": True}, {"cache_aware": True, "special_blur": True}],
+                         ids=["classic", "special", "cache_special"])
+def test_camera_image(pkg, variant):
+    """A whole 640 x 480 image: a single operation that rounds otherwise (a
+    fused one, say) changes a handful of its 307,200 pixels."""
+    check(pkg, 480, 640, **variant)
