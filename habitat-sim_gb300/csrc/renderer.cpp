@@ -1058,7 +1058,8 @@ void Renderer::choose_shape() {
       ItemScene it;
       it.width = sc.width;
       it.height = sc.height;
-      it.tris = scenes_[sc.source].tris;
+      it.tris = scenes_[sc.source].drawn;
+      it.draws = scenes_[sc.source].draw_count;
       uint64_t n, cost;
       split_cost(it, r[0], r[1], 0, n, cost);
       items += n;
@@ -1135,6 +1136,7 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
     cost[s] = tris;
     sc.draw_count = r.draw_count;
     sc.tris = tris;
+    sc.drawn = drawn_tris(tris, max_tris);
   }
   total_nodes_ = nodes;
   total_draws_ = uint32_t(draws.size());
@@ -1364,7 +1366,8 @@ void Renderer::order_items() {
     ItemScene& it = info[s];
     it.width = sc.width;
     it.height = sc.height;
-    it.tris = src.tris;
+    it.tris = src.drawn;
+    it.draws = src.draw_count;
     it.enabled = sc.enabled;
     // Geometry of the source: the mesh of its largest draw.
     uint32_t best = 0;

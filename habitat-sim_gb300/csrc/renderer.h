@@ -88,6 +88,7 @@ struct SceneState {
   uint32_t node_base = 0;  // in the flattened device arrays
   uint32_t draw_count = 0; // draws in the flattened device arrays (at the last rebuild)
   uint64_t tris = 0;       // triangles of those draws
+  uint64_t drawn = 0;      // drawn_tris() of them
   uint32_t source = 0;     // scene whose nodes and draws this scene renders
   uint32_t vis_base = 0;   // first visible record (from the current bindings)
   bool enabled = true;

@@ -15,14 +15,15 @@ namespace gbr {
 // What the ordering needs to know of a scene.
 struct ItemScene {
   int width = 0, height = 0;  // viewport
-  uint64_t tris = 0;          // triangles of the scene it renders (its source)
+  uint64_t tris = 0;          // drawn_tris() of the scene it renders (its source)
   uint32_t geometry = 0;      // groups items of equal cost (the mesh of the source's largest draw)
   bool enabled = true;
+  uint32_t draws = 0;         // draws of that scene
 };
 
 // Region halvings a costly scene's items may get, and the most when the
 // whole step has fewer items than the grid has CTAs.
-constexpr int kMaxSplits = 2;
+constexpr int kMaxSplits = 4;
 constexpr int kMaxFewSplits = 6;
 
 // Region of a scene's items after `level` splits of the batched form's
@@ -42,24 +43,31 @@ inline void split_region(int width, int height, int region_w, int region_h, int 
   }
 }
 
-// Estimated cost of a w x h region of a W x H viewport, in triangles drawn:
-// half of its share of the scene's (the rest is out of view), a twentieth of
-// them for the region's culling, 6000 for the phases that every region goes
-// through, and four per pixel for rasterising and shading it.  (One 128 x 128
-// view of a furnished room, 500k triangles: 83 us for a 16 x 32 region, 96 for
-// 32 x 32, 119 for 64 x 32, about 160 for 64 x 64; of a bare room, 49k
-// triangles: 34, 42 and 47 us.)
-inline uint64_t item_cost(uint64_t tris, int w, int h, int W, int H) {
+// Triangles that a view of a scene draws, for item_cost: a camera sees most of
+// a large draw around it, but few of many small draws.
+inline uint64_t drawn_tris(uint64_t tris, uint64_t largest_draw) {
+  return (26 * largest_draw + 7 * (tris - largest_draw)) / 20;
+}
+
+// Estimated cost of a w x h region of a W x H viewport in nanoseconds of a
+// 512-thread CTA, two per SM: its share of the drawn triangles, 7 per pixel for
+// rasterising and shading it, 18000 for the phases that every region goes
+// through, a fiftieth of the triangles and 100 per draw for culling the scene.
+// Fitted to the mean item of eight scene sets at five region sizes (bare and
+// furnished rooms, scans, lit rooms; 128 x 64 to 16 x 32): within 10 % except
+// lit rooms (half).
+inline uint64_t item_cost(uint64_t tris, int w, int h, int W, int H, uint32_t draws = 0) {
   const uint64_t px = uint64_t(w) * uint64_t(h);
-  return tris * px / (2 * uint64_t(W) * uint64_t(H)) + tris / 20 + 6000 + 4 * px;
+  return tris * px / (uint64_t(W) * uint64_t(H)) + 7 * px + 18000 + tris / 50 + 100 * uint64_t(draws);
 }
 
 // Estimated time of `items` items of total cost `total`, the largest costing
-// `largest`, on `grid` CTAs.  Items of equal estimate differ by half of it
-// either way: a single wave ends with its longest; in more waves the last
-// one, of halved items (build_work_items), overlaps the rest.
+// `largest`, on `grid` CTAs, longest first: one wave ends with its longest item,
+// several with a mean one.  The longest of equal estimates takes 2.5 times that
+// (the views of a step differ that much).
 inline double step_cost(uint64_t items, double total, double largest, uint64_t grid) {
-  return items <= grid ? 1.4 * largest : total / double(grid) + 0.8 * largest;
+  if (items <= grid) return 2.5 * largest;
+  return std::max(2.5 * largest, total / double(grid) + 2.5 * total / double(items));
 }
 
 // Items of one scene split `level` times and the cost of the largest.
@@ -67,7 +75,7 @@ inline void split_cost(const ItemScene& sc, int region_w, int region_h, int leve
   int rw, rh;
   split_region(sc.width, sc.height, region_w, region_h, level, rw, rh);
   items = uint64_t((sc.width + rw - 1) / rw) * uint64_t((sc.height + rh - 1) / rh);
-  cost = item_cost(sc.tris, rw, rh, sc.width, sc.height);
+  cost = item_cost(sc.tris, rw, rh, sc.width, sc.height, sc.draws);
 }
 
 // Items the list can ever hold: every scene at its finest split, plus the
@@ -124,7 +132,7 @@ inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scen
   uint64_t best_limit = limit;
   for (int most : {kMaxSplits, kMaxFewSplits}) {
     uint64_t t = limit;
-    for (int i = 0; i < 14 && t > 0; ++i, t = t * 7 / 10) {
+    for (int i = 0; i < 28 && t > 0; ++i, t = t * 17 / 20) {
       uint64_t items = 0, total = 0, largest = 0;
       bool few = false;
       for (uint32_t s = 0; s < S; ++s) {
@@ -162,7 +170,7 @@ inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scen
         it.w = uint16_t(std::min(rw, sc.width - x));
         it.h = uint16_t(std::min(rh, sc.height - y));
         items.push_back(it);
-        cost.push_back(item_cost(sc.tris, it.w, it.h, sc.width, sc.height));
+        cost.push_back(item_cost(sc.tris, it.w, it.h, sc.width, sc.height, sc.draws));
         key.push_back(sc.geometry);
       }
   }
@@ -191,8 +199,8 @@ inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scen
       }
       const ItemScene& sc = scenes[it.scene];
       const uint32_t geometry = key[perm[i]];
-      cost[perm[i]] = item_cost(sc.tris, it.w, it.h, sc.width, sc.height);
-      const uint64_t bcost = item_cost(sc.tris, b.w, b.h, sc.width, sc.height);
+      cost[perm[i]] = item_cost(sc.tris, it.w, it.h, sc.width, sc.height, sc.draws);
+      const uint64_t bcost = item_cost(sc.tris, b.w, b.h, sc.width, sc.height, sc.draws);
       items.push_back(b);  // `it` is not used past this point
       cost.push_back(bcost);
       key.push_back(geometry);
