@@ -55,12 +55,49 @@ __host__ __device__ inline void philox4x32_10(uint32_t c[4], uint32_t k0, uint32
   }
 }
 
-__device__ __forceinline__ float normal_variate(uint32_t bits, const float* __restrict__ table) {
+// What a block keeps in shared memory for a batch large enough to repay it:
+// the quantile function's segments as (value, rise), the output of each small
+// quantised disparity, and the model cell of each column and row of an image
+// (premultiplied; all images of a tile grid have one size).
+constexpr int kSegments = kKnots - 1, kOutputs = 1024, kCells = 4096;
+struct Tables {
+  float2 normal[kSegments];
+  float out[kOutputs];
+  uint16_t cell[kCells];  // columns, then rows
+};
+
+template <bool Table>
+__device__ __forceinline__ float normal_variate(uint32_t bits, const float* __restrict__ table, const Tables* t) {
   const uint32_t u = bits >> 8;
   const uint32_t k = u >> 12;
-  const float f = __fmul_rn(float(u & 4095u), 1.0f / 4096.0f);
+  // The fraction (u & 4095) / 4096, exactly, from the mantissa of [1, 2).
+  const float f = __fsub_rn(__uint_as_float(0x3f800000u | ((u & 4095u) << 11)), 1.0f);
+  if (Table) {
+    const float2 seg = t->normal[k];
+    return __fadd_rn(seg.x, __fmul_rn(f, seg.y));
+  }
   const float t0 = __ldg(table + k), t1 = __ldg(table + k + 1);
   return __fadd_rn(t0, __fmul_rn(f, __fsub_rn(t1, t0)));
+}
+
+// n / d for n < 2^31 (Granlund and Montgomery, "Division by invariant integers
+// using multiplication", PLDI 1994).
+struct Divisor {
+  uint32_t d, m, s1, s2;
+  __device__ __forceinline__ uint32_t divide(uint32_t n) const {
+    const uint32_t t = __umulhi(m, n);
+    return (t + ((n - t) >> s1)) >> s2;
+  }
+};
+Divisor make_divisor(uint32_t d) {
+  uint32_t l = 0;
+  while ((uint64_t(1) << l) < d) ++l;
+  Divisor v;
+  v.d = d;
+  v.m = uint32_t((uint64_t(1) << 32) * ((uint64_t(1) << l) - d) / d + 1);
+  v.s1 = std::min(l, 1u);
+  v.s2 = l > 0 ? l - 1 : 0;
+  return v;
 }
 
 struct TileArgs {
@@ -74,16 +111,31 @@ struct TileArgs {
   uint32_t key0, key1, call0, call1;
 };
 
-// One output pixel (row-major index idx) of image img, whose top-left pixel
-// is src / dst with `pitch` floats per row and tw x th pixels.
-__device__ __forceinline__ void noise_pixel(const TileArgs& a, int img, int idx, const float* src, float* dst,
-                                            long long pitch, int tw, int th) {
+// Model cell of column x (remapped to 640) and of row y (to 480): offsets into
+// the table (a 1-pixel axis maps to 0).
+__device__ __forceinline__ uint32_t cell_of_column(int x, float xmax) {
+  const int ux = xmax > 0.0f ? int(__fadd_rn(__fmul_rn(__fdiv_rn(float(x), xmax), 639.0f), 0.5f)) : 0;
+  return uint32_t(ux / 8) * kModelDims;
+}
+__device__ __forceinline__ uint32_t cell_of_row(int y, float ymax) {
+  const int uy = ymax > 0.0f ? int(__fadd_rn(__fmul_rn(__fdiv_rn(float(y), ymax), 479.0f), 0.5f)) : 0;
+  return uint32_t(uy / 6) * kModelCols * kModelDims;
+}
+
+__device__ __forceinline__ float output_of(float denom) {
+  return denom > 1e-5f ? __fdiv_rn(35.130f * 8.0f, denom) : 0.0f;
+}
+
+// One output pixel (row r, column col: row-major index idx) of image img, whose
+// top-left pixel is src / dst with `pitch` floats per row and tw x th pixels.
+template <bool Table>
+__device__ __forceinline__ void noise_pixel(const TileArgs& a, int img, int idx, int r, int col, const float* src,
+                                            float* dst, long long pitch, int tw, int th, const Tables* t, bool cells) {
   const float ymax = float(th - 1), xmax = float(tw - 1);
   uint32_t c[4] = {uint32_t(idx), uint32_t(img), a.call0, a.call1};
   philox4x32_10(c, a.key0, a.key1);
-  const float n0 = normal_variate(c[0], a.table), n1 = normal_variate(c[1], a.table),
-              n2 = normal_variate(c[2], a.table);
-  const int r = idx / tw, col = idx % tw;
+  const float n0 = normal_variate<Table>(c[0], a.table, t), n1 = normal_variate<Table>(c[1], a.table, t),
+              n2 = normal_variate<Table>(c[2], a.table, t);
   const int y = int(__fadd_rn(fminf(fmaxf(__fadd_rn(float(r), __fmul_rn(__fmul_rn(n0, 0.25f), a.mult)),
                                           0.0f),
                                     ymax),
@@ -92,54 +144,86 @@ __device__ __forceinline__ void noise_pixel(const TileArgs& a, int img, int idx,
                                           0.0f),
                                     xmax),
                               0.5f));
-  const float d = src[(long long)(y - y % 2) * pitch + (x - x % 2)];
+  const float d = src[uint64_t(uint32_t(y & ~1)) * uint64_t(pitch) + uint32_t(x & ~1)];
   float out = 0.0f;
   if (!(d >= 10.0f)) {
-    // Remap to the model's 640 x 480 sensor (a 1-pixel axis maps to 0).
-    const int ux = xmax > 0.0f ? int(__fadd_rn(__fmul_rn(__fdiv_rn(float(x), xmax), 639.0f), 0.5f)) : 0;
-    const int uy = ymax > 0.0f ? int(__fadd_rn(__fmul_rn(__fdiv_rn(float(y), ymax), 479.0f), 0.5f)) : 0;
+    const uint32_t at = Table && cells ? uint32_t(t->cell[x]) + t->cell[tw + y] : cell_of_column(x, xmax) + cell_of_row(y, ymax);
     // v / 2 and v * 0.5 are the same correctly rounded value.
     const int i2 = int(__fmul_rn(__fadd_rn(d, 1.0f), 0.5f));
     const int i1 = i2 - 1;
     const float w = __fmul_rn(__fsub_rn(d, __fadd_rn(__fmul_rn(float(i1), 2.0f), 1.0f)), 0.5f);
-    const float* cell = a.model + ((uy / 6) * kModelCols + ux / 8) * kModelDims;
+    const float* cell = a.model + at;
     // Bins clamped to 0..4 (the reference clamps the upper bin only from
     // above: equal for every depth >= 0).
     const float f = __fadd_rn(__fmul_rn(__fsub_rn(1.0f, w), __ldg(cell + min(max(i1, 0), 4))),
                               __fmul_rn(w, __ldg(cell + min(max(i2, 0), 4))));
-    const float ud = f < 1e-5f ? 0.0f : __fdiv_rn(d, f);
-    if (ud != 0.0f) {
-      // round((35.130 / d' + noise) * 8) is defined in double.  The float
-      // evaluation differs from it by less than `margin` (three roundings
-      // of at most 2^-24 relative each), so it rounds to the same integer
-      // unless it lies within the margin of a half; only those pixels
-      // take the double path (FP64 throughput is low on this part).
-      const float nz = __fmul_rn(__fmul_rn(n2, 0.027778f), a.mult);
-      const float inv = __fdiv_rn(35.130f, ud);
-      const float qf = __fmul_rn(__fadd_rn(inv, nz), 8.0f);
-      const float margin = __fmul_rn(1e-6f, __fadd_rn(fabsf(qf), __fmul_rn(8.0f, fabsf(nz))));
-      const float frac = fabsf(__fsub_rn(qf, truncf(qf)));
-      float denom;
-      if (fabsf(__fsub_rn(frac, 0.5f)) > margin && isfinite(qf)) {
-        denom = roundf(qf);
-      } else {
+    const float nz = __fmul_rn(__fmul_rn(n2, 0.027778f), a.mult);
+    // round((35.130 / d' + noise) * 8) with d' = d / f rounded, in double.  A
+    // float estimate with an approximate reciprocal (2^-23) and four roundings
+    // (2^-24) differs from it by less than `margin`, so it rounds to the same
+    // integer unless it lies within the margin of a half: those pixels, and
+    // values outside the estimate's range, take the double path (FP64
+    // throughput is low on this part).
+    float rcp;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(rcp) : "f"(d));
+    const float qf = __fmul_rn(__fmaf_rn(__fmul_rn(35.130f, f), rcp, nz), 8.0f);
+    const float margin = __fmul_rn(1e-6f, __fadd_rn(fabsf(qf), __fmul_rn(8.0f, fabsf(nz))));
+    const float half = __fadd_rn(qf, 0.5f);
+    const float off = __fsub_rn(half, floorf(half));  // distance of qf above the last half
+    if (f >= 1e-5f && d > 1e-30f && qf > 1.0f && qf < float(kOutputs - 2) && off > margin && off < 1.0f - margin) {
+      const int denom = int(half);
+      out = Table ? t->out[denom] : output_of(float(denom));
+    } else {
+      const float ud = f < 1e-5f ? 0.0f : __fdiv_rn(d, f);
+      if (ud != 0.0f) {
         const double q = (double(35.130f) / double(ud) + double(nz)) * 8.0;
-        denom = float(round(q));
+        out = output_of(float(round(q)));
       }
-      out = denom > 1e-5f ? __fdiv_rn(35.130f * 8.0f, denom) : 0.0f;
     }
   }
-  dst[(long long)r * pitch + col] = out;
+  dst[uint64_t(uint32_t(r)) * uint64_t(pitch) + uint32_t(col)] = out;
 }
 
-// Images as the tiles of a grid: blockIdx.y walks images, x their pixels.
-__global__ void __launch_bounds__(256) redwood_kernel(TileArgs a) {
+// Images as the tiles of a grid, cut into chunks of pixels that the blocks
+// walk: unit u is chunk u % chunks of image u / chunks.
+//
+// Bound by instruction issue (73 %, 211 instructions per 32 pixels): Philox' ten
+// rounds and what the arithmetic above fixes.  With Table, blocks of 1024
+// threads, two per SM, first fill 44 KB of shared memory with what would be
+// gathers from L1 (28 lines per warp and variate), two divisions per pixel for
+// the model's cell and one for the output; filling it takes a few microseconds,
+// so only batches of kTablePixels and more do (64 images of 128 x 128: 14.4 us
+// against 16.5 without; 32: 11.7 against 10.3; 1024: 130 against 203).
+constexpr int kTableThreads = 1024, kPlainThreads = 256;
+constexpr uint64_t kTablePixels = 1u << 20;
+template <bool Table>
+__global__ void __launch_bounds__(Table ? kTableThreads : kPlainThreads, Table ? 2 : 8)
+    redwood_kernel(const TileArgs a, const Divisor width, const Divisor chunks, uint32_t units, int chunk) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  Tables* t = reinterpret_cast<Tables*>(smem);
+  constexpr int kThreads = Table ? kTableThreads : kPlainThreads;
+  const bool cells = a.tw <= kCells && a.th <= kCells - a.tw;
+  if (Table) {
+    for (int k = threadIdx.x; k < kSegments; k += kThreads) {
+      const float t0 = __ldg(a.table + k);
+      t->normal[k] = make_float2(t0, __fsub_rn(__ldg(a.table + k + 1), t0));
+    }
+    for (int k = threadIdx.x; k < kOutputs; k += kThreads) t->out[k] = output_of(float(k));
+    if (cells)
+      for (int k = threadIdx.x; k < a.tw + a.th; k += kThreads)
+        t->cell[k] = uint16_t(k < a.tw ? cell_of_column(k, float(a.tw - 1)) : cell_of_row(k - a.tw, float(a.th - 1)));
+    __syncthreads();
+  }
   const int pixels = a.tw * a.th;
-  for (int img = blockIdx.y; img < a.count; img += gridDim.y) {
-    const long long base =
-        (long long)(img / a.tiles_x) * a.th * a.pitch + (long long)(img % a.tiles_x) * a.tw;
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < pixels; idx += gridDim.x * blockDim.x)
-      noise_pixel(a, img, idx, a.src + base, a.dst + base, a.pitch, a.tw, a.th);
+  for (uint32_t u = blockIdx.x; u < units; u += gridDim.x) {
+    const uint32_t img = chunks.divide(u);
+    const long long base = (long long)(img / a.tiles_x) * a.th * a.pitch + (long long)(img % a.tiles_x) * a.tw;
+    const long long first = (long long)(u - img * chunks.d) * chunk;
+    for (int k = threadIdx.x; k < chunk; k += kThreads) {
+      if (first + k >= pixels) break;
+      const int idx = int(first) + k, r = int(width.divide(uint32_t(idx)));
+      noise_pixel<Table>(a, int(img), idx, r, idx - r * a.tw, a.src + base, a.dst + base, a.pitch, a.tw, a.th, t, cells);
+    }
   }
 }
 
@@ -166,7 +250,8 @@ __global__ void __launch_bounds__(256) redwood_images_kernel(TileArgs a, const l
   const long long base = layout[4 * img], pitch = layout[4 * img + 1];
   const int tw = int(layout[4 * img + 2]), th = int(layout[4 * img + 3]);
   const int idx = int((long long)blockIdx.x - blocks[img]) * 256 + int(threadIdx.x);
-  if (idx < tw * th) noise_pixel(a, img, idx, a.src + base, a.dst + base, pitch, tw, th);
+  if (idx < tw * th)
+    noise_pixel<false>(a, img, idx, idx / tw, idx % tw, a.src + base, a.dst + base, pitch, tw, th, nullptr, false);
 }
 
 // Standard normal quantile in double: Halley steps on erfc from the
@@ -262,11 +347,22 @@ TileArgs make_args(gbr_redwood_noise* m, const float* src, float* dst, long long
 
 gbr_status launch(gbr_redwood_noise* m, const float* src, float* dst, long long pitch, int tw, int th,
                   int tiles_x, int count, cudaStream_t stream) {
+  const uint64_t pixels = uint64_t(tw) * uint64_t(th), total = pixels * uint64_t(count);
+  const bool table = total >= kTablePixels;
+  // Chunks of four pixels per thread where that leaves every block several.
+  const uint64_t chunk = !table ? kPlainThreads : kTableThreads * (total >= 4 * kTablePixels ? 4 : 1), chunks = (pixels + chunk - 1) / chunk;
+  const uint64_t units = chunks * uint64_t(count);
+  if (units > 0xffffffffull)
+    return fail(GBR_ERROR_INVALID_ARGUMENT, "RedwoodNoiseModel: too many pixels in one batch");
   const TileArgs a = make_args(m, src, dst, pitch, tw, th, tiles_x, count);
-  const int pixels = tw * th;
-  const int per_image = std::max(1, std::min((pixels + 255) / 256, 8 * m->sms));
-  const int images = std::max(1, std::min(count, 65535));
-  redwood_kernel<<<dim3(per_image, images), 256, 0, stream>>>(a);
+  const Divisor width = make_divisor(uint32_t(tw)), per_image = make_divisor(uint32_t(chunks));
+  const unsigned resident = unsigned(2 * m->sms);
+  if (table)
+    redwood_kernel<true><<<unsigned(std::min<uint64_t>(units, resident)), kTableThreads, sizeof(Tables), stream>>>(
+        a, width, per_image, uint32_t(units), int(chunk));
+  else
+    redwood_kernel<false><<<unsigned(std::min<uint64_t>(units, 0x7fffffffu)), kPlainThreads, 0, stream>>>(
+        a, width, per_image, uint32_t(units), int(chunk));
   if (cudaError_t e = cudaGetLastError()) return cuda_fail(e, "redwood noise launch");
   return GBR_OK;
 }
