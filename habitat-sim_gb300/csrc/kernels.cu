@@ -418,31 +418,28 @@ struct QEntry {
   int16_t x0, y0, x1, y1;
 };
 
-// Dynamic shared-memory layout of raster_kernel; every section starts on a
-// 16-byte boundary.
-struct SmemLayout {
-  size_t queue, qoff, prefix, chunks, clusters, tiles, coarse, total;
-};
-
 // Depth tiles of the occlusion test: kTile x kTile pixels of the region,
 // and coarse tiles of kCoarse x kCoarse tiles.
 constexpr int kTile = 8, kCoarse = 4;
-__host__ __device__ __forceinline__ int tile_capacity(int region_px, int side) {
-  // ceil(w / s) * ceil(h / s) <= w h / s^2 + (w + h) / s + 1 with w, h <= 1024
-  return region_px / (side * side) + 2 * 1024 / side + 1;
+__host__ __device__ __forceinline__ int tile_capacity(int w, int h, int side) {
+  return ((w + side - 1) / side) * ((h + side - 1) / side);
 }
-__host__ __device__ __forceinline__ size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
-__host__ __device__ __forceinline__ SmemLayout smem_layout(int threads, int region_px,
-                                                           int prefix_cap) {
+// Entries of the shared triangle queue.  With 352 of them two 512-thread CTAs
+// on 128 x 64 regions need 196 KB of shared memory and leave 60 KB to the L1
+// cache (with 512: 228 and 28), through which the vertices, boxes and records
+// are read.
+__host__ __device__ constexpr int queue_capacity(int threads) { return threads * 11 / 16; }
+uint32_t align16(size_t x) { return uint32_t((x + 15) & ~size_t(15)); }
+SmemLayout smem_layout(int threads, int region_w, int region_h, int prefix_cap) {
   SmemLayout l;
-  l.queue = align16(size_t(region_px) * 8);
-  l.qoff = align16(l.queue + size_t(threads) * sizeof(QEntry));
-  l.prefix = align16(l.qoff + size_t(threads + 1) * 4);
-  l.chunks = align16(l.prefix + size_t(prefix_cap + 1) * 4);
+  l.queue = align16(size_t(region_w) * size_t(region_h) * 8);
+  l.qoff = align16(l.queue + size_t(queue_capacity(threads)) * sizeof(QEntry));
+  l.prefix = align16(l.qoff + size_t(queue_capacity(threads) + 1) * 4);
+  l.chunks = align16(l.prefix + size_t(prefix_cap) * 4);
   l.clusters = align16(l.chunks + size_t(ring_capacity(threads)) * sizeof(uint2));
   l.tiles = align16(l.clusters + size_t(kClusterRing) * sizeof(uint2));
-  l.coarse = align16(l.tiles + size_t(tile_capacity(region_px, kTile)) * 4);
-  l.total = align16(l.coarse + size_t(tile_capacity(region_px, kTile * kCoarse)) * 4);
+  l.coarse = align16(l.tiles + size_t(tile_capacity(region_w, region_h, kTile)) * 4);
+  l.total = align16(l.coarse + size_t(tile_capacity(region_w, region_h, kTile * kCoarse)) * 4);
   return l;
 }
 
@@ -457,9 +454,9 @@ struct Setup {
 struct Ctx {
   uint64_t* keys;
   QEntry* queue;
-  QEntry* spill;  // this CTA's global spill area (qcap more entries), or null
+  QEntry* spill;  // this CTA's global spill area (spill_cap more entries), or null
   uint32_t* qcount;
-  int qcap;
+  int qcap, spill_cap;
   int rx0, ry0, rw, rh;  // region
   int W, H;              // viewport
   int small_area;
@@ -621,7 +618,7 @@ __device__ __forceinline__ void emit(const float4* q, uint32_t ordinal, const Ct
       store_entry(c.queue[slot], st, ordinal);
       return;
     }
-    if (c.spill && slot < 2u * uint32_t(c.qcap)) {
+    if (c.spill && slot < uint32_t(c.qcap + c.spill_cap)) {
       store_entry(c.spill[slot - c.qcap], st, ordinal);
       return;
     }
@@ -1271,9 +1268,11 @@ __device__ __forceinline__ bool chunk_keep(const float* mvp, const ChunkBox& b, 
 }
 
 template <int T, bool Lod>
-__global__ void __launch_bounds__(T, 1024 / T) raster_kernel(const RasterParams p) {
+__global__ void __launch_bounds__(T, 1024 / T)
+    raster_kernel(const __grid_constant__ RasterParams p, const __grid_constant__ SmemLayout layout) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const SmemLayout L = smem_layout(T, p.region_px, p.prefix_cap);
+  // The offsets come from the launch: constants that need no registers.
+  const SmemLayout& L = layout;
   uint64_t* keys = reinterpret_cast<uint64_t*>(smem);
   QEntry* queue = reinterpret_cast<QEntry*>(smem + L.queue);
   uint32_t* qoff = reinterpret_cast<uint32_t*>(smem + L.qoff);
@@ -1282,6 +1281,7 @@ __global__ void __launch_bounds__(T, 1024 / T) raster_kernel(const RasterParams 
   uint2* cring = reinterpret_cast<uint2*>(smem + L.clusters);
   uint32_t* tiles = reinterpret_cast<uint32_t*>(smem + L.tiles);
   uint32_t* coarse = reinterpret_cast<uint32_t*>(smem + L.coarse);
+  __shared__ uint32_t s_moved;  // entries of the spill area already moved into the queue
   __shared__ uint32_t s_item, s_qcount, s_total, s_rd, s_wr, s_crd, s_cwr, s_next;
   __shared__ uint32_t s_warp[T / 32];
   __shared__ QEntry* s_spill;
@@ -1323,7 +1323,9 @@ __global__ void __launch_bounds__(T, 1024 / T) raster_kernel(const RasterParams 
     c.queue = queue;
     c.spill = s_spill;
     c.qcount = &s_qcount;
-    c.qcap = T;
+    constexpr uint32_t kQueue = queue_capacity(T);
+    c.qcap = kQueue;
+    c.spill_cap = T;
     c.rx0 = wi.x0;
     c.ry0 = wi.y0;
     c.rw = wi.w;
@@ -1340,7 +1342,7 @@ __global__ void __launch_bounds__(T, 1024 / T) raster_kernel(const RasterParams 
     const bool cached = shift == kOrdinalRunning && nvis <= uint32_t(p.prefix_cap);
     if (cached)
       for (uint32_t i = threadIdx.x; i < nvis; i += T) prefix[i] = vis[i].ordinal;
-    if (threadIdx.x == 0) s_qcount = 0;
+    if (threadIdx.x == 0) s_qcount = s_moved = 0;
     __syncthreads();
 
     // Clusters (1024 triangles) and chunks (32 triangles) of the visible
@@ -1374,13 +1376,13 @@ __global__ void __launch_bounds__(T, 1024 / T) raster_kernel(const RasterParams 
     __syncthreads();
     for (;;) {
       const uint32_t rd = s_rd, wr = s_wr, crd = s_crd, cwr = s_cwr, next = s_next,
-                     queued = min(s_qcount, uint32_t(c.spill ? 2 * T : T)),
-                     nq = min(queued, uint32_t(T));
+                     queued = min(s_qcount, c.spill ? kQueue + uint32_t(T) : kQueue),
+                     nq = min(queued, kQueue);
       __syncthreads();  // everyone has read the counters
       const bool low = wr - rd < uint32_t(T / 32);
       const bool clusters_left = next < nclusters, have_clusters = cwr != crd;
       const bool need_cull = low && (clusters_left || have_clusters);
-      // A round adds at most T entries to fewer than flush_at <= T: the queue and the
+      // A round adds at most T entries to fewer than flush_at: the queue and the
       // spill area (T each) hold them.
       if (nq > 0 && (nq >= p.flush_at || need_cull || wr == rd)) {
         // ---- flush: every thread takes a contiguous run of the queued
@@ -1434,8 +1436,14 @@ __global__ void __launch_bounds__(T, 1024 / T) raster_kernel(const RasterParams 
         if (queued > nq) {
           // A round queued more than the shared queue holds: the rest went to
           // this CTA's spill area; move it into the emptied queue.
-          for (uint32_t i = threadIdx.x; i < queued - nq; i += T) queue[i] = c.spill[i];
-          if (threadIdx.x == 0) s_qcount = queued - nq;
+          // (What does not fit follows at the next flush, which comes at once.)
+          const uint32_t rest = queued - nq, moved = min(rest, kQueue), from = s_moved;
+          for (uint32_t i = threadIdx.x; i < moved; i += T) queue[i] = c.spill[from + i];
+          __syncthreads();
+          if (threadIdx.x == 0) {
+            s_qcount = rest;
+            s_moved = rest > moved ? from + moved : 0u;
+          }
           __syncthreads();
         }
         continue;
@@ -1613,7 +1621,7 @@ __global__ void __launch_bounds__(T, 1024 / T) raster_kernel(const RasterParams 
     // coordinates, in the idle queue (a side is at most 1024): one division
     // per column and row instead of two per pixel.
     float* ndc = reinterpret_cast<float*>(queue);
-    static_assert(sizeof(QEntry) * 256 >= 2 * 1024 * sizeof(float), "the queue holds both tables");
+    static_assert(sizeof(QEntry) * queue_capacity(256) >= 2 * 1024 * sizeof(float), "the queue holds both tables");
     for (int i = threadIdx.x; i < c.rw + c.rh; i += T)
       ndc[i] = i < c.rw ? __fdiv_rn(float(2 * (c.rx0 + i) + 1 - c.W), float(c.W))
                         : __fdiv_rn(float(2 * (c.ry0 + i - c.rw) + 1 - c.H), float(c.H));
@@ -1774,8 +1782,12 @@ cudaError_t launch_prepare(const PrepareParams& p, uint32_t scene_count, cudaStr
   return cudaGetLastError();
 }
 
-size_t raster_smem_bytes(int threads, int region_px, int prefix_cap) {
-  return smem_layout(threads, region_px, prefix_cap).total;
+size_t raster_smem_bytes(int threads, int region_w, int region_h, int prefix_cap) {
+  return smem_layout(threads, region_w, region_h, prefix_cap).total;
+}
+
+uint32_t raster_flush_at(int threads, int percent) {
+  return uint32_t(std::max(1, std::min(threads * percent / 100, queue_capacity(threads))));
 }
 
 size_t raster_spill_bytes(int threads, uint32_t grid) {
@@ -1833,6 +1845,7 @@ cudaError_t launch_raster(const RasterParams& p, int threads, uint32_t grid, siz
   // Programmatic dependent launch: the CTAs start while the kernel before
   // them finishes and wait for it in the kernel, which takes the launch's own
   // latency (2-3 us of a small draw's 40-50) off the path.
+  const SmemLayout layout = smem_layout(threads, p.region_w, p.region_h, p.prefix_cap);
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -1846,9 +1859,9 @@ cudaError_t launch_raster(const RasterParams& p, int threads, uint32_t grid, siz
   cudaError_t e = cudaSuccess;
 #define GBR_LAUNCH(T)                                           \
   if (p.any_lod)                                                \
-    e = cudaLaunchKernelEx(&config, raster_kernel<T, true>, p); \
+    e = cudaLaunchKernelEx(&config, raster_kernel<T, true>, p, layout); \
   else                                                          \
-    e = cudaLaunchKernelEx(&config, raster_kernel<T, false>, p);
+    e = cudaLaunchKernelEx(&config, raster_kernel<T, false>, p, layout);
   GBR_RASTER_SWITCH(threads, GBR_LAUNCH)
 #undef GBR_LAUNCH
   return e != cudaSuccess ? e : cudaGetLastError();
@@ -2114,7 +2127,7 @@ extern "C" gbr_status gbr_render_mesh_no_alloc(
   constexpr int kThreads = 1024;
   size_t max_dyn = 0, static_bytes = 0;
   e = raster_configure(kThreads, &max_dyn, &static_bytes);
-  const size_t smem = raster_smem_bytes(kThreads, kNoAllocRegion * kNoAllocRegion, 1);
+  const size_t smem = raster_smem_bytes(kThreads, kNoAllocRegion, kNoAllocRegion, 1);
   int occ = 0, sms = 0;
   if (e == cudaSuccess) e = raster_max_ctas_per_sm(kThreads, smem, &occ);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -2147,10 +2160,10 @@ extern "C" gbr_status gbr_render_mesh_no_alloc(
   p.out.depth = depth;
   p.out.linear = linear_depth;
   p.out.semantic = semantic;
-  p.region_px = kNoAllocRegion * kNoAllocRegion;
+  p.region_w = p.region_h = kNoAllocRegion;
   p.prefix_cap = 1;
   p.small_area = 1;
-  p.flush_at = 3 * kThreads / 4;
+  p.flush_at = raster_flush_at(kThreads, 75);
   const uint32_t grid = std::min<uint32_t>(a.items, uint32_t(sms) * uint32_t(occ));
   e = launch_raster(p, kThreads, grid, smem, false, st);
   if (e != cudaSuccess)

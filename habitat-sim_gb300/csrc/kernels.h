@@ -80,11 +80,11 @@ struct RasterParams {
   uint32_t* counter;  // persistent mode: next item
   int32_t persistent;
   Planes out;
-  int32_t region_px;   // capacity of the shared z-buffer, pixels
+  int32_t region_w, region_h;  // largest item: the shared z-buffer and depth tiles are sized for it
   int32_t prefix_cap;  // visible draws whose ordinals are cached in shared memory
   int32_t small_area;  // boxes up to this many pixels are rasterised by one lane
   int32_t occlusion;   // skip chunks hidden behind the depths written so far
-  uint32_t flush_at;   // the queue is rasterised once it holds this many triangles (1..threads)
+  uint32_t flush_at;   // the queue is rasterised once it holds this many triangles (raster_flush_at)
   // Lighting (max_lights > 0): lights per scene, per-draw model data, normals.
   const WorldLight* lights;
   const ModelRec* model;
@@ -94,8 +94,17 @@ struct RasterParams {
   int any_lod;  // some texture has mip levels or a minification filter of its own
 };
 
+// Dynamic shared memory of the raster kernel: byte offsets of its sections (the
+// z-buffer is first), each on a 16-byte boundary.
+struct SmemLayout {
+  uint32_t queue, qoff, prefix, chunks, clusters, tiles, coarse, total;
+};
+
 cudaError_t launch_prepare(const PrepareParams& p, uint32_t scene_count, cudaStream_t stream);
-size_t raster_smem_bytes(int threads, int region_px, int prefix_cap);
+size_t raster_smem_bytes(int threads, int region_w, int region_h, int prefix_cap);
+// Triangles at which a CTA rasterises its queue: `percent` of its threads, at
+// most what the queue holds.
+uint32_t raster_flush_at(int threads, int percent);
 // Bytes of the queue spill area for `grid` CTAs of `threads` threads.
 size_t raster_spill_bytes(int threads, uint32_t grid);
 // Raises the kernel's dynamic shared-memory limit to the device maximum and

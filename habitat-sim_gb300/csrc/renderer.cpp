@@ -1221,8 +1221,6 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
 
 gbr_status Renderer::ensure_raster_config() {
   if (raster_configured_) return GBR_OK;
-  const int region_px = tuning_.region_width * tuning_.region_height;
-  const int plain_px = tuning_.plain_region_width * tuning_.plain_region_height;
   size_t max_dyn = 0, static_smem = 0;
   GBR_CUDA(raster_configure(tuning_.threads, &max_dyn, &static_smem), "raster configure");
   // Room for the requested CTAs per SM: the SM's shared memory less the
@@ -1240,19 +1238,19 @@ gbr_status Renderer::ensure_raster_config() {
   // Shared memory not used by the launch is L1 cache: no table of ordinals
   // unless a scene needs it.
   int cap = search_ordinals_ ? kPrefixCapMax : 0;
-  size_t smem = raster_smem_bytes(tuning_.threads, std::max(region_px, plain_px), cap);
-  while (smem > budget && cap > 64) {
-    cap /= 2;
-    smem = raster_smem_bytes(tuning_.threads, std::max(region_px, plain_px), cap);
-  }
-  if (smem > max_dyn)
+  const auto need = [&](bool plain) {
+    return plain ? raster_smem_bytes(tuning_.threads, tuning_.plain_region_width, tuning_.plain_region_height, cap)
+                 : raster_smem_bytes(tuning_.threads, tuning_.region_width, tuning_.region_height, cap);
+  };
+  while (std::max(need(false), need(true)) > budget && cap > 64) cap /= 2;
+  if (std::max(need(false), need(true)) > max_dyn)
     return fail(GBR_ERROR_INVALID_ARGUMENT, "tuning: region does not fit in shared memory");
-  smem = raster_smem_bytes(tuning_.threads, region_px, cap);
+  const size_t smem = need(false);
   int occ = 0;
   GBR_CUDA(raster_max_ctas_per_sm(tuning_.threads, smem, &occ), "raster occupancy");
   if (occ < 1) return fail(GBR_ERROR_INVALID_ARGUMENT, "tuning: raster kernel cannot be resident");
   ctas_per_sm_ = std::min(occ, std::max(1, tuning_.ctas_per_sm));
-  smem_plain_ = raster_smem_bytes(tuning_.threads, plain_px, cap);
+  smem_plain_ = need(true);
   GBR_CUDA(raster_max_ctas_per_sm(tuning_.threads, smem_plain_, &plain_ctas_per_sm_), "raster occupancy");
   prefix_cap_ = cap;
   raster_configured_ = true;
@@ -1385,14 +1383,17 @@ void Renderer::order_items() {
   // the same boxes through (16 views of a room, 32 x 32 regions: 91 -> 81 us).
   // The size is part of a captured graph, so a step that fills the grid keeps
   // the shape's.
-  int px = tuning_.region_width * tuning_.region_height;
+  int w = tuning_.region_width, h = tuning_.region_height;
   if (items.size() <= grid) {
-    int largest = 1024;
-    for (const WorkItem& it : items) largest = std::max(largest, int(it.w) * int(it.h));
-    while (px / 2 >= largest) px /= 2;
+    w = h = 1;
+    for (const WorkItem& it : items) {
+      w = std::max(w, int(it.w));
+      h = std::max(h, int(it.h));
+    }
   }
-  if (px != lpt_px_) graph_valid_ = false;
-  lpt_px_ = px;
+  if (w != lpt_w_ || h != lpt_h_) graph_valid_ = false;
+  lpt_w_ = w;
+  lpt_h_ = h;
   WorkItem* istage = reinterpret_cast<WorkItem*>(static_cast<char*>(h_stage_[slot_].ptr) +
                                                  camera_block_bytes() +
                                                  size_t(total_nodes_) * 64);
@@ -1452,7 +1453,7 @@ gbr_status Renderer::enqueue_step(cudaStream_t stream, uint32_t mode) {
   rp.spill = d_spill_.ptr;
   rp.small_area = tuning_.small_area;
   rp.occlusion = tuning_.occlusion_culling;
-  rp.flush_at = uint32_t(std::max(1, tuning_.threads * tuning_.queue_fill_percent / 100));
+  rp.flush_at = raster_flush_at(tuning_.threads, tuning_.queue_fill_percent);
   rp.max_lights = max_lights_;
   rp.ambient_factor = cfg_.ambient_factor;
   rp.any_lod = 0;
@@ -1474,17 +1475,19 @@ gbr_status Renderer::enqueue_step(cudaStream_t stream, uint32_t mode) {
     rp.item_count = lpt_count_;
     rp.item_count_dev = reinterpret_cast<const uint32_t*>(d_items_lpt_.as<WorkItem>() + lpt_count_);
     rp.persistent = 1;
-    rp.region_px = lpt_px_;
+    rp.region_w = lpt_w_;
+    rp.region_h = lpt_h_;
     const uint32_t grid =
         std::min<uint32_t>(lpt_count_, uint32_t(sm_count_) * uint32_t(ctas_per_sm_));
-    GBR_CUDA(launch_raster(rp, tuning_.threads, grid, raster_smem_bytes(tuning_.threads, lpt_px_, prefix_cap_),
+    GBR_CUDA(launch_raster(rp, tuning_.threads, grid, raster_smem_bytes(tuning_.threads, lpt_w_, lpt_h_, prefix_cap_),
                            !timing_, stream), "raster launch");
     if (timing_) GBR_CUDA(cudaEventRecordWithFlags(ev_[2], stream, cudaEventRecordExternal), "timing event");
     launches = 2;
   } else {
     rp.items = d_items_.as<WorkItem>();
     rp.persistent = 0;
-    rp.region_px = tuning_.plain_region_width * tuning_.plain_region_height;
+    rp.region_w = tuning_.plain_region_width;
+    rp.region_h = tuning_.plain_region_height;
     rp.spill_owner = d_spill_owner_.as<uint32_t>();
     rp.spill_slots = uint32_t(sm_count_) * uint32_t(plain_ctas_per_sm_);
     rp.item_base = 0;

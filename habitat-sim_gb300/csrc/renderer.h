@@ -250,7 +250,7 @@ class Renderer {
   uint32_t item_count_ = 0;
   uint32_t lpt_count_ = 0;  // batched form: capacity of the item list (every scene at its finest split)
   uint32_t lpt_items_ = 0;  // batched form: items in the current list
-  int lpt_px_ = 0;          // batched form: pixels of the z-buffer a CTA is launched with
+  int lpt_w_ = 0, lpt_h_ = 0;  // batched form: the z-buffer a CTA is launched with
   bool bindings_dirty_ = true;           // sources or enabled flags changed
   bool items_staged_ = false;            // a new item order waits in the staging buffer
   uint64_t vis_needed_ = 0;              // visible records the current bindings need
