@@ -101,6 +101,14 @@ struct SmemLayout {
 };
 
 cudaError_t launch_prepare(const PrepareParams& p, uint32_t scene_count, cudaStream_t stream);
+// Orders the items p.items[0, count) of a persistent launch by what the cameras
+// see, the costliest first, into `sorted`.  The list is in scene order, a
+// scene's regions row by row from the item that its camera record names; `keys`
+// (a word per item) is scratch, `done` a zero word that is zero again
+// afterwards.  Follows the prepare kernel in the stream; `early` as for
+// launch_raster.
+cudaError_t launch_order(const RasterParams& p, uint32_t scene_count, WorkItem* sorted, uint32_t* keys, uint32_t* done,
+                         uint32_t grid, bool early, cudaStream_t stream);
 size_t raster_smem_bytes(int threads, int region_w, int region_h, int prefix_cap);
 // Triangles at which a CTA rasterises its queue: `percent` of its threads, at
 // most what the queue holds.
@@ -110,8 +118,8 @@ size_t raster_spill_bytes(int threads, uint32_t grid);
 // Raises the kernel's dynamic shared-memory limit to the device maximum and
 // returns that maximum and the kernel's static shared memory.
 cudaError_t raster_configure(int threads, size_t* max_dynamic, size_t* static_bytes);
-// early: the launch before it in the stream is the prepare kernel, and this
-// one's CTAs may start while it runs (the kernel waits for its completion).
+// early: the launch before it in the stream is the prepare or the order kernel,
+// and this one's CTAs may start while it runs (the kernel waits for its completion).
 cudaError_t launch_raster(const RasterParams& p, int threads, uint32_t grid, size_t smem, bool early,
                           cudaStream_t stream);
 cudaError_t raster_max_ctas_per_sm(int threads, size_t smem, int* out);

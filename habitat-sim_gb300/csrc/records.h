@@ -108,7 +108,9 @@ struct CameraRec {
   float vrow[4];      // row 2 of the view matrix
   uint32_t source;    // scene whose nodes and draws are rendered
   uint32_t vis_base;  // first visible record of this scene
-  uint32_t enabled;   // 0: not drawn, framebuffer rectangle untouched
+  // 0: not drawn, framebuffer rectangle untouched; else 1, or 1 + the scene's
+  // first item in a list that the device orders (order kernel).
+  uint32_t enabled;
   uint32_t light_count;  // this scene's lights in use (at most the maximum)
 };
 static_assert(sizeof(CameraRec) == 96, "CameraRec layout");

@@ -1212,6 +1212,7 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
     GBR_CUDA(cudaMemcpy(d_items_.ptr, items.data(), items.size() * sizeof(WorkItem),
                         cudaMemcpyHostToDevice), "scene upload");
   GBR_CUDA(cudaMemset(d_status_.ptr, 0, 4), "scene upload");
+  GBR_CUDA(cudaMemset(d_items_lpt_.as<WorkItem>() + lpt_count_, 0, sizeof(WorkItem)), "scene upload");
   for (auto& sc : scenes_) sc.transforms_dirty = true;
   structure_dirty_ = false;
   bindings_dirty_ = true;  // item order and visible-record bases follow the new draws
@@ -1295,7 +1296,7 @@ gbr_status Renderer::upload_step(cudaStream_t stream) {
     for (int k = 0; k < 4; ++k) cams[s].vrow[k] = sc.view[k * 4 + 2];
     cams[s].source = sc.source;
     cams[s].vis_base = sc.vis_base;
-    cams[s].enabled = sc.enabled ? 1u : 0u;
+    cams[s].enabled = sc.enabled ? 1u + sc.first_item : 0u;
     cams[s].light_count = uint32_t(std::min<size_t>(sc.light_nodes.size(), max_lights_));
   }
   if (max_lights_ > 0) {
@@ -1353,9 +1354,9 @@ gbr_status Renderer::upload_step(cudaStream_t stream) {
   return GBR_OK;
 }
 
-// The batched form's work items of the enabled scenes (build_work_items:
-// longest first, costly regions split, the last wave halved), staged for
-// upload_step() with their count.
+// The batched form's work items of the enabled scenes (build_work_items: costly
+// regions split; longest first and the last wave halved, or to be ordered on
+// the device), staged for upload_step() with their count.
 void Renderer::order_items() {
   std::vector<ItemScene> info(scenes_.size());
   for (size_t s = 0; s < scenes_.size(); ++s) {
@@ -1377,7 +1378,27 @@ void Renderer::order_items() {
       }
   }
   const uint64_t grid = std::max<uint64_t>(1, uint64_t(sm_count_) * uint64_t(ctas_per_sm_));
-  const std::vector<WorkItem> items = build_work_items(info, tuning_.region_width, tuning_.region_height, grid);
+  // Steps of several waves are ordered on the device, which knows what the
+  // cameras see (order_kernel: 10-20 us).  A single wave has no order, and with
+  // few scenes -- a CTA each -- the kernel takes longer than it gains (8 views
+  // of 640 x 480: 255 us in the host's order, 267 in the device's; 24 of them:
+  // 484 and 476; 24 of 128 x 128: 82 and 77).  The sorted list and the keys lie
+  // in the list's unused room, so that ordering takes no memory.
+  std::vector<WorkItem> items;
+  bool ordered = false;
+  uint32_t drawn = 0;
+  for (const SceneState& sc : scenes_) drawn += sc.enabled ? 1u : 0u;
+  if (drawn >= 16) {
+    items = build_work_items(info, tuning_.region_width, tuning_.region_height, grid,
+                             std::max(1u, ordered_capacity()));
+    ordered = items.size() > grid && items.size() <= ordered_capacity();
+  }
+  if (!ordered) items = build_work_items(info, tuning_.region_width, tuning_.region_height, grid);
+  if (ordered != lpt_ordered_) graph_valid_ = false;
+  for (SceneState& sc : scenes_) sc.first_item = 0;
+  if (ordered)
+    for (size_t i = items.size(); i-- > 0;) scenes_[items[i].scene].first_item = uint32_t(i);
+  lpt_ordered_ = ordered;
   // A step of few, small items is launched with a z-buffer of their size: the
   // rest of the shared memory is L1 cache, which every region's culling reads
   // the same boxes through (16 views of a room, 32 x 32 regions: 91 -> 81 us).
@@ -1477,12 +1498,23 @@ gbr_status Renderer::enqueue_step(cudaStream_t stream, uint32_t mode) {
     rp.persistent = 1;
     rp.region_w = lpt_w_;
     rp.region_h = lpt_h_;
+    launches = 2;
+    if (lpt_ordered_) {
+      const uint32_t cap = ordered_capacity();
+      WorkItem* list = d_items_lpt_.as<WorkItem>();
+      rp.item_count = cap;
+      GBR_CUDA(launch_order(rp, S, list + cap, reinterpret_cast<uint32_t*>(list + 2 * size_t(cap)),
+                            reinterpret_cast<uint32_t*>(list + lpt_count_) + 1,
+                            std::min<uint32_t>(S, uint32_t(sm_count_) * 4), !timing_, stream),
+               "order launch");
+      rp.item_base = cap;
+      launches = 3;
+    }
     const uint32_t grid =
         std::min<uint32_t>(lpt_count_, uint32_t(sm_count_) * uint32_t(ctas_per_sm_));
     GBR_CUDA(launch_raster(rp, tuning_.threads, grid, raster_smem_bytes(tuning_.threads, lpt_w_, lpt_h_, prefix_cap_),
                            !timing_, stream), "raster launch");
     if (timing_) GBR_CUDA(cudaEventRecordWithFlags(ev_[2], stream, cudaEventRecordExternal), "timing event");
-    launches = 2;
   } else {
     rp.items = d_items_.as<WorkItem>();
     rp.persistent = 0;

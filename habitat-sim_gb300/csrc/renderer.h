@@ -91,6 +91,7 @@ struct SceneState {
   uint64_t drawn = 0;      // drawn_tris() of them
   uint32_t source = 0;     // scene whose nodes and draws this scene renders
   uint32_t vis_base = 0;   // first visible record (from the current bindings)
+  uint32_t first_item = 0;  // in a list that the device orders (from the current bindings)
   bool enabled = true;
   // lights (Renderer.cpp:990-1121): node, type, colour (3 floats), range
   std::vector<int32_t> light_nodes, light_types;
@@ -184,6 +185,8 @@ class Renderer {
   size_t camera_block_bytes() const;  // cameras then light sources, per step
   bool texture_removed(uint32_t t) const { return t < texture_live_.size() && !texture_live_[t]; }
   void order_items();
+  // Items that leave room in the list's buffer for a sorted copy and a key each.
+  uint32_t ordered_capacity() const { return uint32_t(uint64_t(lpt_count_) * 3 / 7); }
 
   gbr_config cfg_{};
   std::vector<int32_t> viewports_;
@@ -250,6 +253,7 @@ class Renderer {
   uint32_t item_count_ = 0;
   uint32_t lpt_count_ = 0;  // batched form: capacity of the item list (every scene at its finest split)
   uint32_t lpt_items_ = 0;  // batched form: items in the current list
+  bool lpt_ordered_ = false;  // batched form: the device orders the list (order kernel)
   int lpt_w_ = 0, lpt_h_ = 0;  // batched form: the z-buffer a CTA is launched with
   bool bindings_dirty_ = true;           // sources or enabled flags changed
   bool items_staged_ = false;            // a new item order waits in the staging buffer
