@@ -35,7 +35,7 @@ enum : uint32_t {
 // VisibleRec::flags bit: the draw's bounding box lies inside the frustum.
 constexpr uint32_t kDrawInsideFrustum = 0x100u;
 
-struct MeshRec {
+struct alignas(16) MeshRec {
   uint32_t vertex_base;
   uint32_t vertex_count;
   uint32_t index_base;
@@ -87,7 +87,7 @@ __host__ __device__ inline uint32_t ordinal_shift(uint32_t draws, uint32_t max_t
   return shift + bits <= 32 && shift < 32 ? shift : kOrdinalRunning;
 }
 
-struct DrawRec {
+struct alignas(16) DrawRec {
   uint32_t node;         // scene-local node index
   uint32_t mesh;
   uint32_t first_index;  // absolute index into the index array
