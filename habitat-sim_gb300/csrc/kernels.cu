@@ -1814,18 +1814,30 @@ __global__ void __launch_bounds__(T, 1024 / T)
       ndc[i] = i < c.rw ? __fdiv_rn(float(2 * (c.rx0 + i) + 1 - c.W), float(c.W))
                         : __fdiv_rn(float(2 * (c.ry0 + i - c.rw) + 1 - c.H), float(c.H));
     __syncthreads();
-    // A thread's pixels are T apart: (column, row) advance by fixed amounts.
-    const int step_x = T % c.rw, step_y = T / c.rw;
-    int cx = int(threadIdx.x) % c.rw, cy = int(threadIdx.x) / c.rw;
+    // A warp shades blocks of 8 x 4 pixels, which share triangles, texels and
+    // their cache lines more than a row of 32 does (1024 textured views 1572 ->
+    // 1560 us).  A warp's blocks are T / 32 apart: (column, row) advance by fixed
+    // amounts.
+    const int bcols = (c.rw + 7) / 8, blocks = bcols * ((c.rh + 3) / 4);
+    const int step_x = (T / 32) % bcols, step_y = (T / 32) / bcols;
+    int bx, by;
+    auto first = [&]() {
+      bx = warp % bcols;
+      by = warp / bcols;
+    };
     auto advance = [&]() {
-      cx += step_x;
-      cy += step_y;
-      if (cx >= c.rw) {
-        cx -= c.rw;
-        ++cy;
+      bx += step_x;
+      by += step_y;
+      if (bx >= bcols) {
+        bx -= bcols;
+        ++by;
       }
     };
-    for (int i = threadIdx.x; i < npx; i += T, advance()) {
+    first();
+    for (int u = warp; u < blocks; u += T / 32, advance()) {
+      const int cx = bx * 8 + (lane & 7), cy = by * 4 + (lane >> 3);
+      if (cx >= c.rw || cy >= c.rh) continue;
+      const int i = cy * c.rw + cx;
       const int px = c.rx0 + cx, py = c.ry0 + cy;
       const uint64_t key = keys[i];
       const int64_t o = sc.fb_offset + int64_t(py) * sc.pitch + px;
@@ -1849,9 +1861,11 @@ __global__ void __launch_bounds__(T, 1024 / T)
       if (p.out.semantic) p.out.semantic[o] = sid;
     }
     if (Lod && __syncthreads_or(deferred)) {
-      cx = int(threadIdx.x) % c.rw;
-      cy = int(threadIdx.x) / c.rw;
-      for (int i = threadIdx.x; i < npx; i += T, advance()) {
+      first();
+      for (int u = warp; u < blocks; u += T / 32, advance()) {
+        const int cx = bx * 8 + (lane & 7), cy = by * 4 + (lane >> 3);
+        if (cx >= c.rw || cy >= c.rh) continue;
+        const int i = cy * c.rw + cx;
         const uint64_t key = keys[i];
         if (key == kEmptyKey || !(key & kDeferred)) continue;
         const int px = c.rx0 + cx, py = c.ry0 + cy;
