@@ -35,7 +35,7 @@ SMALL_AREA = (8, 16)
 # its rasterisation, tried on the best shape.
 QUEUE_FILL = (50, 75, 100)
 PLAIN_SPACE = [dict(plain_region_width=w, plain_region_height=h) for (w, h) in
-               ((16, 32), (32, 32), (16, 16))]
+               ((16, 32), (16, 64), (32, 64))]
 
 
 def signature(renderer, triangles):

@@ -1036,8 +1036,17 @@ gbr_status Renderer::upload_tables() {
 // us against 2423 for one 1024-thread CTA on 128 x 128, 512 mixed views 745
 // against 826).  A draw too small for a region of 16 x 32 px on every other SM
 // takes 1024 threads per CTA: then the threads per region bound it (2 views:
-// 44 us against 51).  The per-scene form has a fixed region for all scenes:
-// the one of least step_cost.
+// 44 us against 51).  The per-scene form has a fixed region for all scenes,
+// taller than wide: the costly parts of a view lie side by side, around its
+// horizon, so that a tall region holds its share of them and a wide one all or
+// nothing (48 furnished 160 x 120 views: 32 x 64 regions 303 us, 64 x 32 353; 256
+// of 128 x 128: 64 x 128 750 us, 128 x 64 793).  The longest item is estimated
+// from the part that its triangles cost, which varies to 3.5 times the mean, or
+// 1.8 times where the region spans the view's height; CTAs start in list order,
+// so a launch of several waves ends with some part of a long one.  Picked so,
+// 48 furnished views take 295 us (a bound of 2.5 times the whole cost picked 64 x
+// 64: 350), 100 of 160 x 120 394 (454), 40 lit views 194 (249), 32 scans 579 (656),
+// 48 bare rooms 116 (131), 4 furnished 640 x 480 views 168 (228).
 void Renderer::choose_shape() {
   if (tuned_) return;
   uint64_t cells = 0;
@@ -1050,10 +1059,11 @@ void Renderer::choose_shape() {
   t.region_height = 64;
   t.small_area = 4;
   const uint64_t grid = uint64_t(sm_count_) * uint64_t(t.ctas_per_sm);
-  const int sizes[][2] = {{128, 64}, {64, 64}, {64, 32}, {32, 32}, {16, 32}};
+  const int sizes[][2] = {{64, 128}, {64, 64}, {32, 64}, {16, 64}, {16, 32}};
   double best = -1.0;
   for (const auto& r : sizes) {
-    uint64_t items = 0, total = 0, largest = 0;
+    uint64_t items = 0;
+    double total = 0.0, longest = 0.0;
     for (const SceneState& sc : scenes_) {
       ItemScene it;
       it.width = sc.width;
@@ -1063,10 +1073,12 @@ void Renderer::choose_shape() {
       uint64_t n, cost;
       split_cost(it, r[0], r[1], 0, n, cost);
       items += n;
-      total += n * cost;
-      largest = std::max(largest, cost);
+      total += double(n) * double(cost);
+      const double part = double(std::min(r[0], it.width)) * double(std::min(r[1], it.height)) /
+                          (double(it.width) * double(it.height));
+      longest = std::max(longest, double(cost) + (r[1] >= it.height ? 0.8 : 2.5) * double(it.tris) * part);
     }
-    const double cost = step_cost(items, double(total), double(largest), grid);
+    const double cost = items <= grid ? longest : std::max(longest, total / double(grid) + 0.4 * longest);
     if (best < 0.0 || cost < best) {
       best = cost;
       t.plain_region_width = r[0];
