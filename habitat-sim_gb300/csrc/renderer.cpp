@@ -1040,13 +1040,10 @@ gbr_status Renderer::upload_tables() {
 // taller than wide: the costly parts of a view lie side by side, around its
 // horizon, so that a tall region holds its share of them and a wide one all or
 // nothing (48 furnished 160 x 120 views: 32 x 64 regions 303 us, 64 x 32 353; 256
-// of 128 x 128: 64 x 128 750 us, 128 x 64 793).  The longest item is estimated
-// from the part that its triangles cost, which varies to 3.5 times the mean, or
-// 1.8 times where the region spans the view's height; CTAs start in list order,
-// so a launch of several waves ends with some part of a long one.  Picked so,
-// 48 furnished views take 295 us (a bound of 2.5 times the whole cost picked 64 x
-// 64: 350), 100 of 160 x 120 394 (454), 40 lit views 194 (249), 32 scans 579 (656),
-// 48 bare rooms 116 (131), 4 furnished 640 x 480 views 168 (228).
+// of 128 x 128: 64 x 128 750 us, 128 x 64 793).  The size is the one
+// of least region_step_cost: 48 furnished 160 x 120 views take 264 us (a bound of
+// 2.5 times the whole cost picked 64 x 64: 350), 100 of them 371 (454), 40 lit views
+// 183 (249), 80 scans 644 (1255), 4 furnished 640 x 480 views 179 (228).
 void Renderer::choose_shape() {
   if (tuned_) return;
   uint64_t cells = 0;
@@ -1059,26 +1056,23 @@ void Renderer::choose_shape() {
   t.region_height = 64;
   t.small_area = 4;
   const uint64_t grid = uint64_t(sm_count_) * uint64_t(t.ctas_per_sm);
-  const int sizes[][2] = {{64, 128}, {64, 64}, {32, 64}, {16, 64}, {16, 32}};
+  const int sizes[][2] = {{64, 128}, {32, 128}, {16, 128}, {64, 64}, {32, 64}, {16, 64}, {16, 32}};
   double best = -1.0;
   for (const auto& r : sizes) {
     uint64_t items = 0;
     double total = 0.0, longest = 0.0;
     for (const SceneState& sc : scenes_) {
-      ItemScene it;
-      it.width = sc.width;
-      it.height = sc.height;
-      it.tris = scenes_[sc.source].drawn;
-      it.draws = scenes_[sc.source].draw_count;
-      uint64_t n, cost;
-      split_cost(it, r[0], r[1], 0, n, cost);
+      const SceneState& src = scenes_[sc.source];
+      const int w = std::min(r[0], sc.width), h = std::min(r[1], sc.height);
+      const uint64_t n = uint64_t((sc.width + w - 1) / w) * uint64_t((sc.height + h - 1) / h);
+      double l;
       items += n;
-      total += double(n) * double(cost);
-      const double part = double(std::min(r[0], it.width)) * double(std::min(r[1], it.height)) /
-                          (double(it.width) * double(it.height));
-      longest = std::max(longest, double(cost) + (r[1] >= it.height ? 0.8 : 2.5) * double(it.tris) * part);
+      total += double(n) * double(region_cost(src.tri_count, w, h, sc.width, sc.height, src.draw_count, l));
+      longest = std::max(longest, l);
     }
-    const double cost = items <= grid ? longest : std::max(longest, total / double(grid) + 0.4 * longest);
+    double cost = region_step_cost(items, total, longest, grid, r[1] > 64);
+    // CTAs start in list order: unordered, the last ones may start a long item.
+    if (items > grid && scenes_.size() < 16) cost = std::max(longest, total / double(grid) + 0.4 * longest);
     if (best < 0.0 || cost < best) {
       best = cost;
       t.plain_region_width = r[0];
@@ -1149,6 +1143,7 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
     sc.draw_count = r.draw_count;
     sc.tris = tris;
     sc.drawn = drawn_tris(tris, max_tris);
+    sc.tri_count = tris;
   }
   total_nodes_ = nodes;
   total_draws_ = uint32_t(draws.size());
@@ -1179,6 +1174,7 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
   };
   std::vector<ItemScene> info(S);
   for (uint32_t s = 0; s < S; ++s) {
+    scenes_[s].plain_item = uint32_t(items.size());
     tile(s, tuning_.plain_region_width, tuning_.plain_region_height, items);
     info[s].width = scenes_[s].width;
     info[s].height = scenes_[s].height;
@@ -1270,7 +1266,7 @@ gbr_status Renderer::ensure_raster_config() {
   return GBR_OK;
 }
 
-gbr_status Renderer::upload_step(cudaStream_t stream) {
+gbr_status Renderer::upload_step(cudaStream_t stream, uint32_t mode) {
   // Cameras always, local transforms of scenes whose view was taken.
   const uint32_t S = uint32_t(scenes_.size());
   if (upload_pending_[slot_]) {  // the step that last used this staging slot
@@ -1308,7 +1304,7 @@ gbr_status Renderer::upload_step(cudaStream_t stream) {
     for (int k = 0; k < 4; ++k) cams[s].vrow[k] = sc.view[k * 4 + 2];
     cams[s].source = sc.source;
     cams[s].vis_base = sc.vis_base;
-    cams[s].enabled = sc.enabled ? 1u + sc.first_item : 0u;
+    cams[s].enabled = sc.enabled ? 1u + (mode == GBR_DRAW_BATCHED ? sc.first_item : sc.plain_item) : 0u;
     cams[s].light_count = uint32_t(std::min<size_t>(sc.light_nodes.size(), max_lights_));
   }
   if (max_lights_ > 0) {
@@ -1378,6 +1374,7 @@ void Renderer::order_items() {
     it.width = sc.width;
     it.height = sc.height;
     it.tris = src.drawn;
+    it.all_tris = src.tri_count;
     it.draws = src.draw_count;
     it.enabled = sc.enabled;
     // Geometry of the source: the mesh of its largest draw.
@@ -1434,6 +1431,17 @@ void Renderer::order_items() {
   lpt_items_ = uint32_t(items.size());
   std::memcpy(istage + lpt_count_, &lpt_items_, 4);
   items_staged_ = true;
+}
+
+// Orders rp's items on the device into the unused room of the batched form's
+// list: the sorted items from ordered_capacity() on, the keys behind them.
+gbr_status Renderer::enqueue_order(const RasterParams& rp, bool early, cudaStream_t stream) {
+  const uint32_t S = uint32_t(scenes_.size()), cap = ordered_capacity();
+  WorkItem* list = d_items_lpt_.as<WorkItem>();
+  GBR_CUDA(launch_order(rp, S, list + cap, reinterpret_cast<uint32_t*>(list + 2 * size_t(cap)),
+                        reinterpret_cast<uint32_t*>(list + lpt_count_) + 1,
+                        std::min<uint32_t>(S, uint32_t(sm_count_) * 4), early, stream), "order launch");
+  return GBR_OK;
 }
 
 gbr_status Renderer::enqueue_step(cudaStream_t stream, uint32_t mode) {
@@ -1512,14 +1520,9 @@ gbr_status Renderer::enqueue_step(cudaStream_t stream, uint32_t mode) {
     rp.region_h = lpt_h_;
     launches = 2;
     if (lpt_ordered_) {
-      const uint32_t cap = ordered_capacity();
-      WorkItem* list = d_items_lpt_.as<WorkItem>();
-      rp.item_count = cap;
-      GBR_CUDA(launch_order(rp, S, list + cap, reinterpret_cast<uint32_t*>(list + 2 * size_t(cap)),
-                            reinterpret_cast<uint32_t*>(list + lpt_count_) + 1,
-                            std::min<uint32_t>(S, uint32_t(sm_count_) * 4), !timing_, stream),
-               "order launch");
-      rp.item_base = cap;
+      rp.item_count = ordered_capacity();
+      if (gbr_status st = enqueue_order(rp, !timing_, stream)) return st;
+      rp.item_base = ordered_capacity();
       launches = 3;
     }
     const uint32_t grid =
@@ -1537,8 +1540,16 @@ gbr_status Renderer::enqueue_step(cudaStream_t stream, uint32_t mode) {
     rp.item_base = 0;
     rp.item_count = item_count_;
     GBR_CUDA(launch_prepare(pp, S, stream), "prepare launch");
-    GBR_CUDA(launch_raster(rp, tuning_.threads, item_count_, smem_plain_, true, stream), "raster launch");
     launches = 2;
+    // CTAs start in the order of the items: launches of several waves are
+    // ordered like the batched form's.
+    if (plain_ordered(S, item_count_) && std::max(item_count_, lpt_items_) <= ordered_capacity()) {
+      if (gbr_status st = enqueue_order(rp, true, stream)) return st;
+      rp.items = d_items_lpt_.as<WorkItem>();
+      rp.item_base = ordered_capacity();
+      launches = 3;
+    }
+    GBR_CUDA(launch_raster(rp, tuning_.threads, item_count_, smem_plain_, true, stream), "raster launch");
   }
   launches_ = launches;
   return GBR_OK;
@@ -1569,7 +1580,7 @@ gbr_status Renderer::draw(cudaStream_t stream, uint32_t mode, bool use_graph) {
   }
   const int prev_slot = slot_;
   slot_ ^= 1;  // this draw's staging slot (and plane set when double-buffered)
-  if (gbr_status s = upload_step(stream)) {
+  if (gbr_status s = upload_step(stream, mode)) {
     slot_ = prev_slot;
     return s;
   }

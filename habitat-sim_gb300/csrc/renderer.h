@@ -89,9 +89,11 @@ struct SceneState {
   uint32_t draw_count = 0; // draws in the flattened device arrays (at the last rebuild)
   uint64_t tris = 0;       // triangles of those draws
   uint64_t drawn = 0;      // drawn_tris() of them
+  uint64_t tri_count = 0;  // their triangles
   uint32_t source = 0;     // scene whose nodes and draws this scene renders
   uint32_t vis_base = 0;   // first visible record (from the current bindings)
   uint32_t first_item = 0;  // in a list that the device orders (from the current bindings)
+  uint32_t plain_item = 0;  // in the per-scene form's list
   bool enabled = true;
   // lights (Renderer.cpp:990-1121): node, type, colour (3 floats), range
   std::vector<int32_t> light_nodes, light_types;
@@ -174,7 +176,12 @@ class Renderer {
   gbr_status check_scene(uint32_t scene, const char* fn) const;
   gbr_status upload_tables();
   gbr_status rebuild(cudaStream_t stream);
-  gbr_status upload_step(cudaStream_t stream);
+  gbr_status upload_step(cudaStream_t stream, uint32_t mode);
+  gbr_status enqueue_order(const RasterParams& rp, bool early, cudaStream_t stream);
+  // Per-scene launches of several waves over enough scenes are ordered.
+  bool plain_ordered(uint64_t scenes, uint64_t items) const {
+    return scenes >= 16 && items > uint64_t(sm_count_) * uint64_t(ctas_per_sm_ > 0 ? ctas_per_sm_ : 2);
+  }
   gbr_status enqueue_step(cudaStream_t stream, uint32_t mode);
   gbr_status ensure_raster_config();
   void choose_shape();

@@ -19,6 +19,7 @@ struct ItemScene {
   uint32_t geometry = 0;      // groups items of equal cost (the mesh of the source's largest draw)
   bool enabled = true;
   uint32_t draws = 0;         // draws of that scene
+  uint64_t all_tris = 0;      // all its triangles
 };
 
 // Region halvings a costly scene's items may get, and the most when the
@@ -41,6 +42,22 @@ inline void split_region(int width, int height, int region_w, int region_h, int 
     else if (rw > side)
       rw = (rw + 1) / 2;
   }
+}
+
+// The same with upright strips: half the area a split, up to 128 rows, then 16
+// columns and fewer rows.  The costly parts of a view lie side by side around its
+// horizon, so that strips share them.  (The plain split where a strip would need
+// more depth tiles than the whole region has.)
+inline void split_region_tall(int width, int height, int region_w, int region_h, int level, int& rw, int& rh) {
+  const int area = (region_w * region_h) >> level;
+  rw = std::max(16, area / 128);
+  rh = std::max(1, area / rw);
+  const auto tiles = [](int w, int h, int side) { return ((w + side - 1) / side) * ((h + side - 1) / side); };
+  if (area < 256 || tiles(rw, rh, 8) > tiles(region_w, region_h, 8) ||
+      tiles(rw, rh, 32) > tiles(region_w, region_h, 32))
+    return split_region(width, height, region_w, region_h, level, rw, rh);
+  rw = std::max(1, std::min(rw, width));
+  rh = std::max(1, std::min(rh, height));
 }
 
 // Triangles that a view of a scene draws, for item_cost: a camera sees most of
@@ -70,20 +87,31 @@ inline double step_cost(uint64_t items, double total, double largest, uint64_t g
   return std::max(2.5 * largest, total / double(grid) + 2.5 * total / double(items));
 }
 
-// The same for a list that the device orders by what the cameras see: the step
-// ends with the cheap items, unless one item takes longer than all.  `longest`
-// is the largest ordered_longest().
-inline double ordered_step_cost(uint64_t items, double total, double longest, uint64_t grid) {
-  return std::max(longest, total / double(grid) + 0.5 * total / double(items));
+// Estimated cost of a w x h region where the longest item matters (lists that
+// the device orders, the per-scene form): 0.9 for each triangle of its share of
+// the scene, 11.5 per pixel, 30000, and 0.03 per triangle and 85 per draw for
+// culling.  The triangles' part varies from view to view, and from region to
+// region less where they span the view's height: `longest` adds as much of it
+// as the longest of a step has.  (A factor on the whole cost, as in step_cost, is
+// too small for furnished rooms or too large for bare ones.)
+inline uint64_t region_cost(uint64_t tris, int w, int h, int W, int H, uint32_t draws, double& longest) {
+  const uint64_t px = uint64_t(w) * uint64_t(h);
+  const uint64_t part = 9 * tris * px / (10 * uint64_t(W) * uint64_t(H));
+  const uint64_t cost = part + 23 * px / 2 + 30000 + 3 * tris / 100 + 85 * uint64_t(draws);
+  longest = double(cost) + (h >= H ? 1.4 : 2.8) * double(part);
+  return cost;
 }
 
-// The longest of a scene's w x h regions: the part that its triangles cost
-// varies from view to view, to five times the mean; the rest does not.  (A
-// factor on the whole cost, as in step_cost, is too small for furnished rooms
-// or too large for bare ones: 320 furnished views, 128 x 64 regions 881 us, 64 x
-// 64 688 us; 1000 bare 64 x 64 views, whole 429 us, halved 519 us.)
-inline uint64_t ordered_longest(uint64_t tris, int w, int h, int W, int H, uint32_t draws) {
-  return item_cost(tris, w, h, W, H, draws) + 4 * (tris * (uint64_t(w) * uint64_t(h)) / (uint64_t(W) * uint64_t(H)));
+// Estimated time of such items on `grid` CTAs, the costliest first, of total cost
+// `total`: one wave ends with its longest item, several when the work is done,
+// with a little of it as the tail.  Strips (regions taller than 64 rows) take a
+// twentieth more for what they draw twice.  With region_cost fitted to whole
+// steps, 34 scene sets (bare and furnished rooms, scans, lit and mixed views; 4 to
+// 1000 views) at nine sizes: the size with the least estimate is 1.2 % slower than
+// the best on average (17 % at most).
+inline double region_step_cost(uint64_t items, double total, double longest, uint64_t grid, bool strips) {
+  const double time = items <= grid ? longest : std::max(longest, total / double(grid) + 0.1 * longest);
+  return strips ? 1.05 * time : time;
 }
 
 // Items of one scene split `level` times and the cost of the largest.
@@ -121,9 +149,10 @@ inline uint64_t work_item_capacity(const std::vector<ItemScene>& scenes, int reg
 // L2.  Halving two waves or quartering the last one was slower than halving
 // one.
 // order_capacity > 0: for a list that the device orders (its keys see the
-// cameras), if that many items hold it: the limit by ordered_step_cost, no halving of the last wave (it only adds items:
-// 1024 textured views 1617 -> 1653 us with it), the items in scene order, each
-// scene's regions row by row.
+// cameras), if that many items hold it: the limit by region_cost, regions or
+// upright strips by the same estimate, no halving of the last wave (it only adds
+// items: 1024 textured views 1617 -> 1653 us with it), the items in scene order,
+// each scene's regions row by row.
 inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scenes, int region_w, int region_h,
                                               uint64_t grid, uint64_t order_capacity = 0) {
   const bool ordered = order_capacity > 0;
@@ -131,22 +160,10 @@ inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scen
   const uint32_t S = uint32_t(scenes.size());
   // Per scene and level: items and largest cost (levels that change nothing repeat).
   struct Level {
-    uint64_t items, cost, longest;
+    uint64_t items, cost;
+    double longest;
   };
-  std::vector<Level> levels(size_t(S) * (kMaxFewSplits + 1), Level{0, 0, 0});
-  uint64_t limit = 1;
-  for (uint32_t s = 0; s < S; ++s) {
-    const ItemScene& sc = scenes[s];
-    if (!sc.enabled || sc.width <= 0 || sc.height <= 0) continue;
-    Level* l = &levels[size_t(s) * (kMaxFewSplits + 1)];
-    for (int k = 0; k <= kMaxFewSplits; ++k) {
-      split_cost(sc, region_w, region_h, k, l[k].items, l[k].cost);
-      int rw, rh;
-      split_region(sc.width, sc.height, region_w, region_h, k, rw, rh);
-      l[k].longest = ordered_longest(sc.tris, rw, rh, sc.width, sc.height, sc.draws);
-    }
-    limit = std::max(limit, l[0].cost);
-  }
+  std::vector<Level> levels(size_t(S) * (kMaxFewSplits + 1), Level{0, 0, 0.0});
   auto level_of = [&](uint32_t s, uint64_t t, int most) {
     const Level* l = &levels[size_t(s) * (kMaxFewSplits + 1)];
     int k = 0;
@@ -155,30 +172,70 @@ inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scen
   };
   int max_splits = kMaxSplits;
   double best = -1.0;
-  uint64_t best_limit = limit;
-  for (int most : {kMaxSplits, kMaxFewSplits}) {
-    uint64_t t = limit;
-    for (int i = 0; i < 28 && t > 0; ++i, t = t * 17 / 20) {
-      uint64_t items = 0, total = 0, largest = 0, longest = 0;
-      bool few = false;
-      for (uint32_t s = 0; s < S; ++s) {
-        const Level* l = &levels[size_t(s) * (kMaxFewSplits + 1)];
-        if (!l[0].items) continue;
-        const int k = level_of(s, t, most);
-        few = few || k > kMaxSplits;
-        items += l[k].items;
-        total += l[k].items * l[k].cost;
-        largest = std::max(largest, l[k].cost);
-        longest = std::max(longest, l[k].longest);
+  uint64_t best_limit = 0;
+  bool tall = false;
+  auto region = [&](uint32_t s, int level, bool strips, int& rw, int& rh) {
+    // (Whole regions stay as they are; 32 x 32 regions are worse than strips.)
+    ((strips && level > 0) || (ordered && level > 2) ? split_region_tall : split_region)(scenes[s].width, scenes[s].height, region_w, region_h, level, rw, rh);
+  };
+  for (const bool strips : {false, true}) {
+    if (strips && !ordered) break;
+    uint64_t limit = 1;
+    for (uint32_t s = 0; s < S; ++s) {
+      const ItemScene& sc = scenes[s];
+      if (!sc.enabled || sc.width <= 0 || sc.height <= 0) continue;
+      Level* l = &levels[size_t(s) * (kMaxFewSplits + 1)];
+      for (int k = 0; k <= kMaxFewSplits; ++k) {
+        if (!ordered) {
+          split_cost(sc, region_w, region_h, k, l[k].items, l[k].cost);
+          continue;
+        }
+        int rw, rh;
+        region(s, k, strips, rw, rh);
+        l[k].items = uint64_t((sc.width + rw - 1) / rw) * uint64_t((sc.height + rh - 1) / rh);
+        l[k].cost = region_cost(std::max(sc.all_tris, sc.tris), rw, rh, sc.width, sc.height, sc.draws, l[k].longest);
       }
-      if (few && items > grid) break;
-      if (ordered && i > 0 && items > order_capacity) break;
-      const double cost = ordered ? ordered_step_cost(items, double(total), double(longest), grid)
-                                  : step_cost(items, double(total), double(largest), grid);
-      if (best < 0.0 || cost < best) {
-        best = cost;
-        best_limit = t;
-        max_splits = most;
+      limit = std::max(limit, l[0].cost);
+    }
+    for (int most : {kMaxSplits, kMaxFewSplits}) {
+      if (ordered && most > kMaxSplits) break;
+      uint64_t t = limit;
+      for (int i = 0; i < 28 && t > 0; ++i, t = t * 17 / 20) {
+        uint64_t items = 0, total = 0, largest = 0;
+        double longest = 0.0;
+        bool few = false;
+        for (uint32_t s = 0; s < S; ++s) {
+          const Level* l = &levels[size_t(s) * (kMaxFewSplits + 1)];
+          if (!l[0].items) continue;
+          const int k = level_of(s, t, most);
+          few = few || k > kMaxSplits;
+          items += l[k].items;
+          total += l[k].items * l[k].cost;
+          largest = std::max(largest, l[k].cost);
+          longest = std::max(longest, l[k].longest);
+        }
+        if (few && items > grid) break;
+        if (ordered && i > 0 && items > order_capacity) break;
+        const double cost = ordered ? region_step_cost(items, double(total), longest, grid, strips)
+                                    : step_cost(items, double(total), double(largest), grid);
+        if (best < 0.0 || cost < best) {
+          best = cost;
+          best_limit = t;
+          max_splits = most;
+          tall = strips;
+        }
+      }
+    }
+  }
+  if (ordered && !tall) {  // the levels of the plain split again
+    for (uint32_t s = 0; s < S; ++s) {
+      Level* l = &levels[size_t(s) * (kMaxFewSplits + 1)];
+      if (!l[0].items) continue;
+      const ItemScene& sc = scenes[s];
+      for (int k = 0; k <= kMaxFewSplits; ++k) {
+        int rw, rh;
+        region(s, k, false, rw, rh);
+        l[k].cost = region_cost(std::max(sc.all_tris, sc.tris), rw, rh, sc.width, sc.height, sc.draws, l[k].longest);
       }
     }
   }
@@ -189,7 +246,7 @@ inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scen
     const ItemScene& sc = scenes[s];
     if (!sc.enabled || sc.width <= 0 || sc.height <= 0) continue;
     int rw, rh;
-    split_region(sc.width, sc.height, region_w, region_h, level_of(s, best_limit, max_splits), rw, rh);
+    region(s, level_of(s, best_limit, max_splits), tall, rw, rh);
     for (int y = 0; y < sc.height; y += rh)
       for (int x = 0; x < sc.width; x += rw) {
         WorkItem it{};

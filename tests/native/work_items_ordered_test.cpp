@@ -36,7 +36,9 @@ static void check_set(const std::vector<ItemScene>& scenes, int rw, int rh, uint
     CHECK(i < items.size() && items[i].scene == s);
     if (i >= items.size()) return;
     const int W = scenes[s].width, H = scenes[s].height, w = items[i].w, h = items[i].h;
-    CHECK(w >= 1 && h >= 1 && w <= rw && h <= rh);
+    CHECK(w >= 1 && h >= 1 && w * h <= rw * rh);
+    const auto tiles = [](int x, int y, int side) { return ((x + side - 1) / side) * ((y + side - 1) / side); };
+    CHECK(tiles(w, h, 8) <= tiles(rw, rh, 8) && tiles(w, h, 32) <= tiles(rw, rh, 32));  // room for the depth tiles
     for (int y = 0; y < H; y += h)
       for (int x = 0; x < W; x += w, ++i) {
         CHECK(i < items.size());

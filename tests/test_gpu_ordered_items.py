@@ -79,3 +79,23 @@ def test_ordered_under_a_graph(pkg):
         seen.add(_launches(a))
         _same(pkg, a, b, [s for s in range(n) if (s * 7) % n < on])
     assert seen == {2, 3}
+
+
+def test_ordered_per_scene_form(pkg):
+    """The per-scene form's launches of several waves are ordered as well, in
+    the room of the batched form's list: both forms in turn on one renderer."""
+    from habitat_sim_gb300 import procedural
+    wl, a, b = _pair(pkg, [(1 + 37 * s % 200, 1 + 53 * s % 150) for s in range(90)], 43)
+    tuned = dict(threads=512, ctas_per_sm=2, region_width=64, region_height=64, plain_region_width=64,
+                 plain_region_height=32)
+    b.setTuning(**tuned)
+    for step in range(3):
+        poses = procedural.camera_poses(wl, step)
+        for r in (a, b):
+            procedural.set_cameras(r, wl, poses)
+        a.draw()
+        b.draw()  # per scene
+        assert _launches(b) == 3
+        _same(pkg, a, b, range(90))
+        b.draw(mode=pkg.DrawMode.Batched)
+        _same(pkg, a, b, range(90))
