@@ -48,3 +48,29 @@ def test_tiles_match_oracle(count, w, h, tiles_x, mult):
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), int((got != want).sum())
     assert m.get_state() == (0xabcdef0123, (1 << 33) + 1)
     m.close()
+
+
+@pytest.mark.parametrize("count", [3, 70])
+def test_close_walls_match_oracle(count):
+    """Depths whose quotients lie beyond the output table and around the end
+    of the estimate's range (131072 / 281 per metre: 2 mm)."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    graft.load_package()
+    from habitat_sim_gb300 import noise
+    w, h = 128, 120
+    rng = np.random.default_rng(count)
+    plane = np.exp(rng.uniform(np.log(1e-4), np.log(0.4), (count * h, w))).astype(np.float32)
+    src = torch.from_numpy(plane).cuda()
+    dst = torch.empty_like(src)
+    model = noise.load_model()
+    m = noise.RedwoodNoiseModelGPUImpl(model, 0, 1.0, seed=7)
+    m.set_state(7, 5)
+    m.simulate_tiles(src.data_ptr(), dst.data_ptr(), w, w, h, 1, count)
+    torch.cuda.synchronize()
+    table = N.normal_table()
+    want = np.concatenate([N.redwood_f32(plane[i * h:(i + 1) * h], model, 1.0, 7, 5, image=i, table=table)
+                           for i in range(count)])
+    assert np.array_equal(dst.cpu().numpy().view(np.uint32), want.view(np.uint32))
+    m.close()
