@@ -446,7 +446,7 @@ def measure(pkg, procedural, name, wl, steps, warmup, plain_steps, e2e_steps, pa
             "p50_ms": float(np.percentile(plain_ms, 50)), "p99_ms": float(np.percentile(plain_ms, 99)),
             "ctas_per_env": {"min": min(plain_ctas), "max": max(plain_ctas),
                              "mean": float(np.mean(plain_ctas))},
-            "form": "one prepare + one raster launch, no graph; "
+            "form": "one prepare, one order and one raster launch, no graph; "
                     "ctas_per_env CTAs of %d threads per env (%d x %d px regions)"
                     % (t["threads"], t["plain_region_width"], t["plain_region_height"])},
         "batched_over_plain": value / plain_fps if plain_fps else None,

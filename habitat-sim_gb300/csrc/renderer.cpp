@@ -1032,9 +1032,9 @@ gbr_status Renderer::upload_tables() {
 
 // Launch shape of a renderer whose caller set none.  512-thread CTAs, two per
 // SM, on 128 x 64 regions with boxes of up to 4 px left to one lane: while one
-// CTA waits at a barrier the other issues (1024 textured 128 x 128 views: 2058
-// us against 2423 for one 1024-thread CTA on 128 x 128, 512 mixed views 745
-// against 826).  A draw too small for a region of 16 x 32 px on every other SM
+// CTA waits at a barrier the other issues (1024 textured 128 x 128 views: 1554
+// us against 2190 with one 1024-thread CTA per SM, 512 mixed views 603 against
+// 751).  A draw too small for a region of 16 x 32 px on every other SM
 // takes 1024 threads per CTA: then the threads per region bound it (2 views:
 // 44 us against 51).  The per-scene form has a fixed region for all scenes,
 // taller than wide: the costly parts of a view lie side by side, around its

@@ -61,8 +61,9 @@ typedef struct gbr_renderer gbr_renderer;
 #define GBR_PLANE_ALL 15u
 
 /* Draw modes for gbr_draw_mode. */
-#define GBR_DRAW_PER_SCENE 0u /* one prepare + one raster launch, one CTA per region */
-#define GBR_DRAW_BATCHED 1u   /* one prepare + one persistent raster launch */
+#define GBR_DRAW_PER_SCENE 0u /* one prepare + one raster launch, one CTA per region; several
+                               waves of at least 16 scenes: ordered by a launch between */
+#define GBR_DRAW_BATCHED 1u   /* one prepare + one persistent raster launch, ordered alike */
 
 /* RendererConfiguration (Renderer.h:45-113) + RendererStandaloneConfiguration
  * (RendererStandalone.h:47-100, setCudaDevice at :67), plus the per-scene viewport extension. */
@@ -327,7 +328,9 @@ typedef struct gbr_tuning {
   int32_t queue_fill_percent;  /* bin capacity in use: the CTA rasterises
                                   its shared triangle queue once it holds
                                   this share of its `threads` entries,
-                                  25..100 (default 75)                      */
+                                  25..100 (default 75; the queue holds 11/16
+                                  of them, so that larger shares mean a full
+                                  queue)                                    */
 } gbr_tuning;
 gbr_status gbr_get_tuning(gbr_renderer* r, gbr_tuning* out);
 gbr_status gbr_set_tuning(gbr_renderer* r, const gbr_tuning* tuning);
@@ -340,7 +343,8 @@ typedef struct gbr_draw_stats {
                                   kernel timing is on (batched mode), else -1 */
 } gbr_draw_stats;
 /* Records CUDA events around the prepare and raster launches of each
- * batched draw (also inside a captured graph). */
+ * batched draw (also inside a captured graph); the launch that orders a large
+ * step counts with the raster kernel. */
 gbr_status gbr_set_kernel_timing(gbr_renderer* r, int32_t enabled);
 gbr_status gbr_last_draw_stats(gbr_renderer* r, gbr_draw_stats* out);
 
