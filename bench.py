@@ -435,7 +435,7 @@ def measure(pkg, procedural, name, wl, steps, warmup, plain_steps, e2e_steps, pa
         for line in open(tpath):
             if line.startswith("dram_bytes_per_launch:"):
                 traffic = float(line.split(":")[1])
-            elif line.startswith("smsp__issue_active.avg.pct_of_peak_sustained_active"):
+            elif line.startswith("smsp__issue_active.avg.pct_of_peak_sustained_active "):
                 issue = float(line.split()[1]) / 100.0
     res = {
         "value": value, "unit": "frames/s", "steps": steps, "warmup": warmup,
