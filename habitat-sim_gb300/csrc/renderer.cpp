@@ -1377,6 +1377,7 @@ void Renderer::order_items() {
     it.all_tris = src.tri_count;
     it.draws = src.draw_count;
     it.enabled = sc.enabled;
+    if (!sc.enabled) continue;
     // Geometry of the source: the mesh of its largest draw.
     uint32_t best = 0;
     it.geometry = 0xffffffffu;

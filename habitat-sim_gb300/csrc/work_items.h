@@ -157,15 +157,19 @@ inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scen
                                               uint64_t grid, uint64_t order_capacity = 0) {
   const bool ordered = order_capacity > 0;
   grid = std::max<uint64_t>(grid, 1);
-  const uint32_t S = uint32_t(scenes.size());
-  // Per scene and level: items and largest cost (levels that change nothing repeat).
+  std::vector<uint32_t> on;  // the scenes that have items
+  for (uint32_t s = 0; s < scenes.size(); ++s)
+    if (scenes[s].enabled && scenes[s].width > 0 && scenes[s].height > 0) on.push_back(s);
+  // Per such scene and level, whole regions and strips: items and largest cost
+  // (levels that change nothing repeat).
   struct Level {
     uint64_t items, cost;
     double longest;
   };
-  std::vector<Level> levels(size_t(S) * (kMaxFewSplits + 1), Level{0, 0, 0.0});
-  auto level_of = [&](uint32_t s, uint64_t t, int most) {
-    const Level* l = &levels[size_t(s) * (kMaxFewSplits + 1)];
+  const int deepest = ordered ? kMaxSplits : kMaxFewSplits;
+  std::vector<Level> levels[2];
+  auto level_of = [&](size_t n, bool strips, uint64_t t, int most) {
+    const Level* l = &levels[strips][n * size_t(deepest + 1)];
     int k = 0;
     while (k < most && l[k].cost > t) ++k;
     return k;
@@ -176,22 +180,23 @@ inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scen
   bool tall = false;
   auto region = [&](uint32_t s, int level, bool strips, int& rw, int& rh) {
     // (Whole regions stay as they are; 32 x 32 regions are worse than strips.)
-    ((strips && level > 0) || (ordered && level > 2) ? split_region_tall : split_region)(scenes[s].width, scenes[s].height, region_w, region_h, level, rw, rh);
+    ((strips && level > 0) || (ordered && level > 2) ? split_region_tall : split_region)(
+        scenes[s].width, scenes[s].height, region_w, region_h, level, rw, rh);
   };
   for (const bool strips : {false, true}) {
     if (strips && !ordered) break;
     uint64_t limit = 1;
-    for (uint32_t s = 0; s < S; ++s) {
-      const ItemScene& sc = scenes[s];
-      if (!sc.enabled || sc.width <= 0 || sc.height <= 0) continue;
-      Level* l = &levels[size_t(s) * (kMaxFewSplits + 1)];
-      for (int k = 0; k <= kMaxFewSplits; ++k) {
+    levels[strips].resize(on.size() * size_t(deepest + 1), Level{0, 0, 0.0});
+    for (size_t n = 0; n < on.size(); ++n) {
+      const ItemScene& sc = scenes[on[n]];
+      Level* l = &levels[strips][n * size_t(deepest + 1)];
+      for (int k = 0; k <= deepest; ++k) {
         if (!ordered) {
           split_cost(sc, region_w, region_h, k, l[k].items, l[k].cost);
           continue;
         }
         int rw, rh;
-        region(s, k, strips, rw, rh);
+        region(on[n], k, strips, rw, rh);
         l[k].items = uint64_t((sc.width + rw - 1) / rw) * uint64_t((sc.height + rh - 1) / rh);
         l[k].cost = region_cost(std::max(sc.all_tris, sc.tris), rw, rh, sc.width, sc.height, sc.draws, l[k].longest);
       }
@@ -204,10 +209,9 @@ inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scen
         uint64_t items = 0, total = 0, largest = 0;
         double longest = 0.0;
         bool few = false;
-        for (uint32_t s = 0; s < S; ++s) {
-          const Level* l = &levels[size_t(s) * (kMaxFewSplits + 1)];
-          if (!l[0].items) continue;
-          const int k = level_of(s, t, most);
+        for (size_t n = 0; n < on.size(); ++n) {
+          const Level* l = &levels[strips][n * size_t(deepest + 1)];
+          const int k = level_of(n, strips, t, most);
           few = few || k > kMaxSplits;
           items += l[k].items;
           total += l[k].items * l[k].cost;
@@ -227,26 +231,14 @@ inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scen
       }
     }
   }
-  if (ordered && !tall) {  // the levels of the plain split again
-    for (uint32_t s = 0; s < S; ++s) {
-      Level* l = &levels[size_t(s) * (kMaxFewSplits + 1)];
-      if (!l[0].items) continue;
-      const ItemScene& sc = scenes[s];
-      for (int k = 0; k <= kMaxFewSplits; ++k) {
-        int rw, rh;
-        region(s, k, false, rw, rh);
-        l[k].cost = region_cost(std::max(sc.all_tris, sc.tris), rw, rh, sc.width, sc.height, sc.draws, l[k].longest);
-      }
-    }
-  }
   std::vector<WorkItem> items;
   std::vector<uint64_t> cost;
   std::vector<uint32_t> key;
-  for (uint32_t s = 0; s < S; ++s) {
+  for (size_t n = 0; n < on.size(); ++n) {
+    const uint32_t s = on[n];
     const ItemScene& sc = scenes[s];
-    if (!sc.enabled || sc.width <= 0 || sc.height <= 0) continue;
     int rw, rh;
-    region(s, level_of(s, best_limit, max_splits), tall, rw, rh);
+    region(s, level_of(n, tall, best_limit, max_splits), tall, rw, rh);
     for (int y = 0; y < sc.height; y += rh)
       for (int x = 0; x < sc.width; x += rw) {
         WorkItem it{};
