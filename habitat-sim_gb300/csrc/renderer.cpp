@@ -1002,30 +1002,38 @@ gbr_status Renderer::memory_usage(uint64_t* live, uint64_t* reserved) const {
 }
 
 // -------------------------------------------------------------- drawing
-gbr_status Renderer::upload_tables() {
+gbr_status Renderer::upload_tables(cudaStream_t stream) {
   if (!tables_dirty_) return GBR_OK;
   if (!d_meshes_.reserve(std::max<size_t>(1, meshes_.size()) * sizeof(MeshRec), false) ||
       !d_materials_.reserve(materials_.size() * sizeof(MaterialRec), false) ||
       !d_textures_.reserve(textures_.size() * sizeof(TextureRec), false) ||
       !d_boxes_.reserve(std::max<size_t>(1, boxes_.size()) * sizeof(ChunkBox), true))
     return fail(GBR_ERROR_OUT_OF_MEMORY, "draw: out of device memory for tables");
+  // On the draw's stream, which need not be ordered with the legacy default
+  // one.  (A stream that the caller captures takes no copy from these host
+  // tables: the plain copy is refused or done at once, by the capture's mode.)
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  const bool captured =
+      cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  const auto copy = [&](void* dst, const void* src, size_t bytes) {
+    return captured ? cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice)
+                    : cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream);
+  };
   // Only the boxes written since the last upload (the device copy keeps the
   // rest, also across growth): a scene loaded into a large resident set
   // costs its own boxes, not the whole table.
   if (boxes_hi_ > boxes_lo_) {
-    GBR_CUDA(cudaMemcpy(d_boxes_.as<ChunkBox>() + boxes_lo_, boxes_.data() + boxes_lo_,
-                        (boxes_hi_ - boxes_lo_) * sizeof(ChunkBox), cudaMemcpyHostToDevice),
-             "table upload");
+    GBR_CUDA(copy(d_boxes_.as<ChunkBox>() + boxes_lo_, boxes_.data() + boxes_lo_,
+                  (boxes_hi_ - boxes_lo_) * sizeof(ChunkBox)), "table upload");
     boxes_lo_ = SIZE_MAX;
     boxes_hi_ = 0;
   }
   if (!meshes_.empty())
-    GBR_CUDA(cudaMemcpy(d_meshes_.ptr, meshes_.data(), meshes_.size() * sizeof(MeshRec),
-                        cudaMemcpyHostToDevice), "table upload");
-  GBR_CUDA(cudaMemcpy(d_materials_.ptr, materials_.data(), materials_.size() * sizeof(MaterialRec),
-                      cudaMemcpyHostToDevice), "table upload");
-  GBR_CUDA(cudaMemcpy(d_textures_.ptr, textures_.data(), textures_.size() * sizeof(TextureRec),
-                      cudaMemcpyHostToDevice), "table upload");
+    GBR_CUDA(copy(d_meshes_.ptr, meshes_.data(), meshes_.size() * sizeof(MeshRec)), "table upload");
+  GBR_CUDA(copy(d_materials_.ptr, materials_.data(), materials_.size() * sizeof(MaterialRec)), "table upload");
+  GBR_CUDA(copy(d_textures_.ptr, textures_.data(), textures_.size() * sizeof(TextureRec)), "table upload");
+  if (!captured) GBR_CUDA(cudaStreamSynchronize(stream), "table upload");  // the host tables may change
   tables_dirty_ = false;
   return GBR_OK;
 }
@@ -1188,7 +1196,7 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
   lpt_count_ = uint32_t(capacity);
 
   cudaSetDevice(device_);
-  if (gbr_status st = upload_tables()) return st;
+  if (gbr_status st = upload_tables(stream)) return st;
   const size_t S1 = std::max<size_t>(S, 1);
   if (!d_scenes_.reserve(S1 * sizeof(SceneRec), false) ||
       !d_parents_.reserve(std::max<size_t>(nodes, 1) * 4, false) ||
@@ -1208,19 +1216,22 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
                            (size_t(lpt_count_) + 1) * sizeof(WorkItem)) ||
       !h_stage_[1].reserve(h_stage_[0].bytes))
     return fail(GBR_ERROR_OUT_OF_MEMORY, "draw: out of memory for scene data");
-  GBR_CUDA(cudaMemcpy(d_scenes_.ptr, recs.data(), S * sizeof(SceneRec), cudaMemcpyHostToDevice),
+  // All on the draw's stream: a non-blocking one is not ordered with the legacy
+  // default stream, on which a late memset would wipe the item count that the
+  // step uploads or the CTA count of a running order kernel.
+  const auto copy = [&](void* dst, const void* src, size_t bytes) {
+    return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream) : cudaSuccess;
+  };
+  GBR_CUDA(copy(d_scenes_.ptr, recs.data(), S * sizeof(SceneRec)), "scene upload");
+  GBR_CUDA(copy(d_parents_.ptr, parents.data(), parents.size() * 4), "scene upload");
+  GBR_CUDA(copy(d_draws_.ptr, draws.data(), draws.size() * sizeof(DrawRec)), "scene upload");
+  GBR_CUDA(copy(d_items_.ptr, items.data(), items.size() * sizeof(WorkItem)), "scene upload");
+  GBR_CUDA(cudaMemsetAsync(d_status_.ptr, 0, 4, stream), "scene upload");
+  // The order kernel's count of finished CTAs, behind the list's item count
+  // (which upload_step() writes).
+  GBR_CUDA(cudaMemsetAsync(reinterpret_cast<uint32_t*>(d_items_lpt_.as<WorkItem>() + lpt_count_) + 1, 0, 4, stream),
            "scene upload");
-  if (nodes)
-    GBR_CUDA(cudaMemcpy(d_parents_.ptr, parents.data(), nodes * 4, cudaMemcpyHostToDevice),
-             "scene upload");
-  if (!draws.empty())
-    GBR_CUDA(cudaMemcpy(d_draws_.ptr, draws.data(), draws.size() * sizeof(DrawRec),
-                        cudaMemcpyHostToDevice), "scene upload");
-  if (!items.empty())
-    GBR_CUDA(cudaMemcpy(d_items_.ptr, items.data(), items.size() * sizeof(WorkItem),
-                        cudaMemcpyHostToDevice), "scene upload");
-  GBR_CUDA(cudaMemset(d_status_.ptr, 0, 4), "scene upload");
-  GBR_CUDA(cudaMemset(d_items_lpt_.as<WorkItem>() + lpt_count_, 0, sizeof(WorkItem)), "scene upload");
+  GBR_CUDA(cudaStreamSynchronize(stream), "scene upload");  // the vectors go
   for (auto& sc : scenes_) sc.transforms_dirty = true;
   structure_dirty_ = false;
   bindings_dirty_ = true;  // item order and visible-record bases follow the new draws
@@ -1564,7 +1575,7 @@ gbr_status Renderer::draw(cudaStream_t stream, uint32_t mode, bool use_graph) {
     if (gbr_status s = rebuild(stream)) return s;
   if (gbr_status s = ensure_raster_config()) return s;
   if (tables_dirty_)
-    if (gbr_status s = upload_tables()) return s;
+    if (gbr_status s = upload_tables(stream)) return s;
   {
     // Queue spill space for every CTA that can be resident (allocated before
     // any graph capture).
@@ -1647,7 +1658,7 @@ gbr_status Renderer::sync_and_check() {
     if (status) {
       // The host's scene records are authoritative: upload them again at the
       // next draw, so that a record damaged on the device does not persist.
-      cudaMemset(d_status_.ptr, 0, 4);
+      cudaMemsetAsync(d_status_.ptr, 0, 4, last_stream_);
       structure_dirty_ = true;
       return fail(GBR_ERROR_DEVICE, "draw: the device reported bad scene data (status " +
                                         std::to_string(status) +

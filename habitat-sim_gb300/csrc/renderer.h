@@ -174,7 +174,7 @@ class Renderer {
   gbr_status fail(gbr_status s, const std::string& msg);
   gbr_status cuda_fail(cudaError_t e, const char* what);
   gbr_status check_scene(uint32_t scene, const char* fn) const;
-  gbr_status upload_tables();
+  gbr_status upload_tables(cudaStream_t stream);
   gbr_status rebuild(cudaStream_t stream);
   gbr_status upload_step(cudaStream_t stream, uint32_t mode);
   gbr_status enqueue_order(const RasterParams& rp, bool early, cudaStream_t stream);

@@ -1,0 +1,8 @@
+"""Native tests of the renderer's host runtime on a fake CUDA runtime (no GPU)."""
+import pytest
+from test_native_host import test_native as _run
+
+
+@pytest.mark.parametrize("name", ["draw_stream_test"])
+def test_renderer_runtime(name, tmp_path):
+    _run(name, tmp_path)
