@@ -770,8 +770,9 @@ __device__ __noinline__ void clip_and_emit(float4 v0, float4 v1, float4 v2, uint
 }
 
 // `simple`: the triangle's chunk lies between the near and far planes and in
-// the guard band by a margin (chunk_keep), so it is never clipped; if it lies
-// beside the viewport, its bounding box holds no pixel of the region.
+// the guard band by margins that cover every rounding (chunk_keep), so it is
+// never clipped; if it lies beside the viewport, its bounding box holds no pixel
+// of the region.
 __device__ __forceinline__ void triangle(const float4* cv, uint32_t ordinal, bool simple, const Ctx& c) {
   if (simple) {
     emit(cv, ordinal, c);
@@ -1205,23 +1206,33 @@ __device__ __forceinline__ uint32_t find_cluster_draw(const uint2* order, uint32
 // Culling of a 32-triangle chunk or a 1024-triangle cluster by its
 // object-space box, decided by the thread that owns it.  Rejected when
 //  * frustum: all eight corners lie beyond one clip plane (outcode margins);
-//  * region: the box projects (two pixels of margin) outside the region;
+//  * region: the box projects outside the region, by a margin;
 //  * occlusion: every fragment it could produce loses the depth test against
 //    what the z-buffer already holds -- the box lies in front of the camera,
-//    and its nearest window depth, minus a margin above the rounding of either
-//    computation (a fixed part, and one that grows where w is small against the
-//    terms it is the sum of), is beyond the deepest value of every depth tile its
-//    projection (plus one pixel) touches.  Depths only decrease, so the
-//    chunk stays hidden.
+//    and its nearest window depth, less a margin, is beyond the deepest value of
+//    every depth tile its projection (and a margin) touches.  Depths only
+//    decrease, so the chunk stays hidden.
 // Every test is conservative: a rejected chunk has no fragment in the final
 // image.  The corners are sums of one corner and the edges' changes, and the
 // planes are decided from sums of the changes' signs: about 220 operations per
 // box where eight full transforms with their outcodes took 440 (a tenth of the
-// kernel's time on 1024 textured views).  `simple` is set for a kept box whose
-// triangles need no clipping (see triangle): between the near and far planes by
-// 1e-5 of window depth, and within 16000 pixels of the origin, half the guard
-// band.  `rect`, if given, receives the bounds of a kept box that lies before
-// the camera, in pixels (x0, y0, x1, y1).
+// kernel's time on 1024 textured views).
+//
+// Margins.  With u = 2^-24 and T_r the sum of the magnitudes of row r's terms, a
+// vertex transform is off by at most 3 u T_r (three roundings), a corner here by 10
+// u T_r (three, four of an edge's length and product, three of the sums).  A
+// coordinate divided by w differs from the vertex's by (13 u T_r + |it| 13 u T_3)
+// / w and the reciprocal's 2^-21, for w the smallest of the box (itself good to
+// 3 %, being above 2e-5 T_3): at the planes and regions of the decisions, where
+// the quotient is at most 1, by less than 1e-6 (T_r + T_3) / w.  That is added to the
+// fixed margins: 1 pixel for the snapped edges and 2e-6 of depth for its
+// interpolation, doubled.
+//
+// `simple` is set for a kept box whose triangles need no clipping (see
+// triangle): by these margins between the near and far planes, and within 16000
+// pixels of the viewport's centre, where the guard band ends at 16384.
+// `rect`, if given, receives the bounds of a kept box that lies before the
+// camera, in pixels (x0, y0, x1, y1).
 __device__ __forceinline__ bool chunk_keep(const float* mvp, const ChunkBox& b, const Ctx& c,
                                            bool frustum, bool region, const uint32_t* tiles,
                                            const uint32_t* coarse, int tcols, int ccols, bool& simple,
@@ -1285,6 +1296,8 @@ __device__ __forceinline__ bool chunk_keep(const float* mvp, const ChunkBox& b, 
     zmin = fminf(zmin, nz);
     zmax = fmaxf(zmax, nz);
   }
+  // The farthest corner from the viewport's centre, in pixels.
+  const float reach = fmaxf(fmaxf(x1, -x0) * c.hw, fmaxf(y1, -y0) * c.hh);
   x0 = fma_(x0, c.hw, c.hw);
   x1 = fma_(x1, c.hw, c.hw);
   y0 = fma_(y0, c.hh, c.hh);
@@ -1295,19 +1308,24 @@ __device__ __forceinline__ bool chunk_keep(const float* mvp, const ChunkBox& b, 
     rect[2] = x1;
     rect[3] = y1;
   }
-  if (region && (x1 + 2.0f < float(c.rx0) || x0 - 2.0f > float(c.rx0 + c.rw) ||
-                 y1 + 2.0f < float(c.ry0) || y0 - 2.0f > float(c.ry0 + c.rh)))
+  const float ew = __fdividef(1e-6f, wmin);
+  const float mp = fma_(fmaxf(c.hw, c.hh) * ew, fmaxf(terms[0], terms[1]) + terms[3], 1.0f);  // of pixels
+  const float mz = 0.5f * ew * (terms[2] + terms[3]);                                         // of window depth
+  if (region && (x1 + mp < float(c.rx0 - 1) || x0 - mp > float(c.rx0 + c.rw + 1) ||
+                 y1 + mp < float(c.ry0 - 1) || y0 - mp > float(c.ry0 + c.rh + 1)))
     return false;
   const bool front = zmin >= -1.0f;
   zmin = fma_(zmin, 0.5f, 0.5f);
-  simple = zmin > 1e-5f && zmax < 1.0f - 2e-5f && x0 > -16000.0f && x1 < 16000.0f && y0 > -16000.0f && y1 < 16000.0f;
+  // (At 16000 pixels the margin is below 100 and 160: the guard band holds it.)
+  simple = zmin > 1e-5f + mz && zmax < 1.0f - 2e-5f - 2.0f * mz && reach < 16000.0f && mp < 100.0f &&
+           wmin > 1e-4f * terms[3];
   if (!tiles || !front) return true;
-  zmin -= 4e-6f + 1.2e-7f * __fdividef(terms[2] + terms[3], wmin);
+  zmin -= 4e-6f + mz;
   if (!(zmin > 0.0f)) return true;
-  // Pixel range of the box in region coordinates, one pixel of margin.
-  const float fx0 = fmaxf(x0 - 1.0f - float(c.rx0), 0.0f), fy0 = fmaxf(y0 - 1.0f - float(c.ry0), 0.0f);
-  const float fx1 = fminf(x1 + 1.0f - float(c.rx0), float(c.rw - 1));
-  const float fy1 = fminf(y1 + 1.0f - float(c.ry0), float(c.rh - 1));
+  // Pixel range of the box in region coordinates, with the margin.
+  const float fx0 = fmaxf(x0 - mp - float(c.rx0), 0.0f), fy0 = fmaxf(y0 - mp - float(c.ry0), 0.0f);
+  const float fx1 = fminf(x1 + mp - float(c.rx0), float(c.rw - 1));
+  const float fy1 = fminf(y1 + mp - float(c.ry0), float(c.rh - 1));
   if (!(fx0 <= fx1 && fy0 <= fy1)) return false;  // no pixel of the region
   const uint32_t zbits = __float_as_uint(zmin);
   int tx0 = int(fx0) / kTile, tx1 = int(fx1) / kTile, ty0 = int(fy0) / kTile, ty1 = int(fy1) / kTile;
