@@ -442,18 +442,17 @@ __global__ void __launch_bounds__(256, 5)
     }
   }
   // A byte result (or three, without the blur) is decided by the occlusion at
-  // both ends of the estimate's error unless they round differently.  Per
-  // sample the estimate is off by at most 8e-7: N.V / |V| by 5 roundings of
-  // products of at most |N| |V| on either side (6e-7), the reciprocal root's
-  // 2^-22.9 and as much for the falloff's; the sum by 2 x 32 roundings of at
-  // most 2^-24 of it; poly_pow by less than 2e-7 and 1.2e-7 of the exponent.
+  // both ends of the estimate's error unless they round differently: the sum's
+  // (kAoSumError), 4e-7 for the two roundings of either side that make it an
+  // occlusion and the one of each end, and poly_pow's own (kAoPowSlack).
   const long long at = s.offset + (long long)y * s.pitch + x;
   const bool byte_plane = !Special && (!p.no_blur || CacheAware);  // the result is a byte first
   bool open = !near;
   uint32_t result = 0;
   if (estimated) {
     const float est = 1.0f - 2.0f * p.ao_scale * ao;
-    const float err = 2.0f * p.ao_scale * (2.6e-5f + 5e-6f * ao) + 4e-7f, slack = 5e-7f + 3e-7f * p.pow_exp;
+    const float err = 2.0f * p.ao_scale * (kAoSumError + kAoSumRelative * ao) + 4e-7f;
+    const float slack = kAoPowSlack + kAoPowSlackPerExponent * p.pow_exp;
     const float lo = poly_pow(clamp01(est - err), p.pow_exp) - slack, hi = poly_pow(clamp01(est + err), p.pow_exp) + slack;
     if (byte_plane) {
       result = unorm8(lo);

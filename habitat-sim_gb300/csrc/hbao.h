@@ -33,6 +33,28 @@ inline long long hbao_blocks(int w, int h, int tile) {
   return ((w + tile - 1LL) / tile) * ((h + tile - 1LL) / tile);
 }
 
+// How far the AO kernel's estimated sum of 32 samples (reciprocal root by
+// rsqrt.approx, fused sums) may be from the specification's, both in single
+// precision from the same N, V, radius and bias; u = 2^-24, n = |N|.
+//   Specification: N.V off by 3 u n |V| (a product and two sums, Cauchy-Schwarz),
+//   |V| by 2.5 u (|V|^2 by 3 u, the root halves it and rounds), the quotient
+//   rounds: 6.5 u n.  Less the bias: u.  The falloff (the product of |V|^2 by
+//   4 u, the sum 1 u) 5 u, the product of both u: (6.5 n + 7) u.
+//   Estimate: N.V 3 u n |V|, the reciprocal root 2^-22.9 < 2.15 u and half of
+//   |V|^2's 3 u, the product u: 7.65 u n.  The bias u, the falloff 4 u (fused);
+//   the last product is exact inside the sum: (7.65 n + 5) u.
+// Both factors are clamped to [0, 1], which does not add.  The cache-aware normal
+// comes from bytes: each component within 1/255, so n <= 1 + sqrt(3) / 255.
+// The sums of non-negative terms round 31 and 32 times, by u of the sum each.
+constexpr double kAoUnit = 1.0 / 16777216.0, kAoNormal = 1.0 + 1.7320509 / 255.0;
+constexpr double kAoSampleError = (14.15 * kAoNormal + 12.0) * kAoUnit;
+constexpr float kAoSumError = 5.1e-5f, kAoSumRelative = 5e-6f;
+static_assert(32.0 * kAoSampleError < 0.99 * kAoSumError && 63.0 * kAoUnit < 0.99 * kAoSumRelative,
+              "the estimate's bound holds every rounding (and those of the bound itself)");
+// poly_pow(a, e) for a in [0, 1] is off a^e by less than half of this, at
+// whichever e (measured, tests/test_hbao_bound_host.py).
+constexpr float kAoPowSlack = 5e-7f, kAoPowSlackPerExponent = 3e-7f;
+
 struct HbaoParams {
   float neg_inv_r2, bias, bias2, ao_scale, pow_exp, sharpness;  // bias2: see hbao_ao_kernel
   int no_blur;
