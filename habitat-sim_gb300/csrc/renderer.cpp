@@ -322,8 +322,9 @@ Renderer::~Renderer() {
   cudaSetDevice(device_);
   if (last_stream_ || upload_pending_[0] || upload_pending_[1]) cudaDeviceSynchronize();
   if (copy_stream_) cudaStreamSynchronize(copy_stream_);
-  for (auto& g : graph_exec_)
-    if (g) cudaGraphExecDestroy(g);
+  for (auto& slot : graphs_)
+    for (StepGraph& g : slot)
+      if (g.exec) cudaGraphExecDestroy(g.exec);
   for (auto& e : copy_done_)
     if (e) cudaEventDestroy(e);
   if (copy_stream_) cudaStreamDestroy(copy_stream_);
@@ -1415,27 +1416,21 @@ void Renderer::order_items() {
     ordered = items.size() > grid && items.size() <= ordered_capacity();
   }
   if (!ordered) items = build_work_items(info, tuning_.region_width, tuning_.region_height, grid);
-  if (ordered != lpt_ordered_) graph_valid_ = false;
   for (SceneState& sc : scenes_) sc.first_item = 0;
   if (ordered)
     for (size_t i = items.size(); i-- > 0;) scenes_[items[i].scene].first_item = uint32_t(i);
-  lpt_ordered_ = ordered;
-  // A step of few, small items is launched with a z-buffer of their size: the
-  // rest of the shared memory is L1 cache, which every region's culling reads
-  // the same boxes through (16 views of a room, 32 x 32 regions: 91 -> 81 us).
-  // The size is part of a captured graph, so a step that fills the grid keeps
-  // the shape's.
-  int w = tuning_.region_width, h = tuning_.region_height;
-  if (items.size() <= grid) {
-    w = h = 1;
-    for (const WorkItem& it : items) {
-      w = std::max(w, int(it.w));
-      h = std::max(h, int(it.h));
-    }
-  }
-  if (w != lpt_w_ || h != lpt_h_) graph_valid_ = false;
-  lpt_w_ = w;
-  lpt_h_ = h;
+  // A step of few, small items is launched with a z-buffer of a quarter of a
+  // region: the rest of the shared memory is L1 cache, which every region's
+  // culling reads the same boxes through (16 views of a room: 91 us with whole
+  // ones, 81 with these).  The size is part of a captured graph, so there are
+  // two of them, not one per step: with the items' own size a renderer of 96
+  // views of which 1 to 24 are drawn captured at almost every step, 101 us
+  // a step instead of 78.
+  int w, h;
+  form_region(kSmall, w, h);
+  bool small = items.size() <= grid;
+  for (const WorkItem& it : items) small = small && it.w <= w && it.h <= h;
+  form_ = ordered ? kOrdered : small ? kSmall : kWhole;
   WorkItem* istage = reinterpret_cast<WorkItem*>(static_cast<char*>(h_stage_[slot_].ptr) +
                                                  camera_block_bytes() +
                                                  size_t(total_nodes_) * 64);
@@ -1443,6 +1438,11 @@ void Renderer::order_items() {
   lpt_items_ = uint32_t(items.size());
   std::memcpy(istage + lpt_count_, &lpt_items_, 4);
   items_staged_ = true;
+}
+
+void Renderer::form_region(StepForm form, int& w, int& h) const {
+  split_region(tuning_.region_width, tuning_.region_height, tuning_.region_width, tuning_.region_height,
+               form == kSmall ? 2 : 0, w, h);
 }
 
 // Orders rp's items on the device into the unused room of the batched form's
@@ -1528,10 +1528,12 @@ gbr_status Renderer::enqueue_step(cudaStream_t stream, uint32_t mode) {
     rp.item_count = lpt_count_;
     rp.item_count_dev = reinterpret_cast<const uint32_t*>(d_items_lpt_.as<WorkItem>() + lpt_count_);
     rp.persistent = 1;
-    rp.region_w = lpt_w_;
-    rp.region_h = lpt_h_;
+    int w, h;
+    form_region(form_, w, h);
+    rp.region_w = w;
+    rp.region_h = h;
     launches = 2;
-    if (lpt_ordered_) {
+    if (form_ == kOrdered) {
       rp.item_count = ordered_capacity();
       if (gbr_status st = enqueue_order(rp, !timing_, stream)) return st;
       rp.item_base = ordered_capacity();
@@ -1539,8 +1541,8 @@ gbr_status Renderer::enqueue_step(cudaStream_t stream, uint32_t mode) {
     }
     const uint32_t grid =
         std::min<uint32_t>(lpt_count_, uint32_t(sm_count_) * uint32_t(ctas_per_sm_));
-    GBR_CUDA(launch_raster(rp, tuning_.threads, grid, raster_smem_bytes(tuning_.threads, lpt_w_, lpt_h_, prefix_cap_),
-                           !timing_, stream), "raster launch");
+    GBR_CUDA(launch_raster(rp, tuning_.threads, grid, raster_smem_bytes(tuning_.threads, w, h, prefix_cap_), !timing_,
+                           stream), "raster launch");
     if (timing_) GBR_CUDA(cudaEventRecordWithFlags(ev_[2], stream, cudaEventRecordExternal), "timing event");
   } else {
     rp.items = d_items_.as<WorkItem>();
@@ -1607,31 +1609,35 @@ gbr_status Renderer::draw(cudaStream_t stream, uint32_t mode, bool use_graph) {
     copy_pending_[set] = false;
   }
   if (!graph_valid_) {
-    graph_built_[0] = graph_built_[1] = false;
+    for (auto& slot : graphs_)
+      for (StepGraph& g : slot) g.built = false;
     graph_valid_ = true;
   }
-  const int gi = slot_;  // graphs by staging slot (and with it the plane set)
   if (mode == GBR_DRAW_BATCHED && use_graph) {
-    if (!graph_built_[gi] || graph_stream_[gi] != stream) {
-      if (graph_exec_[gi]) {
-        cudaGraphExecDestroy(graph_exec_[gi]);
-        graph_exec_[gi] = nullptr;
+    StepGraph& sg = graphs_[slot_][form_];
+    if (!sg.built || sg.stream != stream) {
+      if (sg.exec) {
+        cudaGraphExecDestroy(sg.exec);
+        sg.exec = nullptr;
+        sg.built = false;
       }
       cudaGraph_t g;
       GBR_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "graph capture");
-      cudaError_t e = cudaMemcpyAsync(d_cameras_.ptr, h_stage_[gi].ptr, cam_bytes,
+      cudaError_t e = cudaMemcpyAsync(d_cameras_.ptr, h_stage_[slot_].ptr, cam_bytes,
                                       cudaMemcpyHostToDevice, stream);
       gbr_status st = e == cudaSuccess ? enqueue_step(stream, mode) : cuda_fail(e, "graph camera copy");
       cudaError_t e2 = cudaStreamEndCapture(stream, &g);
       if (st != GBR_OK) return st;
       GBR_CUDA(e2, "graph capture");
-      e = cudaGraphInstantiate(&graph_exec_[gi], g, 0);
+      e = cudaGraphInstantiate(&sg.exec, g, 0);
       cudaGraphDestroy(g);
       GBR_CUDA(e, "graph instantiate");
-      graph_built_[gi] = true;
-      graph_stream_[gi] = stream;
+      sg.built = true;
+      sg.stream = stream;
+      sg.launches = launches_;
     }
-    GBR_CUDA(cudaGraphLaunch(graph_exec_[gi], stream), "graph launch");
+    launches_ = sg.launches;
+    GBR_CUDA(cudaGraphLaunch(sg.exec, stream), "graph launch");
   } else {
     GBR_CUDA(cudaMemcpyAsync(d_cameras_.ptr, h_stage_[slot_].ptr, cam_bytes,
                              cudaMemcpyHostToDevice, stream),

@@ -260,8 +260,13 @@ class Renderer {
   uint32_t item_count_ = 0;
   uint32_t lpt_count_ = 0;  // batched form: capacity of the item list (every scene at its finest split)
   uint32_t lpt_items_ = 0;  // batched form: items in the current list
-  bool lpt_ordered_ = false;  // batched form: the device orders the list (order kernel)
-  int lpt_w_ = 0, lpt_h_ = 0;  // batched form: the z-buffer a CTA is launched with
+  // Batched form: how the current list is drawn.  Whole and Small: in the host's
+  // order, a CTA launched with the z-buffer of a whole region or of a quarter
+  // of one.  Ordered: by the device (order kernel), whole regions.
+  enum StepForm { kWhole, kSmall, kOrdered, kStepForms };
+  StepForm form_ = kWhole;
+  // The z-buffer of a form's CTAs.
+  void form_region(StepForm form, int& w, int& h) const;
   bool bindings_dirty_ = true;           // sources or enabled flags changed
   bool items_staged_ = false;            // a new item order waits in the staging buffer
   uint64_t vis_needed_ = 0;              // visible records the current bindings need
@@ -275,10 +280,15 @@ class Renderer {
   int ctas_per_sm_ = 1;
   int plain_ctas_per_sm_ = 1;  // CTAs of the per-scene form that can be resident on an SM
 
-  // CUDA graphs of the batched step, one per plane set
-  cudaGraphExec_t graph_exec_[2] = {nullptr, nullptr};
-  cudaStream_t graph_stream_[2] = {nullptr, nullptr};
-  bool graph_built_[2] = {false, false};
+  // CUDA graphs of the batched step, one per staging slot (and with it the plane
+  // set) and form, so that steps whose scenes come and go capture each once.
+  struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    cudaStream_t stream = nullptr;
+    uint64_t launches = 0;
+    bool built = false;
+  };
+  StepGraph graphs_[2][kStepForms];
   bool graph_valid_ = false;  // false: every graph must be re-captured
 
   gbr_draw_stats last_stats_{};
