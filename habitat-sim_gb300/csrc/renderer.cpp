@@ -1043,16 +1043,9 @@ gbr_status Renderer::upload_tables(cudaStream_t stream) {
 // SM, on 128 x 64 regions with boxes of up to 4 px left to one lane: while one
 // CTA waits at a barrier the other issues (1024 textured 128 x 128 views: 1554
 // us against 2190 with one 1024-thread CTA per SM, 512 mixed views 603 against
-// 751).  A draw too small for a region of 16 x 32 px on every other SM
+// 751).  A renderer too small for a region of 16 x 32 px on every other SM
 // takes 1024 threads per CTA: then the threads per region bound it (2 views:
-// 44 us against 51).  The per-scene form has a fixed region for all scenes,
-// taller than wide: the costly parts of a view lie side by side, around its
-// horizon, so that a tall region holds its share of them and a wide one all or
-// nothing (48 furnished 160 x 120 views: 32 x 64 regions 303 us, 64 x 32 353; 256
-// of 128 x 128: 64 x 128 750 us, 128 x 64 793).  The size is the one
-// of least region_step_cost: 48 furnished 160 x 120 views take 264 us (a bound of
-// 2.5 times the whole cost picked 64 x 64: 350), 100 of them 371 (454), 40 lit views
-// 183 (249), 80 scans 644 (1255), 4 furnished 640 x 480 views 179 (228).
+// 44 us against 51).
 void Renderer::choose_shape() {
   if (tuned_) return;
   uint64_t cells = 0;
@@ -1064,13 +1057,33 @@ void Renderer::choose_shape() {
   t.region_width = 128;
   t.region_height = 64;
   t.small_area = 4;
-  const uint64_t grid = uint64_t(sm_count_) * uint64_t(t.ctas_per_sm);
+  if (std::memcmp(&t, &tuning_, sizeof t) == 0) return;
+  tuning_ = t;
+  raster_configured_ = false;
+}
+
+// The per-scene form's region, one size for all drawn scenes, where the caller
+// set none: taller than wide, because the costly parts of a view lie side by
+// side, around its horizon, so that a tall region holds its share of them and
+// a wide one all or nothing (48 furnished 160 x 120 views: 32 x 64 regions 303
+// us, 64 x 32 353; 256 of 128 x 128: 64 x 128 750 us, 128 x 64 793).  The size is
+// the one of least region_step_cost over the drawn scenes: 48 furnished 160 x 120
+// views take 264 us (a bound of 2.5 times the whole cost picked 64 x 64: 350), 100
+// of them 371 (454), 40 lit views 183 (249), 80 scans 644 (1255), 4 furnished
+// 640 x 480 views 179 (228).
+void Renderer::choose_plain_region() {
+  if (tuned_) return;
+  const uint64_t grid = uint64_t(sm_count_) * uint64_t(tuning_.ctas_per_sm);
   const int sizes[][2] = {{64, 128}, {32, 128}, {16, 128}, {64, 64}, {32, 64}, {16, 64}, {16, 32}};
   double best = -1.0;
+  gbr_tuning t = tuning_;
   for (const auto& r : sizes) {
     uint64_t items = 0;
+    uint32_t drawn = 0;
     double total = 0.0, longest = 0.0;
     for (const SceneState& sc : scenes_) {
+      if (!sc.enabled) continue;
+      ++drawn;
       const SceneState& src = scenes_[sc.source];
       const int w = std::min(r[0], sc.width), h = std::min(r[1], sc.height);
       const uint64_t n = uint64_t((sc.width + w - 1) / w) * uint64_t((sc.height + h - 1) / h);
@@ -1081,7 +1094,7 @@ void Renderer::choose_shape() {
     }
     double cost = region_step_cost(items, total, longest, grid, r[1] > 64);
     // CTAs start in list order: unordered, the last ones may start a long item.
-    if (items > grid && scenes_.size() < 16) cost = std::max(longest, total / double(grid) + 0.4 * longest);
+    if (items > grid && drawn < 16) cost = std::max(longest, total / double(grid) + 0.4 * longest);
     if (best < 0.0 || cost < best) {
       best = cost;
       t.plain_region_width = r[0];
@@ -1091,6 +1104,48 @@ void Renderer::choose_shape() {
   if (std::memcmp(&t, &tuning_, sizeof t) == 0) return;
   tuning_ = t;
   raster_configured_ = false;
+}
+
+// The per-scene form's items: each drawn scene's viewport cut into regions, row
+// by row, staged in this draw's slot and uploaded.  (With all scenes' items and a
+// region chosen for all of them, one drawn scene of 256 took 117 us instead of
+// 41, and 46 with a fixed region of 16 x 32 and launches of its own.)
+gbr_status Renderer::upload_plain_items(cudaStream_t stream) {
+  uint64_t count = 0;
+  const int rw = tuning_.plain_region_width, rh = tuning_.plain_region_height;
+  plain_scenes_ = 0;
+  for (const SceneState& sc : scenes_) {
+    if (!sc.enabled) continue;
+    ++plain_scenes_;
+    count += uint64_t((sc.width + rw - 1) / rw) * uint64_t((sc.height + rh - 1) / rh);
+  }
+  if (count > 0xffffffffull) return fail(GBR_ERROR_INVALID_ARGUMENT, "draw: too many work items");
+  const size_t bytes = std::max<size_t>(count, 1) * sizeof(WorkItem);
+  if (!d_items_.reserve(bytes, false) || !h_items_[slot_].reserve(bytes))
+    return fail(GBR_ERROR_OUT_OF_MEMORY, "draw: out of memory for work items");
+  WorkItem* out = static_cast<WorkItem*>(h_items_[slot_].ptr);
+  uint32_t n = 0;
+  for (uint32_t s = 0; s < scenes_.size(); ++s) {
+    SceneState& sc = scenes_[s];
+    sc.plain_item = n;
+    if (!sc.enabled) continue;
+    for (int y = 0; y < sc.height; y += rh)
+      for (int x = 0; x < sc.width; x += rw) {
+        WorkItem it{};
+        it.scene = s;
+        it.x0 = uint16_t(x);
+        it.y0 = uint16_t(y);
+        it.w = uint16_t(std::min(rw, sc.width - x));
+        it.h = uint16_t(std::min(rh, sc.height - y));
+        out[n++] = it;
+      }
+  }
+  if (n)
+    GBR_CUDA(cudaMemcpyAsync(d_items_.ptr, out, n * sizeof(WorkItem), cudaMemcpyHostToDevice, stream),
+             "work item upload");
+  item_count_ = n;
+  plain_dirty_ = false;
+  return GBR_OK;
 }
 
 gbr_status Renderer::rebuild(cudaStream_t stream) {
@@ -1163,28 +1218,8 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
   for (const SceneRec& r : recs) search_ordinals_ = search_ordinals_ || r.ordinal_shift == kOrdinalRunning;
   if (search != search_ordinals_) raster_configured_ = false;
   choose_shape();
-  // Work items: each scene's viewport cut into regions.  The per-scene form
-  // has one region size, small where few scenes have to spread over the GPU;
-  // the batched form uses large ones (fewer redundant triangle setups), split
-  // and ordered longest first for the persistent grid by order_items().
-  std::vector<WorkItem> items;
-  auto tile = [&](uint32_t s, int rwm, int rhm, std::vector<WorkItem>& out) {
-    const SceneState& sc = scenes_[s];
-    for (int y = 0; y < sc.height; y += rhm)
-      for (int x = 0; x < sc.width; x += rwm) {
-        WorkItem it{};
-        it.scene = s;
-        it.x0 = uint16_t(x);
-        it.y0 = uint16_t(y);
-        it.w = uint16_t(std::min(rwm, sc.width - x));
-        it.h = uint16_t(std::min(rhm, sc.height - y));
-        out.push_back(it);
-      }
-  };
   std::vector<ItemScene> info(S);
   for (uint32_t s = 0; s < S; ++s) {
-    scenes_[s].plain_item = uint32_t(items.size());
-    tile(s, tuning_.plain_region_width, tuning_.plain_region_height, items);
     info[s].width = scenes_[s].width;
     info[s].height = scenes_[s].height;
   }
@@ -1193,7 +1228,6 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
   const uint64_t capacity =
       work_item_capacity(info, tuning_.region_width, tuning_.region_height, uint64_t(sm_count_) * 8);
   if (capacity > 0xffffffffull) return fail(GBR_ERROR_INVALID_ARGUMENT, "draw: too many work items");
-  item_count_ = uint32_t(items.size());
   lpt_count_ = uint32_t(capacity);
 
   cudaSetDevice(device_);
@@ -1210,7 +1244,6 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
       !d_vis_count_.reserve(S1 * 4, false) || !d_vis_tris_.reserve(S1 * 4, false) ||
       !d_vis_clusters_.reserve(S1 * 4, false) ||
       !d_status_.reserve(4, false) || !d_counter_.reserve(4, false) ||
-      !d_items_.reserve(std::max<size_t>(items.size(), 1) * sizeof(WorkItem), false) ||
       !d_items_lpt_.reserve((size_t(lpt_count_) + 1) * sizeof(WorkItem), false) ||
       !h_stage_[0].reserve(std::max<size_t>(camera_block_bytes(), 1) +
                            std::max<size_t>(nodes, 1) * 64 +
@@ -1226,7 +1259,6 @@ gbr_status Renderer::rebuild(cudaStream_t stream) {
   GBR_CUDA(copy(d_scenes_.ptr, recs.data(), S * sizeof(SceneRec)), "scene upload");
   GBR_CUDA(copy(d_parents_.ptr, parents.data(), parents.size() * 4), "scene upload");
   GBR_CUDA(copy(d_draws_.ptr, draws.data(), draws.size() * sizeof(DrawRec)), "scene upload");
-  GBR_CUDA(copy(d_items_.ptr, items.data(), items.size() * sizeof(WorkItem)), "scene upload");
   GBR_CUDA(cudaMemsetAsync(d_status_.ptr, 0, 4, stream), "scene upload");
   // The order kernel's count of finished CTAs, behind the list's item count
   // (which upload_step() writes).
@@ -1309,6 +1341,8 @@ gbr_status Renderer::upload_step(cudaStream_t stream, uint32_t mode) {
     order_items();
     bindings_dirty_ = false;
   }
+  if (mode != GBR_DRAW_BATCHED && plain_dirty_)
+    if (gbr_status st = upload_plain_items(stream)) return st;
   CameraRec* cams = reinterpret_cast<CameraRec*>(stage);
   for (uint32_t s = 0; s < S; ++s) {
     const SceneState& sc = scenes_[s];
@@ -1554,10 +1588,10 @@ gbr_status Renderer::enqueue_step(cudaStream_t stream, uint32_t mode) {
     rp.item_base = 0;
     rp.item_count = item_count_;
     GBR_CUDA(launch_prepare(pp, S, stream), "prepare launch");
-    launches = 2;
+    launches = item_count_ ? 2 : 1;
     // CTAs start in the order of the items: launches of several waves are
     // ordered like the batched form's.
-    if (plain_ordered(S, item_count_) && std::max(item_count_, lpt_items_) <= ordered_capacity()) {
+    if (plain_ordered(plain_scenes_, item_count_) && std::max(item_count_, lpt_items_) <= ordered_capacity()) {
       if (gbr_status st = enqueue_order(rp, true, stream)) return st;
       rp.items = d_items_lpt_.as<WorkItem>();
       rp.item_base = ordered_capacity();
@@ -1575,6 +1609,8 @@ gbr_status Renderer::draw(cudaStream_t stream, uint32_t mode, bool use_graph) {
   if (use_graph && mode == GBR_DRAW_BATCHED && stream == nullptr) stream = own_stream_;
   if (structure_dirty_)
     if (gbr_status s = rebuild(stream)) return s;
+  if (bindings_dirty_) plain_dirty_ = true;  // the scenes that are drawn, or what they show, changed
+  if (mode != GBR_DRAW_BATCHED && plain_dirty_) choose_plain_region();
   if (gbr_status s = ensure_raster_config()) return s;
   if (tables_dirty_)
     if (gbr_status s = upload_tables(stream)) return s;

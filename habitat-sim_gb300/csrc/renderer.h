@@ -185,6 +185,8 @@ class Renderer {
   gbr_status enqueue_step(cudaStream_t stream, uint32_t mode);
   gbr_status ensure_raster_config();
   void choose_shape();
+  void choose_plain_region();
+  gbr_status upload_plain_items(cudaStream_t stream);
   void build_chunk_boxes(uint32_t first_view, uint32_t last_view);
   void* plane_ptr(uint32_t plane, size_t* elem) const;
   gbr_status sync_and_check();
@@ -248,6 +250,7 @@ class Renderer {
   // that the host stages draw k + 1 while draw k runs; upload_done_[slot]
   // follows the whole step that last used the slot.
   PinnedBuffer h_stage_[2];
+  PinnedBuffer h_items_[2];  // the per-scene form's items, by slot
   PinnedBuffer h_mesh_stage_;  // addMesh uploads
   cudaEvent_t upload_done_[2] = {nullptr, nullptr};
   bool upload_pending_[2] = {false, false};
@@ -257,7 +260,9 @@ class Renderer {
 
   uint32_t total_nodes_ = 0, total_draws_ = 0;
   uint64_t total_tris_ = 0;
-  uint32_t item_count_ = 0;
+  uint32_t item_count_ = 0;    // per-scene form: items of the drawn scenes
+  uint32_t plain_scenes_ = 0;  // per-scene form: drawn scenes
+  bool plain_dirty_ = true;    // per-scene form: the list follows other bindings
   uint32_t lpt_count_ = 0;  // batched form: capacity of the item list (every scene at its finest split)
   uint32_t lpt_items_ = 0;  // batched form: items in the current list
   // Batched form: how the current list is drawn.  Whole and Small: in the host's
