@@ -29,12 +29,17 @@
 #include <vector>
 
 #include "../../include/gbr_noise.h"
+#include "noise_plan.h"
 
 namespace gbr {
 void set_last_error(const std::string& msg);
 }
 
 namespace {
+
+using gbr::kNoisePlainThreads;
+using gbr::kNoiseTableThreads;
+using gbr::NoisePlan;
 
 constexpr int kModelCols = 80, kModelDims = 5;
 constexpr int kModelFloats = 80 * kModelCols * kModelDims;
@@ -187,24 +192,25 @@ __device__ __forceinline__ void noise_pixel(const TileArgs& a, int img, int idx,
   dst[uint64_t(uint32_t(r)) * uint64_t(pitch) + uint32_t(col)] = out;
 }
 
-// Images as the tiles of a grid, cut into chunks of pixels that the blocks
-// walk: unit u is chunk u % chunks of image u / chunks.
+// Images as the tiles of a grid, cut into chunks of pixels that the blocks walk
+// (NoisePlan).
 //
 // Bound by instruction issue (73 %, 211 instructions per 32 pixels): Philox' ten
 // rounds and what the arithmetic above fixes.  With Table, blocks of 1024
 // threads, two per SM, first fill 44 KB of shared memory with what would be
 // gathers from L1 (28 lines per warp and variate), two divisions per pixel for
-// the model's cell and one for the output; filling it takes a few microseconds,
-// so only batches of kTablePixels and more do (64 images of 128 x 128: 14.4 us
-// against 16.5 without; 32: 11.7 against 10.3; 1024: 130 against 203).
-constexpr int kTableThreads = 1024, kPlainThreads = 256;
-constexpr uint64_t kTablePixels = 1u << 20;
-template <bool Table>
-__global__ void __launch_bounds__(Table ? kTableThreads : kPlainThreads, Table ? 2 : 8)
-    redwood_kernel(const TileArgs a, const Divisor width, const Divisor chunks, uint32_t units, int chunk) {
+// the model's cell and one for the output; filling it takes a few microseconds
+// (1024 images of 128 x 128: 130 us against 203).
+template <NoisePlan::Form F>
+__global__ void __launch_bounds__(F >= NoisePlan::kTable ? kNoiseTableThreads : kNoisePlainThreads,
+                                  F >= NoisePlan::kTable ? 2 : 8)
+    redwood_kernel(const TileArgs a, const Divisor width, const Divisor split, uint32_t pack, uint32_t units,
+                   int chunk) {
+  constexpr bool Table = F >= NoisePlan::kTable, Packed = F == NoisePlan::kPacked,
+                 Spread = F == NoisePlan::kTableSpread;
   extern __shared__ __align__(16) unsigned char smem[];
   Tables* t = reinterpret_cast<Tables*>(smem);
-  constexpr int kThreads = Table ? kTableThreads : kPlainThreads;
+  constexpr int kThreads = Table ? kNoiseTableThreads : kNoisePlainThreads;
   const bool cells = a.tw <= kCells && a.th <= kCells - a.tw;
   if (Table) {
     for (int k = threadIdx.x; k < kSegments; k += kThreads) {
@@ -218,11 +224,23 @@ __global__ void __launch_bounds__(Table ? kTableThreads : kPlainThreads, Table ?
     __syncthreads();
   }
   const int pixels = a.tw * a.th;
+  // Packed: this thread's image of the unit, and its pixel of that.
+  const uint32_t sub = Packed ? threadIdx.x / uint32_t(pixels) : 0u;
+  const int pixel = int(threadIdx.x - sub * uint32_t(pixels));
+  if (Packed && sub >= pack) return;
   for (uint32_t u = blockIdx.x; u < units; u += gridDim.x) {
-    const uint32_t img = chunks.divide(u);
+    uint32_t img, part = 0u;
+    if (Packed) {
+      img = u * pack + sub;
+      if (img >= uint32_t(a.count)) break;
+    } else {
+      const uint32_t q = split.divide(u), rest = u - q * split.d;
+      img = Spread ? rest : q;
+      part = Spread ? q : rest;
+    }
     const long long base = (long long)(img / a.tiles_x) * a.th * a.pitch + (long long)(img % a.tiles_x) * a.tw;
-    const long long first = (long long)(u - img * chunks.d) * chunk;
-    for (int k = threadIdx.x; k < chunk; k += kThreads) {
+    const long long first = (long long)part * chunk;
+    for (int k = pixel; k < chunk; k += kThreads) {
       if (first + k >= pixels) break;
       const int idx = int(first) + k, r = int(width.divide(uint32_t(idx)));
       noise_pixel<Table>(a, int(img), idx, r, idx - r * a.tw, a.src + base, a.dst + base, a.pitch, a.tw, a.th, t, cells);
@@ -350,22 +368,19 @@ TileArgs make_args(gbr_redwood_noise* m, const float* src, float* dst, long long
 
 gbr_status launch(gbr_redwood_noise* m, const float* src, float* dst, long long pitch, int tw, int th,
                   int tiles_x, int count, cudaStream_t stream) {
-  const uint64_t pixels = uint64_t(tw) * uint64_t(th), total = pixels * uint64_t(count);
-  const bool table = total >= kTablePixels;
-  // Chunks of four pixels per thread where that leaves every block several.
-  const uint64_t chunk = !table ? kPlainThreads : kTableThreads * (total >= 4 * kTablePixels ? 4 : 1), chunks = (pixels + chunk - 1) / chunk;
-  const uint64_t units = chunks * uint64_t(count);
-  if (units > 0xffffffffull)
+  const NoisePlan p = gbr::noise_plan(uint32_t(tw), uint32_t(th), uint32_t(count), uint32_t(m->sms));
+  if (p.units > 0xffffffffull)
     return fail(GBR_ERROR_INVALID_ARGUMENT, "RedwoodNoiseModel: too many pixels in one batch");
   const TileArgs a = make_args(m, src, dst, pitch, tw, th, tiles_x, count);
-  const Divisor width = make_divisor(uint32_t(tw)), per_image = make_divisor(uint32_t(chunks));
-  const unsigned resident = unsigned(2 * m->sms);
-  if (table)
-    redwood_kernel<true><<<unsigned(std::min<uint64_t>(units, resident)), kTableThreads, sizeof(Tables), stream>>>(
-        a, width, per_image, uint32_t(units), int(chunk));
-  else
-    redwood_kernel<false><<<unsigned(std::min<uint64_t>(units, 0x7fffffffu)), kPlainThreads, 0, stream>>>(
-        a, width, per_image, uint32_t(units), int(chunk));
+  const Divisor width = make_divisor(uint32_t(tw)),
+                split = make_divisor(p.form == NoisePlan::kTableSpread ? uint32_t(count) : p.chunks);
+  const auto kernel = p.form == NoisePlan::kTable         ? redwood_kernel<NoisePlan::kTable>
+                      : p.form == NoisePlan::kTableSpread ? redwood_kernel<NoisePlan::kTableSpread>
+                      : p.form == NoisePlan::kPacked      ? redwood_kernel<NoisePlan::kPacked>
+                                                          : redwood_kernel<NoisePlan::kPlain>;
+  const bool table = p.form >= NoisePlan::kTable;
+  kernel<<<p.grid, table ? kNoiseTableThreads : kNoisePlainThreads, table ? sizeof(Tables) : 0, stream>>>(
+      a, width, split, p.pack, uint32_t(p.units), int(p.chunk));
   if (cudaError_t e = cudaGetLastError()) return cuda_fail(e, "redwood noise launch");
   return GBR_OK;
 }
