@@ -140,6 +140,7 @@ PROTOTYPES = {
     "gbr_unproject_depth_device": (_ST, [c_float_p, _P, _U64, _U64, _U64, _P]),
     "gbr_get_tuning": (_ST, [_P, ctypes.POINTER(Tuning)]),
     "gbr_set_tuning": (_ST, [_P, ctypes.POINTER(Tuning)]),
+    "gbr_set_tuning_fields": (_ST, [_P, ctypes.POINTER(Tuning), _U32]),
     "gbr_last_draw_stats": (_ST, [_P, ctypes.POINTER(DrawStats)]),
     "gbr_set_kernel_timing": (_ST, [_P, _I32]),
     "gbr_set_device_memory_limit": (_ST, [_P, _U64]),

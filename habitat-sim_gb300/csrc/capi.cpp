@@ -426,6 +426,12 @@ gbr_status gbr_set_tuning(gbr_renderer* r, const gbr_tuning* t) {
   return R(r)->set_tuning(*t);
 }
 
+gbr_status gbr_set_tuning_fields(gbr_renderer* r, const gbr_tuning* t, uint32_t fields) {
+  GBR_HANDLE(r);
+  GBR_ARG(t);
+  return R(r)->set_tuning(*t, fields);
+}
+
 gbr_status gbr_last_draw_stats(gbr_renderer* r, gbr_draw_stats* out) {
   GBR_HANDLE(r);
   GBR_ARG(out);

@@ -1039,31 +1039,33 @@ gbr_status Renderer::upload_tables(cudaStream_t stream) {
   return GBR_OK;
 }
 
-// Launch shape of a renderer whose caller set none.  512-thread CTAs, two per
+// Launch shape: the fields that the caller did not set.  512-thread CTAs, two per
 // SM, on 128 x 64 regions with boxes of up to 4 px left to one lane: while one
 // CTA waits at a barrier the other issues (1024 textured 128 x 128 views: 1554
 // us against 2190 with one 1024-thread CTA per SM, 512 mixed views 603 against
 // 751).  A renderer too small for a region of 16 x 32 px on every other SM
 // takes 1024 threads per CTA: then the threads per region bound it (2 views:
-// 44 us against 51).
+// 44 us against 51).  So does a caller's region too large for two z-buffers in an
+// SM's shared memory; a caller's 256 threads get regions of 64 x 64.
 void Renderer::choose_shape() {
-  if (tuned_) return;
   uint64_t cells = 0;
   for (const SceneState& sc : scenes_) cells += uint64_t((sc.width + 15) / 16) * uint64_t((sc.height + 31) / 32);
-  const bool few = 2 * cells <= uint64_t(sm_count_);
   gbr_tuning t = tuning_;
-  t.threads = few ? 1024 : 512;
-  t.ctas_per_sm = few ? 1 : 2;
-  t.region_width = 128;
-  t.region_height = 64;
-  t.small_area = 4;
+  const bool w = tuned_ & kRegionWidth, h = tuned_ & kRegionHeight;
+  const bool narrow = (tuned_ & kThreads) && t.threads == 256;
+  if (!w) t.region_width = h ? std::max(4, std::min(128, 8192 / t.region_height)) : narrow ? 64 : 128;
+  if (!h) t.region_height = w ? std::max(1, std::min(64, 8192 / t.region_width)) : 64;
+  const bool whole = 2 * cells <= uint64_t(sm_count_) || t.region_width * t.region_height > 8192;
+  if (!(tuned_ & kThreads)) t.threads = whole ? 1024 : 512;
+  if (!(tuned_ & kCtasPerSm)) t.ctas_per_sm = 1024 / t.threads;
+  if (!(tuned_ & kSmallArea)) t.small_area = 4;
   if (std::memcmp(&t, &tuning_, sizeof t) == 0) return;
   tuning_ = t;
   raster_configured_ = false;
 }
 
-// The per-scene form's region, one size for all drawn scenes, where the caller
-// set none: taller than wide, because the costly parts of a view lie side by
+// The per-scene form's region, one size for all drawn scenes, as far as the caller
+// did not set it: taller than wide, because the costly parts of a view lie side by
 // side, around its horizon, so that a tall region holds its share of them and
 // a wide one all or nothing (48 furnished 160 x 120 views: 32 x 64 regions 303
 // us, 64 x 32 353; 256 of 128 x 128: 64 x 128 750 us, 128 x 64 793).  The size is
@@ -1072,12 +1074,15 @@ void Renderer::choose_shape() {
 // of them 371 (454), 40 lit views 183 (249), 80 scans 644 (1255), 4 furnished
 // 640 x 480 views 179 (228).
 void Renderer::choose_plain_region() {
-  if (tuned_) return;
+  if ((tuned_ & kPlainWidth) && (tuned_ & kPlainHeight)) return;
   const uint64_t grid = uint64_t(sm_count_) * uint64_t(tuning_.ctas_per_sm);
   const int sizes[][2] = {{64, 128}, {32, 128}, {16, 128}, {64, 64}, {32, 64}, {16, 64}, {16, 32}};
   double best = -1.0;
   gbr_tuning t = tuning_;
-  for (const auto& r : sizes) {
+  for (const auto& size : sizes) {
+    const int r[2] = {tuned_ & kPlainWidth ? t.plain_region_width : size[0],
+                      tuned_ & kPlainHeight ? t.plain_region_height : size[1]};
+    if (r[0] * r[1] > 16384 && (best >= 0.0 || &size != std::end(sizes) - 1)) continue;
     uint64_t items = 0;
     uint32_t drawn = 0;
     double total = 0.0, longest = 0.0;
@@ -1968,22 +1973,40 @@ gbr_status Renderer::set_kernel_timing(bool on) {
   return GBR_OK;
 }
 
-gbr_status Renderer::get_tuning(gbr_tuning* t) const {
+gbr_status Renderer::get_tuning(gbr_tuning* t) {
+  if (structure_dirty_)  // what the choices go by, as the next draw will find it
+    for (SceneState& sc : scenes_) {
+      sc.tri_count = 0;
+      for (const HostDraw& d : sc.draws) sc.tri_count += d.index_count / 3;
+      sc.draw_count = uint32_t(sc.draws.size());
+    }
+  choose_shape();
+  choose_plain_region();
   *t = tuning_;
   return GBR_OK;
 }
 
-gbr_status Renderer::set_tuning(const gbr_tuning& t) {
+gbr_status Renderer::set_tuning(const gbr_tuning& given, uint32_t fields) {
+  static_assert(sizeof(gbr_tuning) == 9 * sizeof(int32_t), "one bit per member");
+  gbr_tuning t = tuning_;
+  fields &= kAllFields;
+  for (int k = 0; k < 9; ++k)
+    if (fields >> k & 1u)
+      std::memcpy(reinterpret_cast<int32_t*>(&t) + k, reinterpret_cast<const int32_t*>(&given) + k, 4);
+  const uint32_t set = tuned_ | fields;
+  const auto both = [&](uint32_t a, uint32_t b) { return (set & a) && (set & b); };
   if ((t.threads != 256 && t.threads != 512 && t.threads != 1024) || t.region_width < 4 ||
       t.region_height < 1 || t.region_width > 1024 || t.region_height > 1024 ||
-      t.region_width * t.region_height > 32768 || t.small_area < 1 || t.ctas_per_sm < 1 ||
-      t.plain_region_width < 4 || t.plain_region_height < 1 || t.plain_region_width > 1024 ||
-      t.plain_region_height > 1024 || t.plain_region_width * t.plain_region_height > 32768 ||
+      (both(kRegionWidth, kRegionHeight) && t.region_width * t.region_height > 32768) || t.small_area < 1 ||
+      t.ctas_per_sm < 1 || t.plain_region_width < 4 || t.plain_region_height < 1 || t.plain_region_width > 1024 ||
+      t.plain_region_height > 1024 ||
+      (both(kPlainWidth, kPlainHeight) && t.plain_region_width * t.plain_region_height > 32768) ||
       t.occlusion_culling < 0 || t.occlusion_culling > 1 || t.queue_fill_percent < 25 ||
       t.queue_fill_percent > 100)
     return fail(GBR_ERROR_INVALID_ARGUMENT, "setTuning: out of range");
+  if (!fields) return GBR_OK;
   tuning_ = t;
-  tuned_ = true;
+  tuned_ = set;
   raster_configured_ = false;
   structure_dirty_ = true;  // regions change
   return GBR_OK;

@@ -141,6 +141,18 @@ class Renderer {
   gbr_status light_ranges(uint32_t scene, float** out, uint64_t* count);
   gbr_status set_enabled(uint32_t scene, bool enabled);
 
+  // Bits of gbr_tuning's members.
+  enum : uint32_t {
+    kThreads = 1,
+    kRegionWidth = 2,
+    kRegionHeight = 4,
+    kSmallArea = 8,
+    kCtasPerSm = 16,
+    kPlainWidth = 32,
+    kPlainHeight = 64,
+    kAllFields = 511,
+  };
+
   // -- drawing
   gbr_status draw(cudaStream_t stream, uint32_t mode, bool use_graph);
   // Ambient occlusion on the colour plane of every enabled scene of the last draw.
@@ -154,8 +166,9 @@ class Renderer {
   gbr_status scene_image_into(uint32_t plane, uint32_t scene, void* dst, uint64_t row_bytes);
   gbr_status plane_pointer(uint32_t plane, void** out, uint64_t* bytes);
   gbr_status plane_dlpack(uint32_t plane, void** out);
-  gbr_status get_tuning(gbr_tuning* t) const;
-  gbr_status set_tuning(const gbr_tuning& t);
+  gbr_status get_tuning(gbr_tuning* t);
+  // The fields whose bits are set (bit k: the k-th member); the rest stay as they are.
+  gbr_status set_tuning(const gbr_tuning& t, uint32_t fields = kAllFields);
   gbr_status last_stats(gbr_draw_stats* out);
   gbr_status set_kernel_timing(bool on);
   gbr_status set_memory_limit(uint64_t bytes);
@@ -276,8 +289,8 @@ class Renderer {
   bool items_staged_ = false;            // a new item order waits in the staging buffer
   uint64_t vis_needed_ = 0;              // visible records the current bindings need
 
-  gbr_tuning tuning_{1024, 128, 128, 1, 1, 16, 32, 1, 75};
-  bool tuned_ = false;  // set by the caller: choose_shape() keeps out
+  gbr_tuning tuning_{512, 128, 64, 4, 2, 16, 32, 1, 75};
+  uint32_t tuned_ = 0;  // fields set by the caller (bits): the others are choose_shape()'s and choose_plain_region()'s
   size_t smem_plain_ = 0;
   bool search_ordinals_ = false;  // some scene's triangle ordinals do not name their draw
   int prefix_cap_ = 0;

@@ -596,11 +596,14 @@ class RendererStandalone:
         return {k: int(getattr(t, k)) for k, _ in _lib.Tuning._fields_}
 
     def setTuning(self, **kw):
+        """Sets the named fields; the others stay as set before, or the library's choice."""
         t = _lib.Tuning()
-        check(self._lib.gbr_get_tuning(self._h, ctypes.byref(t)))
-        for k, v in kw.items():
-            setattr(t, k, int(v))
-        check(self._lib.gbr_set_tuning(self._h, ctypes.byref(t)))
+        fields = 0
+        for k, (name, _) in enumerate(_lib.Tuning._fields_):
+            if name in kw:
+                setattr(t, name, int(kw[name]))
+                fields |= 1 << k
+        check(self._lib.gbr_set_tuning_fields(self._h, ctypes.byref(t), fields))
 
     # ------------------------------------------------------------ images
     def _image(self, plane, dtype, channels=None):

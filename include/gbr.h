@@ -332,8 +332,14 @@ typedef struct gbr_tuning {
                                   of them, so that larger shares mean a full
                                   queue)                                    */
 } gbr_tuning;
+/* What the caller set, and the library's own choice for the rest (also before
+ * the first draw; it follows the renderer's viewports and drawn scenes). */
 gbr_status gbr_get_tuning(gbr_renderer* r, gbr_tuning* out);
+/* Sets every field: the library chooses none of them any more. */
 gbr_status gbr_set_tuning(gbr_renderer* r, const gbr_tuning* tuning);
+/* Sets the fields of `fields` alone (bit k: the k-th member of gbr_tuning);
+ * those not set so far stay the library's choice. */
+gbr_status gbr_set_tuning_fields(gbr_renderer* r, const gbr_tuning* tuning, uint32_t fields);
 
 /* Counters of the last draw (host-read after the stream is synchronised). */
 typedef struct gbr_draw_stats {
