@@ -375,12 +375,8 @@ class RenderServer:
         # reads one set while step k + 1 draws into the other.
         self.r = pkg.RendererStandalone(cfg, pkg.RendererStandaloneConfiguration().setCudaDevice(
             device).setFlags(pkg.RendererStandaloneFlags.QuietLog | pkg.RendererStandaloneFlags.DoubleBuffer))
-        # The launch shape that served best (two 512-thread CTAs per SM on
-        # 128 x 64 regions, 4 px small-triangle threshold: a step of 320
-        # requests over 24 scenes in 1.46 ms against 1.49 for 64 x 64 regions
-        # and 1.55 for 1024-thread CTAs); tune() picks one for the caller's
-        # own catalog.
-        self.r.setTuning(threads=512, region_width=128, region_height=64, small_area=4, ctas_per_sm=2)
+        # The launch shape is the library's choice for these viewports; tune()
+        # picks one for the caller's own catalog.
         for s in range(len(viewports)):
             self.r.setSceneEnabled(s, False)
         self.enabled = np.zeros(self.n_slots, bool)
