@@ -475,17 +475,17 @@ constexpr int kTile = 8, kCoarse = 4;
 __host__ __device__ __forceinline__ int tile_capacity(int w, int h, int side) {
   return ((w + side - 1) / side) * ((h + side - 1) / side);
 }
-// Entries of the shared triangle queue.  With 352 of them two 512-thread CTAs
+// Least entries of the shared triangle queue.  With 352 of them two 512-thread CTAs
 // on 128 x 64 regions need 196 KB of shared memory and leave 60 KB to the L1
 // cache (with 512: 228 and 28), through which the vertices, boxes and records
 // are read.
-__host__ __device__ constexpr int queue_capacity(int threads) { return threads * 11 / 16; }
+__host__ __device__ constexpr uint32_t queue_capacity(int threads) { return uint32_t(threads) * 11 / 16; }
 uint32_t align16(size_t x) { return uint32_t((x + 15) & ~size_t(15)); }
-SmemLayout smem_layout(int threads, int region_w, int region_h, int prefix_cap) {
+SmemLayout smem_layout(int threads, int region_w, int region_h, int prefix_cap, uint32_t queue_cap) {
   SmemLayout l;
   l.queue = align16(size_t(region_w) * size_t(region_h) * 8);
-  l.qoff = align16(l.queue + size_t(queue_capacity(threads)) * sizeof(QEntry));
-  l.prefix = align16(l.qoff + size_t(queue_capacity(threads) + 1) * 4);
+  l.qoff = align16(l.queue + size_t(queue_cap) * sizeof(QEntry));
+  l.prefix = align16(l.qoff + size_t(queue_cap + 1) * 4);
   l.chunks = align16(l.prefix + size_t(prefix_cap) * 4);
   l.clusters = align16(l.chunks + size_t(ring_capacity(threads)) * sizeof(uint2));
   l.tiles = align16(l.clusters + size_t(kClusterRing) * sizeof(uint2));
@@ -1525,8 +1525,8 @@ __global__ void __launch_bounds__(T, 1024 / T)
     c.queue = queue;
     c.spill = s_spill;
     c.qcount = &s_qcount;
-    constexpr uint32_t kQueue = queue_capacity(T);
-    c.qcap = kQueue;
+    const uint32_t qcap = p.queue_cap;  // at most T: a thread per entry
+    c.qcap = int(qcap);
     c.spill_cap = T;
     c.rx0 = wi.x0;
     c.ry0 = wi.y0;
@@ -1578,14 +1578,14 @@ __global__ void __launch_bounds__(T, 1024 / T)
     __syncthreads();
     for (;;) {
       const uint32_t rd = s_rd, wr = s_wr, crd = s_crd, cwr = s_cwr, next = s_next,
-                     queued = min(s_qcount, c.spill ? kQueue + uint32_t(T) : kQueue),
-                     nq = min(queued, kQueue);
+                     queued = min(s_qcount, c.spill ? qcap + uint32_t(T) : qcap),
+                     nq = min(queued, qcap);
       __syncthreads();  // everyone has read the counters
       const bool low = wr - rd < uint32_t(T / 32);
       const bool clusters_left = next < nclusters, have_clusters = cwr != crd;
       const bool need_cull = low && (clusters_left || have_clusters);
-      // A round adds at most T entries to fewer than flush_at: the queue and the
-      // spill area (T each) hold them.
+      // A round adds at most T entries (and a few where triangles are clipped) to
+      // fewer than flush_at: the queue's qcap and the spill area's T hold them.
       if (nq > 0 && (nq >= p.flush_at || need_cull || wr == rd)) {
         // ---- flush: every thread takes a contiguous run of the queued
         // triangles' bounding-box pixels.
@@ -1639,7 +1639,7 @@ __global__ void __launch_bounds__(T, 1024 / T)
           // A round queued more than the shared queue holds: the rest went to
           // this CTA's spill area; move it into the emptied queue.
           // (What does not fit follows at the next flush, which comes at once.)
-          const uint32_t rest = queued - nq, moved = min(rest, kQueue), from = s_moved;
+          const uint32_t rest = queued - nq, moved = min(rest, qcap), from = s_moved;
           for (uint32_t i = threadIdx.x; i < moved; i += T) queue[i] = c.spill[from + i];
           __syncthreads();
           if (threadIdx.x == 0) {
@@ -2023,12 +2023,16 @@ cudaError_t launch_order(const RasterParams& p, uint32_t scene_count, WorkItem* 
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-size_t raster_smem_bytes(int threads, int region_w, int region_h, int prefix_cap) {
-  return smem_layout(threads, region_w, region_h, prefix_cap).total;
+size_t raster_smem_bytes(int threads, int region_w, int region_h, int prefix_cap, uint32_t queue_cap) {
+  return smem_layout(threads, region_w, region_h, prefix_cap, queue_cap).total;
+}
+
+uint32_t raster_queue_cap(int threads, int percent) {
+  return std::max(queue_capacity(threads), percent > 75 ? uint32_t(threads * percent / 100) : 0u);
 }
 
 uint32_t raster_flush_at(int threads, int percent) {
-  return uint32_t(std::max(1, std::min(threads * percent / 100, queue_capacity(threads))));
+  return std::max(1u, std::min(uint32_t(threads * percent / 100), raster_queue_cap(threads, percent)));
 }
 
 size_t raster_spill_bytes(int threads, uint32_t grid) {
@@ -2086,7 +2090,7 @@ cudaError_t launch_raster(const RasterParams& p, int threads, uint32_t grid, siz
   // Programmatic dependent launch: the CTAs start while the kernel before
   // them finishes and wait for it in the kernel, which takes the launch's own
   // latency (2-3 us of a small draw's 40-50) off the path.
-  const SmemLayout layout = smem_layout(threads, p.region_w, p.region_h, p.prefix_cap);
+  const SmemLayout layout = smem_layout(threads, p.region_w, p.region_h, p.prefix_cap, p.queue_cap);
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -2368,7 +2372,7 @@ extern "C" gbr_status gbr_render_mesh_no_alloc(
   constexpr int kThreads = 1024;
   size_t max_dyn = 0, static_bytes = 0;
   e = raster_configure(kThreads, &max_dyn, &static_bytes);
-  const size_t smem = raster_smem_bytes(kThreads, kNoAllocRegion, kNoAllocRegion, 1);
+  const size_t smem = raster_smem_bytes(kThreads, kNoAllocRegion, kNoAllocRegion, 1, raster_queue_cap(kThreads, 75));
   int occ = 0, sms = 0;
   if (e == cudaSuccess) e = raster_max_ctas_per_sm(kThreads, smem, &occ);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -2404,6 +2408,7 @@ extern "C" gbr_status gbr_render_mesh_no_alloc(
   p.region_w = p.region_h = kNoAllocRegion;
   p.prefix_cap = 1;
   p.small_area = 1;
+  p.queue_cap = raster_queue_cap(kThreads, 75);
   p.flush_at = raster_flush_at(kThreads, 75);
   const uint32_t grid = std::min<uint32_t>(a.items, uint32_t(sms) * uint32_t(occ));
   e = launch_raster(p, kThreads, grid, smem, false, st);

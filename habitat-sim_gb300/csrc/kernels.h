@@ -84,6 +84,7 @@ struct RasterParams {
   int32_t prefix_cap;  // visible draws whose ordinals are cached in shared memory
   int32_t small_area;  // boxes up to this many pixels are rasterised by one lane
   int32_t occlusion;   // skip chunks hidden behind the depths written so far
+  uint32_t queue_cap;  // entries of the shared queue (raster_queue_cap)
   uint32_t flush_at;   // the queue is rasterised once it holds this many triangles (raster_flush_at)
   // Lighting (max_lights > 0): lights per scene, per-draw model data, normals.
   const WorldLight* lights;
@@ -109,9 +110,11 @@ cudaError_t launch_prepare(const PrepareParams& p, uint32_t scene_count, cudaStr
 // launch_raster.
 cudaError_t launch_order(const RasterParams& p, uint32_t scene_count, WorkItem* sorted, uint32_t* keys, uint32_t* done,
                          uint32_t grid, bool early, cudaStream_t stream);
-size_t raster_smem_bytes(int threads, int region_w, int region_h, int prefix_cap);
-// Triangles at which a CTA rasterises its queue: `percent` of its threads, at
-// most what the queue holds.
+size_t raster_smem_bytes(int threads, int region_w, int region_h, int prefix_cap, uint32_t queue_cap);
+// Entries of a CTA's triangle queue (11/16 of its threads, or `percent` of them
+// above 75), and how many make it rasterise them: `percent` of its threads, at most
+// what the queue holds.
+uint32_t raster_queue_cap(int threads, int percent);
 uint32_t raster_flush_at(int threads, int percent);
 // Bytes of the queue spill area for `grid` CTAs of `threads` threads.
 size_t raster_spill_bytes(int threads, uint32_t grid);

@@ -1296,9 +1296,11 @@ gbr_status Renderer::ensure_raster_config() {
   // Shared memory not used by the launch is L1 cache: no table of ordinals
   // unless a scene needs it.
   int cap = search_ordinals_ ? kPrefixCapMax : 0;
+  queue_cap_ = raster_queue_cap(tuning_.threads, tuning_.queue_fill_percent);
   const auto need = [&](bool plain) {
-    return plain ? raster_smem_bytes(tuning_.threads, tuning_.plain_region_width, tuning_.plain_region_height, cap)
-                 : raster_smem_bytes(tuning_.threads, tuning_.region_width, tuning_.region_height, cap);
+    return plain ? raster_smem_bytes(tuning_.threads, tuning_.plain_region_width, tuning_.plain_region_height, cap,
+                                     queue_cap_)
+                 : raster_smem_bytes(tuning_.threads, tuning_.region_width, tuning_.region_height, cap, queue_cap_);
   };
   while (std::max(need(false), need(true)) > budget && cap > 64) cap /= 2;
   if (std::max(need(false), need(true)) > max_dyn)
@@ -1545,6 +1547,7 @@ gbr_status Renderer::enqueue_step(cudaStream_t stream, uint32_t mode) {
   rp.spill = d_spill_.ptr;
   rp.small_area = tuning_.small_area;
   rp.occlusion = tuning_.occlusion_culling;
+  rp.queue_cap = queue_cap_;
   rp.flush_at = raster_flush_at(tuning_.threads, tuning_.queue_fill_percent);
   rp.max_lights = max_lights_;
   rp.ambient_factor = cfg_.ambient_factor;
@@ -1580,8 +1583,9 @@ gbr_status Renderer::enqueue_step(cudaStream_t stream, uint32_t mode) {
     }
     const uint32_t grid =
         std::min<uint32_t>(lpt_count_, uint32_t(sm_count_) * uint32_t(ctas_per_sm_));
-    GBR_CUDA(launch_raster(rp, tuning_.threads, grid, raster_smem_bytes(tuning_.threads, w, h, prefix_cap_), !timing_,
-                           stream), "raster launch");
+    GBR_CUDA(launch_raster(rp, tuning_.threads, grid,
+                           raster_smem_bytes(tuning_.threads, w, h, prefix_cap_, queue_cap_), !timing_, stream),
+             "raster launch");
     if (timing_) GBR_CUDA(cudaEventRecordWithFlags(ev_[2], stream, cudaEventRecordExternal), "timing event");
   } else {
     rp.items = d_items_.as<WorkItem>();

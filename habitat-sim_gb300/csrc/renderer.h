@@ -294,6 +294,7 @@ class Renderer {
   size_t smem_plain_ = 0;
   bool search_ordinals_ = false;  // some scene's triangle ordinals do not name their draw
   int prefix_cap_ = 0;
+  uint32_t queue_cap_ = 0;
   bool raster_configured_ = false;
   int ctas_per_sm_ = 1;
   int plain_ctas_per_sm_ = 1;  // CTAs of the per-scene form that can be resident on an SM

@@ -328,9 +328,9 @@ typedef struct gbr_tuning {
   int32_t queue_fill_percent;  /* bin capacity in use: the CTA rasterises
                                   its shared triangle queue once it holds
                                   this share of its `threads` entries,
-                                  25..100 (default 75; the queue holds 11/16
-                                  of them, so that larger shares mean a full
-                                  queue)                                    */
+                                  25..100 (default 75).  The queue holds
+                                  11/16 of them, so that 69 to 75 mean a full
+                                  one; above 75 it is as large as the share */
 } gbr_tuning;
 /* What the caller set, and the library's own choice for the rest (also before
  * the first draw; it follows the renderer's viewports and drawn scenes). */

@@ -24,7 +24,7 @@ static void run(uint32_t n, int w, int h, const gbr_tuning* tuning) {
   };
   fake::on_raster = [&](const RasterParams& p, int threads, uint32_t, size_t smem) {
     ++launched;
-    CHECK(smem == raster_smem_bytes(threads, p.region_w, p.region_h, p.prefix_cap));
+    CHECK(smem == raster_smem_bytes(threads, p.region_w, p.region_h, p.prefix_cap, p.queue_cap));
     CHECK((p.item_base != 0) == ordered);
     const uint32_t count = *p.item_count_dev;
     CHECK(count <= p.item_count);
