@@ -1447,16 +1447,17 @@ void Renderer::order_items() {
   // of 640 x 480: 255 us in the host's order, 267 in the device's; 24 of them:
   // 484 and 476; 24 of 128 x 128: 82 and 77).  The sorted list and the keys lie
   // in the list's unused room, so that ordering takes no memory.
-  std::vector<WorkItem> items;
-  bool ordered = false;
+  const int rw = tuning_.region_width, rh = tuning_.region_height;
   uint32_t drawn = 0;
   for (const SceneState& sc : scenes_) drawn += sc.enabled ? 1u : 0u;
-  if (drawn >= 16) {
-    items = build_work_items(info, tuning_.region_width, tuning_.region_height, grid,
-                             std::max(1u, ordered_capacity()));
-    ordered = items.size() > grid && items.size() <= ordered_capacity();
+  bool ordered = drawn >= 16;
+  ItemPlan plan;
+  if (ordered) {
+    plan = plan_work_items(info, rw, rh, grid, std::max(1u, ordered_capacity()));
+    ordered = plan.items > grid && plan.items <= ordered_capacity();
   }
-  if (!ordered) items = build_work_items(info, tuning_.region_width, tuning_.region_height, grid);
+  if (!ordered) plan = plan_work_items(info, rw, rh, grid);
+  const std::vector<WorkItem> items = emit_work_items(plan, info, grid);
   for (SceneState& sc : scenes_) sc.first_item = 0;
   if (ordered)
     for (size_t i = items.size(); i-- > 0;) scenes_[items[i].scene].first_item = uint32_t(i);

@@ -114,14 +114,6 @@ inline double region_step_cost(uint64_t items, double total, double longest, uin
   return strips ? 1.05 * time : time;
 }
 
-// Items of one scene split `level` times and the cost of the largest.
-inline void split_cost(const ItemScene& sc, int region_w, int region_h, int level, uint64_t& items, uint64_t& cost) {
-  int rw, rh;
-  split_region(sc.width, sc.height, region_w, region_h, level, rw, rh);
-  items = uint64_t((sc.width + rw - 1) / rw) * uint64_t((sc.height + rh - 1) / rh);
-  cost = item_cost(sc.tris, rw, rh, sc.width, sc.height, sc.draws);
-}
-
 // Items the list can ever hold: every scene at its finest split, plus the
 // halves of the last wave (one per resident CTA, at most `max_grid`).
 inline uint64_t work_item_capacity(const std::vector<ItemScene>& scenes, int region_w, int region_h,
@@ -136,87 +128,142 @@ inline uint64_t work_item_capacity(const std::vector<ItemScene>& scenes, int reg
   return capacity;
 }
 
-// The items of the enabled scenes for a persistent grid of `grid` CTAs,
-// longest first.  No item may cost more than a limit: a scene whose regions
-// do gets them halved (at most kMaxSplits times, or kMaxFewSplits while the
-// step has no more items than CTAs).  The limit, the largest whole region's
-// cost or one of a falling sequence below it, is the one with the least
-// step_cost: it breaks up a small viewport bound to a large scene beside light
-// ones, and spreads a few views over the whole GPU.  Then the cheapest `grid` items --
-// the last wave -- are halved (longer side, not below 32 px), so that the CTAs
-// finishing the step wait for half an item at most.  Items of equal cost are
-// grouped by geometry, so that the CTAs in flight read the same vertices from
-// L2.  Halving two waves or quartering the last one was slower than halving
-// one.
+// Scenes that are cut alike: of one size and cost.
+struct ItemClass {
+  int width, height;
+  uint64_t tris, all_tris;
+  uint32_t draws;
+  uint32_t scenes;  // how many
+  int rw, rh;       // the region chosen for them
+};
+
+// How a step is cut.
+struct ItemPlan {
+  std::vector<uint32_t> on;        // the scenes that have items
+  std::vector<uint32_t> class_of;  // of each of those
+  std::vector<ItemClass> classes;
+  uint64_t items = 0;
+  bool ordered = false;
+};
+
+// The regions of the enabled scenes for a persistent grid of `grid` CTAs.  No
+// item may cost more than a limit: a scene whose regions do gets them halved (at
+// most kMaxSplits times, or kMaxFewSplits while the step has no more items than
+// CTAs).  The limit, the largest whole region's cost or one of a falling sequence
+// below it, is the one with the least step_cost: it breaks up a small viewport
+// bound to a large scene beside light ones, and spreads a few views over the
+// whole GPU.
 // order_capacity > 0: for a list that the device orders (its keys see the
 // cameras), if that many items hold it: the limit by region_cost, regions or
-// upright strips by the same estimate, no halving of the last wave (it only adds
-// items: 1024 textured views 1617 -> 1653 us with it), the items in scene order,
-// each scene's regions row by row.
-inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scenes, int region_w, int region_h,
-                                              uint64_t grid, uint64_t order_capacity = 0) {
-  const bool ordered = order_capacity > 0;
+// upright strips by the same estimate.
+//
+// Made again whenever the drawn scenes change, on the path of a server's step,
+// so it goes by classes of scenes, and down the limits each class moves from
+// level to level once: with the list, 1024 views of 4 scenes take 50 us and of
+// 24 at three sizes 65 (an x86 core); scene by scene, 235 and 551.
+inline ItemPlan plan_work_items(const std::vector<ItemScene>& scenes, int region_w, int region_h, uint64_t grid,
+                                uint64_t order_capacity = 0) {
+  ItemPlan plan;
+  const bool ordered = plan.ordered = order_capacity > 0;
   grid = std::max<uint64_t>(grid, 1);
-  std::vector<uint32_t> on;  // the scenes that have items
-  for (uint32_t s = 0; s < scenes.size(); ++s)
-    if (scenes[s].enabled && scenes[s].width > 0 && scenes[s].height > 0) on.push_back(s);
-  // Per such scene and level, whole regions and strips: items and largest cost
-  // (levels that change nothing repeat).
+  std::vector<ItemClass>& classes = plan.classes;
+  size_t slots = 16;
+  while (slots < 2 * scenes.size()) slots *= 2;
+  std::vector<uint32_t> table(slots, 0xffffffffu);
+  plan.on.reserve(scenes.size());
+  plan.class_of.reserve(scenes.size());
+  for (uint32_t s = 0; s < scenes.size(); ++s) {
+    const ItemScene& sc = scenes[s];
+    if (!sc.enabled || sc.width <= 0 || sc.height <= 0) continue;
+    uint64_t h = sc.tris;
+    for (const uint64_t v : {uint64_t(sc.all_tris), uint64_t(sc.draws), uint64_t(sc.width) << 32 | uint32_t(sc.height)})
+      h = (h ^ (h >> 29)) * 0x9e3779b97f4a7c15ull + v;
+    h = (h ^ (h >> 32)) * 0x9e3779b97f4a7c15ull;
+    size_t at = size_t(h >> 20) & (slots - 1);
+    for (;; at = (at + 1) & (slots - 1)) {
+      if (table[at] == 0xffffffffu) {
+        table[at] = uint32_t(classes.size());
+        classes.push_back({sc.width, sc.height, sc.tris, sc.all_tris, sc.draws, 0, 0, 0});
+        break;
+      }
+      const ItemClass& c = classes[table[at]];
+      if (c.width == sc.width && c.height == sc.height && c.tris == sc.tris && c.all_tris == sc.all_tris &&
+          c.draws == sc.draws)
+        break;
+    }
+    ++classes[table[at]].scenes;
+    plan.on.push_back(s);
+    plan.class_of.push_back(table[at]);
+  }
+  // Per class and level, whole regions and strips: items of all its scenes and
+  // largest cost (levels that change nothing repeat).
   struct Level {
     uint64_t items, cost;
     double longest;
   };
+  const size_t C = classes.size();
   const int deepest = ordered ? kMaxSplits : kMaxFewSplits;
   std::vector<Level> levels[2];
-  auto level_of = [&](size_t n, bool strips, uint64_t t, int most) {
-    const Level* l = &levels[strips][n * size_t(deepest + 1)];
-    int k = 0;
-    while (k < most && l[k].cost > t) ++k;
-    return k;
-  };
   int max_splits = kMaxSplits;
   double best = -1.0;
   uint64_t best_limit = 0;
   bool tall = false;
-  auto region = [&](uint32_t s, int level, bool strips, int& rw, int& rh) {
+  auto region = [&](const ItemClass& c, int level, bool strips, int& rw, int& rh) {
     // (Whole regions stay as they are; 32 x 32 regions are worse than strips.)
-    ((strips && level > 0) || (ordered && level > 2) ? split_region_tall : split_region)(
-        scenes[s].width, scenes[s].height, region_w, region_h, level, rw, rh);
+    ((strips && level > 0) || (ordered && level > 2) ? split_region_tall : split_region)(c.width, c.height, region_w,
+                                                                                         region_h, level, rw, rh);
   };
+  std::vector<uint8_t> at(C);            // level of each class at the limit
+  std::vector<uint64_t> cost_at(C);      // and what it costs there
+  std::vector<double> longest_at(C);
   for (const bool strips : {false, true}) {
     if (strips && !ordered) break;
     uint64_t limit = 1;
-    levels[strips].resize(on.size() * size_t(deepest + 1), Level{0, 0, 0.0});
-    for (size_t n = 0; n < on.size(); ++n) {
-      const ItemScene& sc = scenes[on[n]];
+    levels[strips].resize(C * size_t(deepest + 1), Level{0, 0, 0.0});
+    for (size_t n = 0; n < C; ++n) {
+      const ItemClass& c = classes[n];
       Level* l = &levels[strips][n * size_t(deepest + 1)];
       for (int k = 0; k <= deepest; ++k) {
-        if (!ordered) {
-          split_cost(sc, region_w, region_h, k, l[k].items, l[k].cost);
-          continue;
-        }
         int rw, rh;
-        region(on[n], k, strips, rw, rh);
-        l[k].items = uint64_t((sc.width + rw - 1) / rw) * uint64_t((sc.height + rh - 1) / rh);
-        l[k].cost = region_cost(std::max(sc.all_tris, sc.tris), rw, rh, sc.width, sc.height, sc.draws, l[k].longest);
+        region(c, k, strips, rw, rh);
+        l[k].items = uint64_t((c.width + rw - 1) / rw) * uint64_t((c.height + rh - 1) / rh) * c.scenes;
+        l[k].cost = ordered ? region_cost(std::max(c.all_tris, c.tris), rw, rh, c.width, c.height, c.draws, l[k].longest)
+                            : item_cost(c.tris, rw, rh, c.width, c.height, c.draws);
       }
       limit = std::max(limit, l[0].cost);
     }
     for (int most : {kMaxSplits, kMaxFewSplits}) {
       if (ordered && most > kMaxSplits) break;
+      uint64_t items = 0, total = 0;
+      bool few = false;
+      for (size_t n = 0; n < C; ++n) {
+        const Level& l = levels[strips][n * size_t(deepest + 1)];
+        at[n] = 0;
+        cost_at[n] = l.cost;
+        longest_at[n] = l.longest;
+        items += l.items;
+        total += l.items * l.cost;
+      }
       uint64_t t = limit;
       for (int i = 0; i < 28 && t > 0; ++i, t = t * 17 / 20) {
-        uint64_t items = 0, total = 0, largest = 0;
+        uint64_t largest = 0;
         double longest = 0.0;
-        bool few = false;
-        for (size_t n = 0; n < on.size(); ++n) {
-          const Level* l = &levels[strips][n * size_t(deepest + 1)];
-          const int k = level_of(n, strips, t, most);
-          few = few || k > kMaxSplits;
-          items += l[k].items;
-          total += l[k].items * l[k].cost;
-          largest = std::max(largest, l[k].cost);
-          longest = std::max(longest, l[k].longest);
+        for (size_t n = 0; n < C; ++n) {
+          if (cost_at[n] > t && at[n] < most) {
+            const Level* l = &levels[strips][n * size_t(deepest + 1)];
+            int k = at[n];
+            items -= l[k].items;
+            total -= l[k].items * l[k].cost;
+            while (k < most && l[k].cost > t) ++k;
+            items += l[k].items;
+            total += l[k].items * l[k].cost;
+            few = few || k > kMaxSplits;
+            at[n] = uint8_t(k);
+            cost_at[n] = l[k].cost;
+            longest_at[n] = l[k].longest;
+          }
+          largest = std::max(largest, cost_at[n]);
+          longest = std::max(longest, longest_at[n]);
         }
         if (few && items > grid) break;
         if (ordered && i > 0 && items > order_capacity) break;
@@ -227,18 +274,41 @@ inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scen
           best_limit = t;
           max_splits = most;
           tall = strips;
+          plan.items = items;
         }
       }
     }
   }
+  for (size_t n = 0; n < C; ++n) {
+    const Level* l = &levels[tall][n * size_t(deepest + 1)];
+    int k = 0;
+    while (k < max_splits && l[k].cost > best_limit) ++k;
+    region(classes[n], k, tall, classes[n].rw, classes[n].rh);
+  }
+  return plan;
+}
+
+// The plan's items.  For a list that the device orders: in scene order, each
+// scene's regions row by row.  Else longest first, and the cheapest `grid` items
+// -- the last wave -- halved (longer side, not below 32 px), so that the CTAs
+// finishing the step wait for half an item at most.  Items of equal cost are
+// grouped by geometry, so that the CTAs in flight read the same vertices from
+// L2.  Halving two waves or quartering the last one was slower than halving one;
+// in an ordered list it only adds items (1024 textured views 1617 -> 1653 us).
+inline std::vector<WorkItem> emit_work_items(const ItemPlan& plan, const std::vector<ItemScene>& scenes, uint64_t grid) {
+  grid = std::max<uint64_t>(grid, 1);
   std::vector<WorkItem> items;
   std::vector<uint64_t> cost;
   std::vector<uint32_t> key;
-  for (size_t n = 0; n < on.size(); ++n) {
-    const uint32_t s = on[n];
+  items.reserve(plan.items + (plan.ordered ? 0 : grid));
+  if (!plan.ordered) {
+    cost.reserve(plan.items + grid);
+    key.reserve(plan.items + grid);
+  }
+  for (size_t n = 0; n < plan.on.size(); ++n) {
+    const uint32_t s = plan.on[n];
     const ItemScene& sc = scenes[s];
-    int rw, rh;
-    region(s, level_of(n, tall, best_limit, max_splits), tall, rw, rh);
+    const int rw = plan.classes[plan.class_of[n]].rw, rh = plan.classes[plan.class_of[n]].rh;
     for (int y = 0; y < sc.height; y += rh)
       for (int x = 0; x < sc.width; x += rw) {
         WorkItem it{};
@@ -248,11 +318,12 @@ inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scen
         it.w = uint16_t(std::min(rw, sc.width - x));
         it.h = uint16_t(std::min(rh, sc.height - y));
         items.push_back(it);
+        if (plan.ordered) continue;
         cost.push_back(item_cost(sc.tris, it.w, it.h, sc.width, sc.height, sc.draws));
         key.push_back(sc.geometry);
       }
   }
-  if (ordered) return items;
+  if (plan.ordered) return items;
   std::vector<uint32_t> perm(items.size());
   std::iota(perm.begin(), perm.end(), 0u);
   auto by_cost = [&](uint32_t a, uint32_t b) {
@@ -291,6 +362,11 @@ inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scen
   std::vector<WorkItem> out(items.size());
   for (size_t i = 0; i < items.size(); ++i) out[i] = items[perm[i]];
   return out;
+}
+
+inline std::vector<WorkItem> build_work_items(const std::vector<ItemScene>& scenes, int region_w, int region_h,
+                                              uint64_t grid, uint64_t order_capacity = 0) {
+  return emit_work_items(plan_work_items(scenes, region_w, region_h, grid, order_capacity), scenes, grid);
 }
 
 }  // namespace gbr
