@@ -36,6 +36,14 @@ const float kIdentity[16] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1};
 
 size_t plane_elem(uint32_t plane) { return 4; }
 
+// Host memory to the device, complete on return: cudaMemcpy may return while the
+// device's memory is still being written, on the legacy default stream, which
+// the stream of the next draw need not follow.
+cudaError_t upload(void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(nullptr);
+}
+
 int plane_slot(uint32_t plane) {
   switch (plane) {
     case GBR_PLANE_COLOR: return 0;
@@ -71,7 +79,8 @@ bool DeviceBuffer::reserve(size_t n, bool keep, cudaStream_t stream) {
     return false;
   }
   if (keep && ptr && bytes) {
-    if (cudaMemcpy(p, ptr, bytes, cudaMemcpyDeviceToDevice) != cudaSuccess) {
+    if (cudaMemcpy(p, ptr, bytes, cudaMemcpyDeviceToDevice) != cudaSuccess ||
+        cudaStreamSynchronize(nullptr) != cudaSuccess) {
       cudaFree(p);
       return false;
     }
@@ -313,8 +322,7 @@ gbr_status Renderer::debug_corrupt_parent(uint32_t scene, uint64_t node, int32_t
   cudaSetDevice(device_);
   GBR_CUDA(cudaStreamSynchronize(last_stream_), "debugCorruptParent: synchronise");
   const size_t at = size_t(scenes_[scene].node_base) + size_t(node);
-  GBR_CUDA(cudaMemcpy(d_parents_.as<int32_t>() + at, &parent, 4, cudaMemcpyHostToDevice),
-           "debugCorruptParent: write");
+  GBR_CUDA(upload(d_parents_.as<int32_t>() + at, &parent, 4), "debugCorruptParent: write");
   return GBR_OK;
 }
 
@@ -436,8 +444,7 @@ gbr_status Renderer::add_mesh(const gbr_mesh_data& m, uint32_t* id) {
   }
   // The indices need no repacking: one copy from the caller's memory.
   if (m.index_count)
-    GBR_CUDA(cudaMemcpy(d_indices_.as<char>() + size_t(ib) * 4, m.indices, size_t(m.index_count) * 4,
-                        cudaMemcpyHostToDevice),
+    GBR_CUDA(upload(d_indices_.as<char>() + size_t(ib) * 4, m.indices, size_t(m.index_count) * 4),
              "addMesh upload");
   MeshRec rec{};
   rec.vertex_base = uint32_t(vb);
@@ -498,7 +505,7 @@ gbr_status Renderer::add_texture(const gbr_texture_data& t, uint32_t* id) {
     texel_pool_.release(off, n);
     return fail(GBR_ERROR_OUT_OF_MEMORY, "addTexture: out of device memory");
   }
-  GBR_CUDA(cudaMemcpy(d_texels_.as<char>() + off * 4, data, n * 4, cudaMemcpyHostToDevice),
+  GBR_CUDA(upload(d_texels_.as<char>() + off * 4, data, n * 4),
            "addTexture upload");
   TextureRec rec{};
   rec.offset = off;

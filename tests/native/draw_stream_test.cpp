@@ -19,10 +19,17 @@ int main() {
     status = p.status;
   };
   fake::on_order = [&](const RasterParams&, uint32_t, uint32_t* done) { done_word = done; };
-  fake::on_raster = [&](const RasterParams& p, int, uint32_t, size_t) { items = *p.item_count_dev; };
+  bool resources = true;
+  fake::on_raster = [&](const RasterParams& p, int, uint32_t, size_t) {
+    items = *p.item_count_dev;
+    // What the library and the caller added before: texels, indices, boxes.
+    resources = p.texels[0] == 0xffffffffu && p.boxes[0].hi[0] == 1.0f;
+    for (uint32_t i = 0; i < 3; ++i) resources = resources && p.indices[i] == i;
+  };
   for (int round = 0; round < 2; ++round) {
     CHECK(r->draw(stream, GBR_DRAW_BATCHED, false) == GBR_OK);
     CHECK(scenes_seen == 200);
+    CHECK(resources);
     CHECK(items >= 400 && done_word && status);
     if (!done_word || !status) return 1;
     const uint32_t drawn = items;
@@ -41,6 +48,26 @@ int main() {
     gbr_draw_stats st;
     CHECK(r->last_stats(&st) == GBR_ERROR_DEVICE);
     CHECK(*status == 0);
+  }
+  // More of everything: the buffers grow, and what they held is there.
+  for (int k = 0; k < 40; ++k) {
+    const float pos[9] = {0, 0, -1, 1, 0, -1, 0, 1, -1};
+    const uint32_t idx[3] = {2, 1, 0};
+    gbr_mesh_data m{};
+    m.vertex_count = m.index_count = 3;
+    m.positions = pos;
+    m.indices = idx;
+    uint32_t id;
+    CHECK(r->add_mesh(m, &id) == GBR_OK);
+    gbr_mesh_view v{};
+    v.mesh = id;
+    v.index_count = 3;
+    CHECK(r->add_template(("t" + std::to_string(k)).c_str(), 1, &v) == GBR_OK);
+    const uint8_t texel[4] = {1, 2, 3, 4};
+    gbr_texture_data t{1, 1, 1, texel, 0, 0, 0};
+    CHECK(r->add_texture(t, &id) == GBR_OK);
+    CHECK(r->draw(stream, GBR_DRAW_BATCHED, false) == GBR_OK);
+    CHECK(resources);
   }
   delete r;
   return fake::finish();

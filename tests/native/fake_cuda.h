@@ -3,8 +3,10 @@
 //
 // Work on a created stream runs at once; work on the legacy default stream
 // waits until something has to wait for it (a synchronous copy, a blocking
-// stream, a free), as it does when another thread keeps that stream busy.
-// Work that relies on an order between the two then runs out of order.
+// stream), as it does when another thread keeps that stream busy.  A
+// synchronous copy waits for what lies before it; one to the device then returns
+// once it has read the host's memory and writes the device's later, as it may.
+// Work that relies on an order between the two streams then runs out of order.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -69,7 +71,6 @@ cudaError_t cudaMalloc(void** p, size_t n) {
   return cudaSuccess;
 }
 cudaError_t cudaFree(void* p) {
-  fake::run_legacy();
   std::free(p);
   return cudaSuccess;
 }
@@ -78,9 +79,14 @@ cudaError_t cudaFreeHost(void* p) {
   std::free(p);
   return cudaSuccess;
 }
-cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind kind) {
   fake::run_legacy();
-  std::memcpy(d, s, n);
+  if (kind == cudaMemcpyDeviceToHost) {
+    std::memcpy(d, s, n);
+  } else {
+    const std::vector<char> staged(static_cast<const char*>(s), static_cast<const char*>(s) + n);
+    fake::enqueue(nullptr, [=] { std::memcpy(d, staged.data(), staged.size()); });
+  }
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t st) {
