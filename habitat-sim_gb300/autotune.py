@@ -34,6 +34,7 @@ SMALL_AREA = (8, 16)
 # Bin capacity in use: the share of the shared triangle queue that triggers
 # its rasterisation, tried on the best shape.
 QUEUE_FILL = (50, 75, 100)
+# The per-scene form's regions, tried beside the library's own choice.
 PLAIN_SPACE = [dict(plain_region_width=w, plain_region_height=h) for (w, h) in
                ((16, 32), (16, 64), (32, 64))]
 
@@ -138,7 +139,9 @@ def tune(renderer, poses, triangles, cache=DEFAULT_CACHE, draws=2, plain=True, f
     renderer.setTuning(**shape, queue_fill_percent=best["queue_fill_percent"])
     plain_trials = []
     if plain:
-        for cand in PLAIN_SPACE:
+        now = renderer.tuning()
+        own = {k: now[k] for k in ("plain_region_width", "plain_region_height")}
+        for cand in [own] + [c for c in PLAIN_SPACE if c != own]:
             renderer.setTuning(**cand)
             plain_trials.append(dict(cand, step_ms=_time_plain(renderer, poses, 1)))
         pbest = min(plain_trials, key=lambda t: t["step_ms"])
