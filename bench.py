@@ -374,6 +374,7 @@ def measure(pkg, procedural, name, wl, steps, warmup, plain_steps, e2e_steps, pa
         if k > 0:
             plain_ms.append(e0.elapsed_time(e1))
     plain_fps = wl.envs * len(plain_ms) / (sum(plain_ms) / 1e3) if plain_ms else None
+    plain_launches = int(r.lastDrawStats()["kernel_launches"]) if plain_ms else 0
     t = r.tuning()
     plain_ctas = [-(-w // t["plain_region_width"]) * -(-h // t["plain_region_height"]) for (w, h) in wl.viewports]
 
@@ -446,9 +447,11 @@ def measure(pkg, procedural, name, wl, steps, warmup, plain_steps, e2e_steps, pa
             "p50_ms": float(np.percentile(plain_ms, 50)), "p99_ms": float(np.percentile(plain_ms, 99)),
             "ctas_per_env": {"min": min(plain_ctas), "max": max(plain_ctas),
                              "mean": float(np.mean(plain_ctas))},
-            "form": "one prepare, one order and one raster launch, no graph; "
-                    "ctas_per_env CTAs of %d threads per env (%d x %d px regions)"
-                    % (t["threads"], t["plain_region_width"], t["plain_region_height"])},
+            "form": "%s, no graph; ctas_per_env CTAs of %d threads per env (%d x %d px regions)"
+                    % ({2: "one prepare and one raster launch",
+                        3: "one prepare, one order and one raster launch"}.get(
+                            plain_launches, "%d launches" % plain_launches),
+                       t["threads"], t["plain_region_width"], t["plain_region_height"])},
         "batched_over_plain": value / plain_fps if plain_fps else None,
         "e2e": None if e2e_s is None else {
             "value": wl.envs / e2e_s, "unit": "frames/s", "h2d_bytes_per_step": h2d,
