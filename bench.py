@@ -6,7 +6,8 @@ procedural scenes (20k-triangle room + 200 textured instances each), 128 x 128
 RGBA8 + FP32 linear depth + uint32 semantic id per env, fresh camera poses
 every step (uploaded from host memory inside the step).
 
-Printed (rank 0, one JSON line):
+Printed (rank 0): one JSON line with the metric's own figures (headline()); the
+whole result, with the blocks below, goes to the file named by --details:
   value        frames/s of the batched form (one prepare + one persistent
                raster launch per step, replayed from a CUDA graph), geometry
                and textures resident in HBM, L2 flushed before every step
@@ -83,6 +84,8 @@ def parse():
     p.add_argument("--serving-texture-side", type=int, default=2048)
     p.add_argument("--serving-fractions", type=lambda t: [float(x) for x in t.split(",")],
                    default=[0.1, 0.25, 0.5, 0.75, 0.9])
+    p.add_argument("--details", default=os.path.join(ROOT, "bench_details.json"),
+                   help="file for the whole result (none: not written)")
     p.add_argument("--serving-slots", default="64:96,128:160,256:64",
                    type=lambda t: {int(a): int(b) for a, b in (kv.split(":") for kv in t.split(","))},
                    help="render slots per square resolution, e.g. 64:96,128:64,256:16")
@@ -728,6 +731,43 @@ def run_reference_impl(args):
     return 0
 
 
+def headline(full, details=None):
+    """The printed line: the metric's own keys whole, one or two figures of every
+    other block.  (A reader of the output may keep its last few thousand characters
+    only: the whole result takes ten times that.)"""
+    def pick(block, *keys):
+        return None if block is None else {k: block[k] for k in keys if k in block}
+    line = {k: full[k] for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "p50_ms",
+                                 "p99_ms", "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "config")}
+    line.update(pick(full["details"], "form", "l2"))
+    line["e2e"] = pick(full["e2e"], "value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "ms_per_step")
+    line["gpu_launches"] = full["gpu_launches"]
+    line["clocks"] = full["clocks"]
+    line["plain"] = pick(full["plain"], "value", "ms_per_step")
+    line["roofline"] = pick(full["roofline"], "frac", "achieved", "peak", "unit", "issue_active_frac", "avg_launch_ms")
+    line["parity"] = pick(full["parity"], "envs_checked", "mismatched_pixels", "max_linear_depth_err_m")
+    line["cpu_baseline"] = pick(full["cpu_baseline"], "value", "unit", "cores")
+    line["configs"] = {k: {"value": v["value"], "e2e": v["e2e"] and v["e2e"]["value"]}
+                       for k, v in full["configs"].items()}
+    line["serving"] = full["serving"] and pick(full["serving"].get("saturation"), "requests_per_s")
+    line["replay"] = pick(full["replay"], "value")
+    line["details"] = details
+    return line
+
+
+def write_details(full, path):
+    """Stores the whole result; the file's name, or None if it could not be written."""
+    if not path or path == "none":
+        return None
+    try:
+        with open(path, "w") as f:
+            json.dump(full, f, indent=1)
+        return os.path.basename(path)
+    except OSError as e:
+        print(f"details not written: {e}", file=sys.stderr)
+        return None
+
+
 # Per-config sub-blocks of the default run: (steps, warmup, plain steps, e2e
 # steps, envs checked against the oracle).  config3's 100 steps are its
 # stated 100-step camera walk.  The end-to-end windows run for a few hundred
@@ -810,7 +850,8 @@ def main():
             "replay": replay,
             "postprocess": post,
         }
-        print(json.dumps(line))
+        stored = write_details(line, args.details)
+        print(json.dumps(headline(line, stored)))
     if world > 1:
         torch.distributed.destroy_process_group()
     return 0
