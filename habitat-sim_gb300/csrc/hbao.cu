@@ -344,7 +344,10 @@ __global__ void __launch_bounds__(256, 5)
   const int tiles_x = (s.w + kAoTile - 1) / kAoTile;
   int x = (local % tiles_x) * kAoTile + (int(threadIdx.x) & (kAoTile - 1));
   int y = (local / tiles_x) * kAoTile + int(threadIdx.x) / kAoTile;
-  const bool valid = x < s.w && y < s.h;  // the others stay for the warp's sake, at an edge pixel
+  // Lanes beside the image stay for the warp's sake, at an edge pixel; a warp of them
+  // leaves (256 views of 33 x 33, cache-aware: 76 us with them, 68 without).
+  const bool valid = x < s.w && y < s.h;
+  if (!__any_sync(0xffffffffu, valid)) return;
   x = min(x, s.w - 1);
   y = min(y, s.h - 1);
   AoPixel a;
