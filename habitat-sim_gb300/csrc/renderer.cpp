@@ -1624,6 +1624,20 @@ gbr_status Renderer::draw(cudaStream_t stream, uint32_t mode, bool use_graph) {
   TraceRange trace_("gbr.draw");
   cudaSetDevice(device_);
   if (use_graph && mode == GBR_DRAW_BATCHED && stream == nullptr) stream = own_stream_;
+  if (upload_pending_[slot_] && stream != last_stream_) {
+    // A draw on another stream than the last one's follows it: they share the
+    // visible records, the item lists and the kernels' counters, and a count
+    // that two order kernels mixed up would stay wrong.  (A capture cannot wait
+    // for work outside it, nor anything for a draw that was only captured: there
+    // the caller orders the streams.)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(stream, &capture);
+    if (e == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+      e = cudaStreamWaitEvent(stream, upload_done_[slot_], 0);
+      if (e != cudaSuccess && e != cudaErrorCapturedEvent) return cuda_fail(e, "draw: wait for the last draw's stream");
+    }
+    if (e != cudaSuccess) cudaGetLastError();
+  }
   if (structure_dirty_)
     if (gbr_status s = rebuild(stream)) return s;
   if (bindings_dirty_) plain_dirty_ = true;  // the scenes that are drawn, or what they show, changed

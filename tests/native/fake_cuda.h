@@ -16,6 +16,7 @@
 #include <cstring>
 #include <deque>
 #include <functional>
+#include <map>
 #include <vector>
 
 namespace fake {
@@ -30,6 +31,8 @@ struct Graph {
 inline std::deque<std::function<void()>> legacy;
 inline Graph* capture = nullptr;
 inline cudaStream_t capture_stream = nullptr;
+inline std::map<cudaEvent_t, cudaStream_t> recorded;            // the stream of an event's last record
+inline std::vector<std::pair<cudaStream_t, cudaStream_t>> waits;  // (waiting stream, stream waited for)
 inline int captures = 0, instantiations = 0, sms = 152, occupancy = 2;
 inline std::function<void(const gbr::PrepareParams&, uint32_t scenes)> on_prepare;
 inline std::function<void(const gbr::RasterParams&, uint32_t scenes, uint32_t* done)> on_order;
@@ -135,7 +138,10 @@ cudaError_t cudaDeviceSynchronize() {
   fake::run_legacy();
   return cudaSuccess;
 }
-cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
+  fake::waits.push_back({s, fake::recorded[e]});
+  return fake::capture && s == fake::capture_stream ? cudaErrorStreamCaptureIsolation : cudaSuccess;
+}
 cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus* out) {
   *out = fake::capture && s == fake::capture_stream ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
   return cudaSuccess;
@@ -149,7 +155,10 @@ cudaError_t cudaEventDestroy(cudaEvent_t e) {
   std::free(e);
   return cudaSuccess;
 }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+  fake::recorded[e] = s;
+  return cudaSuccess;
+}
 cudaError_t cudaEventRecordWithFlags(cudaEvent_t, cudaStream_t, unsigned) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
