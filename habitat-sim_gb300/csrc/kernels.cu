@@ -1354,17 +1354,17 @@ __device__ __forceinline__ bool chunk_keep(const float* mvp, const ChunkBox& b, 
 // whose boxes project into the item's region (nanoseconds of a CTA, fitted to
 // measured items: correlation 0.8 to 0.96 in rooms, scans, lit and mixed views;
 // the visible triangles of the whole view: 0.35 to 0.6.  Linear in the clusters
-// it ranks the items of mixed views wrongly: 645 us of the step instead of 610).
+// it ranks the items of mixed views wrongly, 6 % of their step).
 // A CTA projects the clusters of a scene once each, a thread per cluster, and
 // counts them in the cells of the scene's regions in shared memory; a warp per
 // item testing the clusters against its region took twice as long.  The last
 // CTA to finish sorts by counting, into buckets of 1/64 of an octave; the order
 // within one does not matter.  Bound by latency (chains of dependent loads; one
 // CTA for the sort): 29 us cold for 1024 scenes, 23 for 64 scans.
-// Whole steps before and after: 1024 textured views 1779 -> 1594 us, 64 views
-// of scans 916 -> 684, replay of 256 episodes 1078 -> 940, 128 lit views
-// 637 -> 562, 512 mixed views 649 -> 605; the per-scene form, 48 furnished views
-// 298 -> 264 us.
+// Whole steps in the host's order and in this one: 1024 textured views 1779 and
+// 1594 us, 64 views of scans 916 and 684, replay of 256 episodes 1078 and 940, 128
+// lit views 637 and 562, 512 mixed views 649 and 605; 48 furnished views by the
+// per-scene form 298 and 264.
 constexpr int kOrderThreads = 256, kOrderBuckets = 1024, kOrderCells = 1024;
 
 __global__ void __launch_bounds__(kOrderThreads) order_kernel(const RasterParams p, uint32_t scene_count,
